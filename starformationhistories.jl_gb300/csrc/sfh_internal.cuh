@@ -462,10 +462,3 @@ int sfh_bfgs_run(sfh_ctx *ctx, int64_t nvar, const double *d_theta0, const sfh_f
 int sfh_row_stats(sfh_ctx *ctx, const float *d_M, int64_t nbins, int64_t nt, float2 *d_out);
 // Builds the BF16 hi/lo planes from an FP32 column-major matrix (batched.cu).
 int sfh_build_bf16_planes(sfh_ctx *ctx, sfh_models *m, const float *d_f32);
-
-// Templates (templates.cu).
-int sfh_launch_stamps(sfh_ctx *ctx, const double *d_x, const double *d_y, const double *d_sx,
-                      const double *d_sy, const double *d_w, const int64_t *d_start,
-                      const int32_t *d_count, const int32_t *d_cov, int64_t ntempl,
-                      double xf, double xs, int64_t nx, double yf, double ys, int64_t ny,
-                      float *d_out);
