@@ -30,9 +30,10 @@
 
 namespace {
 
-constexpr int kStampThreads = 256;
-constexpr int kWarps = kStampThreads / 32;
-constexpr size_t kBandBudget = 110 * 1024;
+constexpr int kNodeWarps = 8;     // warps of a k_stamp_nodes CTA
+constexpr int kTileWarpsMax = 16;  // most warps of a k_stamp_tiles CTA
+constexpr int kNarrowWarps = 4;   // warps of a k_stamp_narrow CTA
+constexpr int kNarrowRows = 64;   // rows of a separable star's y table at a time
 
 struct Grid2 {
     double xf, xs, yf, ys;
@@ -96,18 +97,52 @@ __device__ __forceinline__ float ex2f(float x) {
 enum { kStarNone = 0, kStarWide = 1, kStarMid = 2, kStarNarrow = 3 };
 
 struct __align__(16) StarRec {
-    // wide: hx, bx, by, amp | uref, vref, kx, ky | cu, cv, -, -   (see wide_tile)
+    // wide: hx, bx, by, amp | uref, vref, kx, ky | cu, cv, strips (64 bits)   (see wide_tile)
     // mid: hx, bx, by, amp | uref, vref, kx, du | dv, -, -, -      (see mid_tile)
-    // narrow, covariant: hi, lo of x edge - x, of y row - y, | of the y step, of 1/(sqrt 2 sx),
-    //                    | x step / (sqrt 2 sx), 1/sy, pref, -
+    // narrow, covariant: uref, bx, bx low, sx | sx low, vref, by, pref | k4, k6, vref low, by low
     // narrow, separable: invx, invy, dx0, dy0 | A/4
     float p[12];
     int xlo, xhi, ylo, yhi;  // first and last bin of the window, 0-based, inside the grid
-    float ir, jr;            // wide, mid: reference bin (0-based)
+    float ir, jr;            // reference bin (0-based; not of a separable narrow star)
     int cls, cov;
 };
 
-constexpr float kTileMid = 3.5f;  // offset of an 8-bin tile's centre from its first bin
+__device__ __forceinline__ unsigned long long star_strips(const StarRec &r) {
+    return (unsigned long long)__float_as_uint(r.p[10]) |
+           (unsigned long long)__float_as_uint(r.p[11]) << 32;
+}
+struct StarId {
+    int32_t t, q;  // template, star of the template
+};
+// bits lo .. hi
+__device__ __forceinline__ unsigned long long strip_bits(int lo, int hi) {
+    return (~0ull >> (63 - hi)) & (~0ull << lo);
+}
+
+// The Chebyshev tiles of a grid (smooth stars, see smooth_strips): wx x wy bins, in strips of
+// wy rows, multiples of the 8 x 8 bin tile.  on: the grid has them.
+struct Smooth {
+    int on, wx, wy, nwc, nstrip;
+    __host__ __device__ int tiles() const { return nwc * nstrip; }
+    __host__ __device__ int groups() const { return (nwc * nstrip + 31) / 32; }
+};
+
+// At most 40 columns by 16 rows when the y step is 1.2 to 4 x steps, 40 rows below that, 8 above:
+// about as far in units of sigma each way.  At most 64 strips (a star's mask).  Grids below
+// 4,096 bins have none: the bin tiles of a template are then two warps' worth or less.
+__host__ __device__ inline Smooth smooth_tiling(const Grid2 &g, bool want) {
+    Smooth s{};
+    const double q = fabs(g.ys / g.xs);
+    s.wx = ((g.nx + (g.nx + 39) / 40 - 1) / ((g.nx + 39) / 40) + 7) / 8 * 8;
+    s.nwc = (g.nx + s.wx - 1) / s.wx;
+    s.wy = q <= 1.2 ? 40 : q <= 4.0 ? 16 : 8;
+    const int least = ((g.ny + 63) / 64 + 7) / 8 * 8;
+    if (s.wy < least) s.wy = least;
+    s.nstrip = (g.ny + s.wy - 1) / s.wy;
+    s.on = want && (int64_t)g.nx * g.ny >= 4096;
+    return s;
+}
+
 constexpr float kRoot2G = 1.1774100225154747f;  // sqrt 2 / g: u in units of sigma
 
 // The record of one star: GaussianPSFAsymmetric / GaussianPSFCovariant windows as in
@@ -119,15 +154,15 @@ constexpr float kRoot2G = 1.1774100225154747f;  // sqrt 2 / g: u in units of sig
 // value is amp 2^-(u^2 + v^2) times the correction, u and v linear in the bin's indices.
 //
 // Wide stars (both steps small against the kernel): the box on both axes.  Covariant kernel:
-// the line at 0.06 (y steps in quadrature) and 0.045 (x step), in units of sqrt 2 sigma, keeps
-// the form, with its correction taken to first order over a tile, within 2e-8 of the kernel's
-// peak and 4e-7 of a bin's own value down to 1e-4 of the peak, against the reference's
+// the line at 0.08 (y steps in quadrature) and 0.045 (x step), in units of sqrt 2 sigma, keeps
+// the form, with its correction taken to second order over a tile, within 5e-8 of the kernel's
+// peak and 9e-7 of a bin's own value down to 1e-4 of the peak, against the reference's
 // 3-point rule in 64 bits.  Separable kernel: 0.1 on each axis (the correction is taken at
 // every row and column; sixth-order terms stay below 1e-9 of the peak).
 //
 // Mid stars (covariant kernel, x step small only): the box in x, the reference's three
 // Gauss-Legendre nodes in y as they are.  x step up to 0.1, and x step^2 * y shift up to
-// 2.5e-3 so that one correction serves the three nodes: within 1e-8 of the peak and 1.5e-6
+// 2.5e-3 so that one correction serves the three nodes (y step up to 4): within 1e-8 of the peak and 1.5e-6
 // of a bin's own value down to 1e-4 of the peak.  The rest (a few bins per sigma) is integrated
 // bin by bin with erfc differences.
 __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x, double y,
@@ -165,9 +200,9 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     const double bx = cov ? 0.7071067811865476 * g.ys * isx : 0.0;
     // (a weight that is not a finite float stays bin by bin: 0 * inf must not leave the window)
     const bool fine = fabs(A) <= 1.0e30 && hx > 0.0 && by > 0.0;
-    const bool wide = fine && (cov ? hx <= 0.045 && bx * bx + by * by <= 0.06 * 0.06
+    const bool wide = fine && (cov ? hx <= 0.045 && bx * bx + by * by <= 0.08 * 0.08
                                    : hx <= 0.1 && by <= 0.1);
-    const bool mid = fine && cov != 0 && !wide && hx <= 0.1 && hx * hx * bx <= 2.5e-3;
+    const bool mid = fine && cov != 0 && !wide && hx <= 0.1 && hx * hx * bx <= 2.5e-3 && by <= 4.0;
     if (wide || mid) {
         const double gs = 1.2011224087864498;  // sqrt(log2 e)
         const double c = (double)cov;
@@ -203,6 +238,7 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
                 r.p[7] = (float)(k4y * k4y / 2880.0);
                 r.p[8] = (float)(-2.0 * s * m * qx / gs);
                 r.p[9] = (float)(2.0 * s * qy / gs);
+                r.p[10] = r.p[11] = 0.f;  // no smooth strips
             } else {
                 r.p[3] = (float)(amp * 0.4444444444444444);  // weight 8/9 of the middle node, halved
                 r.p[6] = (float)(k4x * k4x / 2880.0);
@@ -225,17 +261,63 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     const double xr0 = ((double)xlo - 0.5) * g.xs + g.xf, xr1 = ((double)xhi - 0.5) * g.xs + g.xf;
     const double yr0 = ((double)ylo - 0.5) * g.ys + g.yf, yr1 = ((double)yhi - 0.5) * g.ys + g.yf;
     const double xrs = (xr1 - xr0) / (double)(xhi - xlo), yrs = (yr1 - yr0) / (double)(yhi - ylo);
-    const double inv_sx = 0.7071067811865476 / sx;  // 1 / (√2 σx)
-    const double split[4] = {xr0 - xrs / 2.0 - x, yr0 - y, yrs, inv_sx};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        r.p[2 * k] = (float)split[k];
-        r.p[2 * k + 1] = (float)(split[k] - (double)r.p[2 * k]);
+    const int64_t irl = min(max(xc, xlo), xhi), jrl = min(max(yc, ylo), yhi);
+    const double X = xr0 + (double)(irl - xlo) * xrs - x, Y = yr0 + (double)(jrl - ylo) * yrs - y;
+    const double c = (double)cov;
+    // A few bins per sigma (x step up to 0.25 sqrt 2 sigma): a bin's x integral as the Gaussian
+    // with the box's variance, corrected through its sixth cumulant (He8 terms below 3e-9);
+    // u at bin centres, base-2 scale.  Else erfc differences, u = t at the bins' lower edges.
+    const bool gauss = hx > 0.0 && hx <= 0.25;
+    const double vx = gauss ? sx * sx + xrs * xrs / 12.0 : sx * sx;
+    // (a vanishing error: far edges at a large finite t, a hard histogram)
+    const double scale = fmin(0.7071067811865476 / sqrt(vx) * (gauss ? 1.2011224087864498 : 1.0), 1.0e30);
+    const double bxs = c * yrs * scale, sxs = xrs * scale, k = xrs * xrs / vx;
+    r.ir = (float)(irl - 1);
+    r.jr = (float)(jrl - 1);
+    r.p[0] = (float)((X + c * Y - (gauss ? 0.0 : xrs / 2.0)) * scale);
+    r.p[1] = (float)bxs;
+    r.p[2] = (float)(bxs - (double)r.p[1]);
+    r.p[3] = (float)sxs;
+    r.p[4] = (float)(sxs - (double)r.p[3]);
+    const double vref = Y * isy * 0.8493218002880191, bys = yrs * isy * 0.8493218002880191;  // g / √2
+    r.p[5] = (float)vref;
+    r.p[6] = (float)bys;
+    r.p[10] = (float)(vref - (double)r.p[5]);
+    r.p[11] = (float)(bys - (double)r.p[6]);
+    // prefac = A / 2 / sqrt(2π) / σy (:320) times the scale hy = yrs / 2 of the GL weights
+    // (:325), and the unit Gaussian's integral 2/√π xrs / (√2 √vx)
+    r.p[7] = (float)(A / 2.0 / 2.5066282746310002 * isy * (yrs / 2.0) *
+                     (gauss ? 0.7978845608028654 * sqrt(k) : 1.0));
+    r.p[8] = gauss ? (float)(k * k / 2880.0) : -1.f;
+    r.p[9] = (float)(k * k * k / 181440.0);
+}
+
+// The strips over which a wide star's contribution can be interpolated from 8 x 8 Chebyshev
+// points per tile: its window covers the strip, and over a tile's half width its logarithm
+// changes by at most 0.7 on each axis, 0.08 of it by curvature.  The interpolation error of
+// exp(c x) is 2 (c/2)^8 / 8! = 1e-8 of the value at the tile's centre, that of exp(-q x^2)
+// 2 (q/4)^4 / 4! = 1.3e-8; at the tile's far end it is e^0.8 times that of the value there.
+__device__ __forceinline__ unsigned long long smooth_strips(const StarRec &r, const Grid2 &g,
+                                                            const Smooth &sm) {
+    if (r.xlo > 0 || r.xhi < g.nx - 1) return 0ull;
+    const float xh = 0.5f * (float)sm.wx, yh = 0.5f * (float)sm.wy;
+    const float hx = r.p[0], bx = r.p[1], by = r.p[2], ln2 = 0.6931472f;
+    if (!(ln2 * hx * hx * xh * xh <= 0.08f && ln2 * (bx * bx + by * by) * yh * yh <= 0.08f)) return 0ull;
+    unsigned long long m = 0ull;
+    const float i0 = -r.ir - 0.5f, i1 = i0 + (float)(sm.nwc * sm.wx);
+    const float u0 = fmaf(i0, hx, r.p[4]), u1 = fmaf(i1, hx, r.p[4]);
+    for (int k = 0; k < sm.nstrip; ++k) {
+        const int ra = k * sm.wy, rb = min(g.ny, ra + sm.wy) - 1;
+        if (r.ylo > ra || r.yhi < rb) continue;
+        // u and v are linear: largest magnitudes at the corners of the area the tiles cover
+        const float j0 = (float)ra - r.jr - 0.5f, j1 = j0 + (float)sm.wy;
+        const float um = fmaxf(fmaxf(fabsf(fmaf(j0, bx, u0)), fabsf(fmaf(j1, bx, u0))),
+                               fmaxf(fabsf(fmaf(j0, bx, u1)), fabsf(fmaf(j1, bx, u1))));
+        const float vm = fmaxf(fabsf(fmaf(j0, by, r.p[5])), fabsf(fmaf(j1, by, r.p[5])));
+        if (2.f * ln2 * um * hx * xh <= 0.7f && 2.f * ln2 * (um * fabsf(bx) + vm * by) * yh <= 0.7f)
+            m |= 1ull << k;
     }
-    r.p[8] = (float)(xrs * inv_sx);
-    r.p[9] = (float)(1.0 / sy);
-    // prefac = A / 2 / sqrt(2π) / σy (:320) times the scale hy = yrs / 2 of the GL weights (:325)
-    r.p[10] = (float)(A / 2.0 / 2.5066282746310002 / sy * (yrs / 2.0));
+    return m;
 }
 
 constexpr int kPrepThreads = 64;  // small blocks: a few hundred stars already spread over the SMs
@@ -245,70 +327,91 @@ k_star_prep(const double *__restrict__ xs, const double *__restrict__ ys,
             const double *__restrict__ sxs, const double *__restrict__ sys,
             const double *__restrict__ ws, const int64_t *__restrict__ start,
             const int32_t *__restrict__ count, const int32_t *__restrict__ covs, Grid2 g0,
-            const Grid2 *__restrict__ grids, int t0, StarRec *__restrict__ rec) {
+            const Grid2 *__restrict__ grids, int t0, StarRec *__restrict__ rec,
+            StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
     const int t = t0 + blockIdx.y;
     const int q = blockIdx.x * kPrepThreads + threadIdx.x;
     if (q >= count[t]) return;
     const int64_t s = start[t] + q;
     StarRec r{};
-    star_record(r, grids ? grids[t] : g0, xs[s], ys[s], sxs[s], sys[s], ws[s], covs[t]);
+    const Grid2 g = grids ? grids[t] : g0;
+    star_record(r, g, xs[s], ys[s], sxs[s], sys[s], ws[s], covs[t]);
+    if (r.cls == kStarWide) {
+        const Smooth sm = smooth_tiling(g, true);
+        const unsigned long long m = sm.on ? smooth_strips(r, g, sm) : 0ull;
+        r.p[10] = __uint_as_float((unsigned int)m);
+        r.p[11] = __uint_as_float((unsigned int)(m >> 32));
+    }
+    // the narrow stars of all templates in one list (one atomic per warp)
+    const unsigned act = __activemask(), nar = __ballot_sync(act, r.cls == kStarNarrow);
+    if (r.cls == kStarNarrow) {
+        const int lane = threadIdx.x & 31, lead = __ffs(nar) - 1;
+        int at = 0;
+        if (lane == lead) at = atomicAdd(n_narrow, __popc(nar));
+        at = __shfl_sync(nar, at, lead);
+        narrow[at + __popc(nar & ((1u << lane) - 1u))] = StarId{t, q};
+    }
     rec[s] = r;
 }
 
 // ---------------------------------------------------------------- narrow stars
-// A star whose kernel is not wide against the bins: one warp integrates it bin by bin and
-// adds it to the band with shared-memory atomics.  Separable kernel: x and y factor tables.
-__device__ void star_asym(float *band, float *bx_buf, float *by_buf, const StarRec &r, int nx,
-                          int ty0, int tyn, int lane) {
-    const int jlo = max(r.ylo, ty0), jhi = min(r.yhi, ty0 + tyn - 1);
-    if (jlo > jhi) return;
-    const int lx = r.xhi - r.xlo + 1, ly = jhi - jlo + 1, row_off = jlo - r.ylo;
+// A star whose kernel is not wide against the bins: a warp adds it to the template in global
+// memory (L2 adds FP32 natively; a shared-memory FP32 atomicAdd is a compare-and-swap loop).
+// Separable kernel: x and y factor tables.
+__device__ void star_asym(float *__restrict__ out, float *bx_buf, float *by_buf, const StarRec &r,
+                          int nx, int lane) {
+    const int lx = r.xhi - r.xlo + 1;
     const float invx = r.p[0], invy = r.p[1], dx0 = r.p[2], dy0 = r.p[3], a4 = r.p[4];
-    for (int m = lane; m < lx; m += 32) bx_buf[m] = gauss_bin((dx0 + (float)m) * invx, invx);
-    for (int m = lane; m < ly; m += 32)
-        by_buf[m] = a4 * gauss_bin((dy0 + (float)(m + row_off)) * invy, invy);
-    __syncwarp();
-    const int total = lx * ly;
     const float inv_lx = 1.0f / (float)lx;
-    float *base = band + (int64_t)(jlo - ty0) * nx + r.xlo;
-    for (int p = lane; p < total; p += 32) {
-        const int jj = (int)(((float)p + 0.5f) * inv_lx);
-        const int ii = p - jj * lx;
-        atomicAdd(base + (int64_t)jj * nx + ii, bx_buf[ii] * by_buf[jj]);
+    for (int m = lane; m < lx; m += 32) bx_buf[m] = gauss_bin((dx0 + (float)m) * invx, invx);
+    for (int j0 = r.ylo; j0 <= r.yhi; j0 += kNarrowRows) {
+        const int ly = min(kNarrowRows, r.yhi - j0 + 1);
+        for (int m = lane; m < ly; m += 32)
+            by_buf[m] = a4 * gauss_bin((dy0 + (float)(m + j0 - r.ylo)) * invy, invy);
+        __syncwarp();
+        const int total = lx * ly;
+        float *base = out + (int64_t)j0 * nx + r.xlo;
+        for (int p = lane; p < total; p += 32) {
+            const int jj = (int)(((float)p + 0.5f) * inv_lx);
+            const int ii = p - jj * lx;
+            atomicAdd(base + (int64_t)jj * nx + ii, bx_buf[ii] * by_buf[jj]);
+        }
+        __syncwarp();
     }
-    __syncwarp();
 }
 
-// Covariant kernel.  Each lane prepares one row of the window: per Gauss-Legendre node in y
-// its weight, and t of a bin edge near the kernel's centre in that row (in FP64, since edge
-// and shear cancel there), which the warp then reads by shuffles.
-__device__ void star_cov(float *band, const StarRec &r, int nx, int ty0, int tyn, int lane) {
-    const int jlo = max(r.ylo, ty0), jhi = min(r.yhi, ty0 + tyn - 1);
-    if (jlo > jhi) return;
-    const float sxr = r.p[8];
-    const double xe = (double)r.p[0] + (double)r.p[1], dyb = (double)r.p[2] + (double)r.p[3];
-    const double yrs = (double)r.p[4] + (double)r.p[5], isx = (double)r.p[6] + (double)r.p[7];
-    const double cov = (double)r.cov;
-    const int lx = r.xhi - r.xlo + 1;
-    const int nrows = jhi - jlo + 1;
-    float *band_row0 = band + (int64_t)(jlo - ty0) * nx + r.xlo;
-    // bins narrow in t (a star whose exponents leave the range of the tile forms): quadrature
-    // per bin; else erfc at the shared bin edges, neighbours exchanged by shuffles
-    const bool quad = sxr <= 0.05f;
-    const int E = quad ? lx : lx + 1;
-    const int W = min(E, 32), rows_per = 32 / W;
-    const int nb = quad ? W : W - 1;  // bins per segment pass
+// Covariant kernel.  Each lane prepares one row: per Gauss-Legendre node in y its weight, and
+// u of a bin near the kernel's centre in that row (the shear and the bin's offset cancel there:
+// their sum is formed in two floats), which the warp then reads by shuffles.
+__device__ void star_cov(float *__restrict__ out, const StarRec &r, int nx, int lane) {
+    const float sx = r.p[3], k4 = r.p[8], k6 = r.p[9];
+    const int lx = r.xhi - r.xlo + 1, nrows = r.yhi - r.ylo + 1;
+    const float c_first = (float)r.xlo - r.ir, c_last = (float)(r.xhi + 1) - r.ir;
+    float *row0 = out + (int64_t)r.ylo * nx + r.xlo;
+    const bool gauss = k4 >= 0.f;
+    // 1 - k4 He4(z) + k6 He6(z), z^2 = 2 ln 2 u^2, by powers of u^2
+    const float g0 = 1.f - 3.f * k4 - 15.f * k6, g1 = 1.3862943611198906f * (6.f * k4 + 45.f * k6);
+    const float g2 = -1.9218120556728056f * (k4 + 15.f * k6), g3 = 2.6641971970211f * k6;
+    const int W = min(gauss ? lx : lx + 1, 32), rows_per = 32 / W;
+    const int nb = gauss ? W : W - 1;  // bins per segment pass
     const int seg = lane / W, pos = lane - seg * W;
     for (int r0 = 0; r0 < nrows; r0 += 32) {
         float ck[3], tk[3], ek[3];
-        const double dyc = dyb + (double)(jlo - r.ylo + r0 + lane) * yrs;
+        // u (at the reference bin) and v of the row's centre as two floats each
+        const float d = (float)(r.ylo + r0 + lane) - r.jr, bx = r.p[1], by = r.p[6];
+        const float p = d * bx, uh = r.p[0] + p, z = uh - r.p[0];
+        const float ul = ((r.p[0] - (uh - z)) + (p - z)) + fmaf(d, r.p[2], fmaf(d, bx, -p));
+        const float p2 = d * by, vh = r.p[5] + p2, z2 = vh - r.p[5];
+        const float vl = ((r.p[5] - (vh - z2)) + (p2 - z2)) +
+                         fmaf(d, r.p[11], fmaf(d, by, -p2) + r.p[10]);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const double dy = dyc + (k - 1) * 0.3872983346207417 * yrs;  // sqrt(3/5) / 2
-            const double t = (xe + cov * dy) * isx;
-            ek[k] = fminf(fmaxf(rintf(-__fdividef((float)t, sxr)), 0.f), (float)lx);
-            tk[k] = (float)(t + (double)ek[k] * ((double)sxr));
-            ck[k] = r.p[10] * c_glw[k] * exp_negsq(0.7071067811865476f * (float)dy * r.p[9]);
+            const float gk = (float)(k - 1) * 0.38729835f, gl = (float)(k - 1) * -1.0945054e-8f;  // sqrt(3/5) / 2
+            ek[k] = fminf(fmaxf(rintf(-__fdividef(fmaf(gk, bx, uh), sx)), c_first), c_last);
+            const float t = fmaf(ek[k], sx, uh);
+            tk[k] = fmaf(gk, bx, t) + fmaf(gl, bx, fmaf(ek[k], r.p[4], ul));
+            const float v = fmaf(gk, by, vh) + fmaf(gl, by, fmaf(gk, r.p[11], vl)), q = v * v;
+            ck[k] = r.p[7] * c_glw[k] * ex2f(-q) * fmaf(-0.6931471805599453f, fmaf(v, v, -q), 1.f);
         }
         const int rend = min(32, nrows - r0);
         for (int rb = 0; rb < rend; rb += rows_per) {
@@ -319,21 +422,23 @@ __device__ void star_cov(float *band, const StarRec &r, int nx, int ty0, int tyn
             for (int k = 0; k < 3; ++k) {
                 c[k] = __shfl_sync(0xffffffffu, ck[k], row & 31);
                 t0[k] = __shfl_sync(0xffffffffu, tk[k], row & 31);
-                e0k[k] = __shfl_sync(0xffffffffu, ek[k], row & 31);
+                e0k[k] = __shfl_sync(0xffffffffu, ek[k], row & 31) - c_first;
             }
             for (int e0 = 0; e0 < lx; e0 += nb) {
                 const int e = e0 + pos;
                 float v = 0.f;
                 bool put = vrow && e < lx;
-                if (quad) {
+                if (gauss) {
 #pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        v = fmaf(c[k], gl3_bin(fmaf((float)e - e0k[k], sxr, t0[k]), sxr), v);
+                    for (int k = 0; k < 3; ++k) {
+                        const float u = fmaf((float)e - e0k[k], sx, t0[k]), q = u * u;
+                        v = fmaf(c[k] * ex2f(-q), fmaf(q, fmaf(q, fmaf(q, g3, g2), g1), g0), v);
+                    }
                 } else {
                     float ev[3];
 #pragma unroll
                     for (int k = 0; k < 3; ++k)
-                        ev[k] = vrow && e <= lx ? erfc_signed(fmaf((float)e - e0k[k], sxr, t0[k])) : 0.f;
+                        ev[k] = vrow && e <= lx ? erfc_signed(fmaf((float)e - e0k[k], sx, t0[k])) : 0.f;
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const float en = __shfl_down_sync(0xffffffffu, ev[k], 1);
@@ -341,7 +446,7 @@ __device__ void star_cov(float *band, const StarRec &r, int nx, int ty0, int tyn
                     }
                     put = put && pos < W - 1;
                 }
-                if (put) atomicAdd(band_row0 + (int64_t)(r0 + row) * nx + e, v);
+                if (put) atomicAdd(row0 + (int64_t)(r0 + row) * nx + e, v);
             }
         }
     }
@@ -355,66 +460,100 @@ __device__ void star_cov(float *band, const StarRec &r, int nx, int ty0, int tyn
 // so the bin's value is X[di] Y[dj] T[dj][di]: 8 + 8 exponentials per tile, T (the star's
 // own shear table, shared by all tiles) from shared memory, and a multiply and an FMA per
 // bin on packed pairs (no T for the separable kernel).  The He4 corrections of the covariant
-// kernel enter X and Y by their value and slope at the tile's centre.  X and Y are zero
+// kernel enter X and Y by their value, slope and axial curvature at the tile's centre, those
+// of the separable kernel at every row and column.  X and Y are zero
 // outside the star's window.
-template <bool COV>
+//
+// NODES: the same at the 8 x 8 Chebyshev points of a larger tile that the star's window
+// covers (see smooth_strips): the values are interpolated to the bins once, after the sum
+// over stars.  Each (star, strip) is taken by one of the two forms.
+__device__ __forceinline__ float tile_node(bool nodes, int i) {  // ascending, i = 0..7
+    if (!nodes) return (float)i - 3.5f;
+    const int k = i < 4 ? i : 7 - i;
+    const float c = k == 0 ? 0.9807852804032304f : k == 1 ? 0.8314696123025452f
+                  : k == 2 ? 0.5555702330196022f : 0.19509032201612825f;
+    return i < 4 ? -c : c;
+}
+
+struct Tile {
+    int col0, row0;          // first bin (plain tiles)
+    float xc, yc, xh, yh;    // centre in 0-based bins, half widths (NODES)
+    int strip;               // the strip it lies in
+    bool live;
+};
+
+template <bool COV, bool NODES>
 __device__ __forceinline__ void wide_tile(float2 (&acc)[8][4], const StarRec &r,
-                                          const float *__restrict__ T, int col0, int row0,
-                                          bool live) {
-    const bool over = live && col0 <= r.xhi && col0 + 7 >= r.xlo && row0 <= r.yhi && row0 + 7 >= r.ylo;
+                                          const float *__restrict__ T, const Tile &tl) {
+    const int col0 = tl.col0, row0 = tl.row0;
+    const bool own = ((star_strips(r) >> tl.strip & 1ull) != 0ull) == NODES;
+    const bool over = tl.live && own && (NODES || (col0 <= r.xhi && col0 + 7 >= r.xlo &&
+                                                   row0 <= r.yhi && row0 + 7 >= r.ylo));
     if (!__any_sync(0xffffffffu, over)) return;
-    const bool part = over && !(col0 >= r.xlo && col0 + 7 <= r.xhi && row0 >= r.ylo && row0 + 7 <= r.yhi);
-    const float hx = r.p[0], bx = r.p[1], by = r.p[2];
+    const bool part = !NODES && over && !(col0 >= r.xlo && col0 + 7 <= r.xhi && row0 >= r.ylo &&
+                                          row0 + 7 <= r.yhi);
     // a lane outside the window works on the reference bin with amplitude 0
-    const float di0 = over ? (float)col0 + (kTileMid - r.ir) : 0.f;
-    const float dj0 = over ? (float)row0 + (kTileMid - r.jr) : 0.f;
+    const float di0 = over ? (NODES ? tl.xc : (float)col0 + 3.5f) - r.ir : 0.f;
+    const float dj0 = over ? (NODES ? tl.yc : (float)row0 + 3.5f) - r.jr : 0.f;
     const float amp = over ? r.p[3] : 0.f;
-    float u = fmaf(di0, hx, r.p[4]);
-    if (COV) u = fmaf(dj0, bx, u);
-    const float v = fmaf(dj0, by, r.p[5]);
+    float u = fmaf(di0, r.p[0], r.p[4]);
+    if (COV) u = fmaf(dj0, r.p[1], u);
+    const float v = fmaf(dj0, r.p[2], r.p[5]);
+    const float hx = NODES ? r.p[0] * tl.xh : r.p[0], bx = NODES ? r.p[1] * tl.yh : r.p[1];
+    const float by = NODES ? r.p[2] * tl.yh : r.p[2];
     // u^2 + v^2 with its rounding error e
     const float pu = u * u, pv = v * v, s = pu + pv, z = s - pu;
     const float e = (fmaf(u, u, -pu) + fmaf(v, v, -pv)) + ((pu - (s - z)) + (pv - z));
-    const float zx = kRoot2G * u, hx2 = hx * hx;
-    float X[8], Y[8];
-    if (COV) {
-        // 1 - kx He4(zx) - ky He4(xi): value and slopes (of its logarithm, base 2) at the centre
-        const float xi = fmaf(r.p[8], u, r.p[9] * v), zx2 = zx * zx, xi2 = xi * xi;
-        const float lr = -fmaf(r.p[6], fmaf(zx2, zx2 - 6.f, 3.f), r.p[7] * fmaf(xi2, xi2 - 6.f, 3.f));
-        const float hxi = -5.770780163555854f * r.p[7] * xi * (xi2 - 3.f);  // 4 log2 e
-        const float au = fmaf(-2.f, u, fmaf(hxi, r.p[8], -5.770780163555854f * kRoot2G * r.p[6] * zx * (zx2 - 3.f)));
-        const float av = fmaf(-2.f, v, hxi * r.p[9]);
-        const float gx = hx * au, gy = fmaf(bx, au, by * av), b2 = fmaf(bx, bx, by * by);
-        const float A = amp * ex2f(-s) * fmaf(-0.6931471805599453f, e, 1.f + lr);
+    const float zx = kRoot2G * u;
+    float X[8], A, gy, cy, zy = 0.f;  // row j: A 2^(gy d - cy d^2)
+    if (COV || NODES) {
+        // 1 - kx He4(zx) - ky He4(xi) at the centre: its value, and of its logarithm (base 2)
+        // the slopes (4 log2 e He3) and the curvature along the two axes (6 log2 e He2)
+        const float kx = r.p[6], ky = r.p[7], cu = r.p[8], cv = r.p[9];
+        const float xi = fmaf(cu, u, cv * v), zx2 = zx * zx, xi2 = xi * xi;
+        const float lr = -fmaf(kx, fmaf(zx2, zx2 - 6.f, 3.f), ky * fmaf(xi2, xi2 - 6.f, 3.f));
+        const float hxi = -5.770780163555854f * ky * xi * (xi2 - 3.f);
+        const float au = fmaf(-2.f, u, fmaf(hxi, cu, -5.770780163555854f * kRoot2G * kx * zx * (zx2 - 3.f)));
+        const float av = fmaf(-2.f, v, hxi * cv);
+        const float qx = 8.656170245333781f * kRoot2G * kRoot2G * kx * (zx2 - 1.f);
+        const float qy = 8.656170245333781f * ky * (xi2 - 1.f), w = fmaf(cu, bx, cv * by);
+        const float gx = hx * au, cx = hx * hx * fmaf(qy * cu, cu, 1.f + qx);
+        gy = fmaf(bx, au, by * av);
+        cy = fmaf(bx * bx, 1.f + qx, fmaf(qy * w, w, by * by));
+        A = amp * ex2f(-s) * fmaf(-0.6931471805599453f, e, 1.f + lr);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float d = kTileMid - (float)i;
-            const float cx = hx2 * d * d, cy = b2 * d * d;
-            X[i] = ex2f(fmaf(-gx, d, -cx));
-            X[7 - i] = ex2f(fmaf(gx, d, -cx));
-            Y[i] = A * ex2f(fmaf(-gy, d, -cy));
-            Y[7 - i] = A * ex2f(fmaf(gy, d, -cy));
+            const float d = tile_node(NODES, 7 - i), c = cx * (d * d);
+            X[i] = ex2f(fmaf(-gx, d, -c));
+            X[7 - i] = ex2f(fmaf(gx, d, -c));
         }
     } else {
-        const float zy = kRoot2G * v, by2 = by * by, A = amp * ex2f(-s) * fmaf(-0.6931471805599453f, e, 1.f);
+        zy = kRoot2G * v;
+        gy = -2.f * v * by;
+        cy = by * by;
+        A = amp * ex2f(-s) * fmaf(-0.6931471805599453f, e, 1.f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const float d = (float)i - kTileMid;
-            const float a = fmaf(kRoot2G * hx, d, zx), b = fmaf(kRoot2G * by, d, zy), a2 = a * a, b2 = b * b;
-            X[i] = ex2f(-fmaf(2.f * u * hx, d, hx2 * d * d)) * fmaf(-r.p[6], fmaf(a2, a2 - 6.f, 3.f), 1.f);
-            Y[i] = A * ex2f(-fmaf(2.f * v * by, d, by2 * d * d)) * fmaf(-r.p[7], fmaf(b2, b2 - 6.f, 3.f), 1.f);
+            const float d = tile_node(false, i), a = fmaf(kRoot2G * hx, d, zx), a2 = a * a;
+            X[i] = ex2f(-fmaf(2.f * u * hx, d, hx * hx * (d * d))) * fmaf(-r.p[6], fmaf(a2, a2 - 6.f, 3.f), 1.f);
         }
     }
     if (__any_sync(0xffffffffu, part)) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 8; ++i)
             if (col0 + i < r.xlo || col0 + i > r.xhi) X[i] = 0.f;
-            if (row0 + i < r.ylo || row0 + i > r.yhi) Y[i] = 0.f;
-        }
     }
+    const int ylo = NODES ? row0 : r.ylo, yhi = NODES ? row0 + 7 : r.yhi;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const float2 y2 = make_float2(Y[j], Y[j]);
+        const float d = tile_node(NODES, j);
+        float y = A * ex2f(fmaf(gy, d, -(cy * (d * d))));
+        if (!COV && !NODES) {
+            const float b = fmaf(kRoot2G * by, d, zy), b2 = b * b;
+            y *= fmaf(-r.p[7], fmaf(b2, b2 - 6.f, 3.f), 1.f);
+        }
+        if (row0 + j < ylo || row0 + j > yhi) y = 0.f;
+        const float2 y2 = make_float2(y, y);
         if (COV) {
             const float4 t0 = *reinterpret_cast<const float4 *>(T + 8 * j);
             const float4 t1 = *reinterpret_cast<const float4 *>(T + 8 * j + 4);
@@ -422,6 +561,7 @@ __device__ __forceinline__ void wide_tile(float2 (&acc)[8][4], const StarRec &r,
             acc[j][1] = __ffma2_rn(make_float2(X[2], X[3]), __fmul2_rn(make_float2(t0.z, t0.w), y2), acc[j][1]);
             acc[j][2] = __ffma2_rn(make_float2(X[4], X[5]), __fmul2_rn(make_float2(t1.x, t1.y), y2), acc[j][2]);
             acc[j][3] = __ffma2_rn(make_float2(X[6], X[7]), __fmul2_rn(make_float2(t1.z, t1.w), y2), acc[j][3]);
+            asm volatile("" ::: "memory");  // one row's T at a time in registers
         } else {
 #pragma unroll
             for (int c = 0; c < 4; ++c)
@@ -433,13 +573,13 @@ __device__ __forceinline__ void wide_tile(float2 (&acc)[8][4], const StarRec &r,
 // A mid star's tile: the sum over the three y nodes k of X_k[di] Y_k[dj], times T[dj][di] and
 // the x correction 1 - kx He4 at the bin's own u (nine operations per bin).
 __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
-                                         const float *__restrict__ T, int col0, int row0,
-                                         bool live) {
-    const bool over = live && col0 <= r.xhi && col0 + 7 >= r.xlo && row0 <= r.yhi && row0 + 7 >= r.ylo;
+                                         const float *__restrict__ T, const Tile &tl) {
+    const int col0 = tl.col0, row0 = tl.row0;
+    const bool over = tl.live && col0 <= r.xhi && col0 + 7 >= r.xlo && row0 <= r.yhi && row0 + 7 >= r.ylo;
     if (!__any_sync(0xffffffffu, over)) return;
     const float hx = r.p[0], bx = r.p[1], by = r.p[2], dn = r.p[7], en = r.p[8];
-    const float di0 = over ? (float)col0 + (kTileMid - r.ir) : 0.f;
-    const float dj0 = over ? (float)row0 + (kTileMid - r.jr) : 0.f;
+    const float di0 = over ? (float)col0 + 3.5f - r.ir : 0.f;
+    const float dj0 = over ? (float)row0 + 3.5f - r.jr : 0.f;
     const float amp = over ? r.p[3] : 0.f;
     const float u = fmaf(dj0, bx, fmaf(di0, hx, r.p[4])), v = fmaf(dj0, by, r.p[5]);
     // 1 - kx He4(sqrt 2 u / g) = c0 + c1 u^2 + c2 u^4
@@ -453,7 +593,7 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
         float x0[2], xm[2], xp[2], h2[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const float d = (float)(2 * c + q) - kTileMid, cx = hx2 * d * d;
+            const float d = tile_node(false, 2 * c + q), cx = hx2 * d * d;
             const bool in = col0 + 2 * c + q >= r.xlo && col0 + 2 * c + q <= r.xhi;
             x0[q] = in ? ex2f(fmaf(g0, d, -cx)) : 0.f;
             xm[q] = in ? ex2f(fmaf(g0 - gd, d, -cx)) : 0.f;
@@ -467,7 +607,7 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const float d = (float)j - kTileMid, uj = fmaf(bx, d, u), vj = fmaf(by, d, v);
+        const float d = tile_node(false, j), uj = fmaf(bx, d, u), vj = fmaf(by, d, v);
         const float a = row0 + j >= r.ylo && row0 + j <= r.yhi ? amp : 0.f;
         const float um = uj - dn, vm = vj - en, up = uj + dn, vp = vj + en;
         const float y0 = a * ex2f(-fmaf(uj, uj, vj * vj));
@@ -486,189 +626,301 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
             const float2 f = __ffma2_rn(Xp[c], yp2, __ffma2_rn(X0[c], y02, __fmul2_rn(Xm[c], ym2)));
             acc[j][c] = __ffma2_rn(__fmul2_rn(f, t[c]), R, acc[j][c]);
         }
+        asm volatile("" ::: "memory");
     }
 }
 
-// ---------------------------------------------------------------- k_stamps
-constexpr int kBatch = 16;  // wide stars staged at a time
-
-struct StampShared {
-    StarRec rec[kBatch];
-    float T[kBatch][64];
-    int list[kStampThreads];  // one chunk's stars of a class, by position in the template
-    int wcnt[kWarps];
-    int next;
-};
-
+// ---------------------------------------------------------------- the stamp kernels
+// A template's smooth (star, strip) pairs on its Chebyshev tiles (k_stamp_nodes), the wide and
+// mid stars on its 8 x 8 tiles with the interpolated sums of the smooth pairs added
+// (k_stamp_tiles, which writes the template), then the narrow stars (k_stamp_narrow).  Warps
+// work by themselves: where the stars lie differs so much from one part of a diagram to the
+// next that warps sharing a band in shared memory waited a third of their time for one another.
 struct StampStars {
     const double *x, *y, *sx, *sy, *w;
-    const StarRec *rec;  // NULL: records are made while staging
+    const StarRec *rec;  // one per star, where the star counts are known to the host
     const int64_t *start;
     const int32_t *count, *cov;
 };
 
-// Kept out of line: its FP64 registers would otherwise be live beside the accumulators.
-__device__ __noinline__ void make_record(StarRec *r, const StampStars *st, int64_t s, const Grid2 *g,
-                                         int cov) {
-    star_record(*r, *g, st->x[s], st->y[s], st->sx[s], st->sy[s], st->w[s], cov);
-}
-__device__ __forceinline__ void load_record(StarRec &r, const StampStars &st, int64_t s,
-                                            const Grid2 &g, int cov) {
-    if (st.rec) r = st.rec[s];
-    else make_record(&r, &st, s, &g, cov);
-}
-
-// Lists in S.list, in star order, the stars q0 .. q0 + 255 of the template (first star s0,
-// n of them) of one class whose window reaches rows ty0 .. ty1; returns their number.  Every
-// thread of the block calls it.
-__device__ __forceinline__ int list_chunk(StampShared &S, const StampStars &st, int64_t s0, int n,
-                                          int q0, const Grid2 &g, int cov, int ty0, int ty1,
-                                          int want) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = q0 + (int)threadIdx.x;
-    bool take = false;
-    if (q < n) {
-        if (st.rec) {
-            const StarRec *r = st.rec + s0 + q;
-            take = r->cls == want && r->ylo <= ty1 && r->yhi >= ty0;
-        } else {
-            StarRec r;
-            load_record(r, st, s0 + q, g, cov);
-            take = r.cls == want && r.ylo <= ty1 && r.yhi >= ty0;
-        }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    __syncthreads();  // the previous chunk's list is no longer read
-    if (lane == 0) S.wcnt[warp] = __popc(m);
-    if (threadIdx.x == 0) S.next = 0;
-    __syncthreads();
-    int base = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-        if (w == warp) base = tot;
-        tot += S.wcnt[w];
-    }
-    if (take) S.list[base + __popc(m & ((1u << lane) - 1u))] = q;
-    __syncthreads();
-    return tot;
-}
-
-// One band of TY Hess rows of template t.  Its stars are read in chunks of one per thread
-// and listed by class.  Narrow stars first: pulled by warps.  Then the wide stars: staged
-// kBatch at a time with their shear tables, every warp adds them to its 32 tiles; when the
-// band has fewer than 8 warps' worth of tiles, the stars of a batch are dealt out over
-// groups of warps.  (Two scans of the list, so that the 64 accumulators of a lane are not
-// live across the narrow stars' code.)
-template <bool COV>
-__device__ void stamp_band(float *smem, StampShared &S, const StampStars &st, int t, const Grid2 &g,
-                           int ty0, int TY, float *__restrict__ dst) {
-    const int tyn = min(TY, g.ny - ty0);
-    float *band = smem;
-    const int bandn = tyn * g.nx;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t s0 = st.start[t];
-    const int n = st.count[t], cov = st.cov[t];
-    for (int k = threadIdx.x; k < bandn; k += kStampThreads) band[k] = 0.f;
-    for (int q0 = 0; q0 < n; q0 += kStampThreads) {
-        float *wb = smem + (size_t)TY * g.nx + (size_t)warp * (g.nx + TY);
-        const int nn = list_chunk(S, st, s0, n, q0, g, cov, ty0, ty0 + tyn - 1, kStarNarrow);
-        for (;;) {
-            int k = 0;
-            if (lane == 0) k = atomicAdd(&S.next, 1);
-            k = __shfl_sync(0xffffffffu, k, 0);
-            if (k >= nn) break;
-            StarRec r;
-            load_record(r, st, s0 + S.list[k], g, cov);
-            if (COV) star_cov(band, r, g.nx, ty0, tyn, lane);
-            else star_asym(band, wb, wb + g.nx, r, g.nx, ty0, tyn, lane);
-        }
-    }
-    const int ntc = (g.nx + 7) >> 3, ntiles = ntc * ((tyn + 7) >> 3);
-    const int ntg = (ntiles + 31) >> 5;
-    const int ns = ntg >= kWarps ? 1 : kWarps / ntg;  // star groups
-    const int tgs = ntg >= kWarps ? kWarps : ntg;     // tile groups per pass
-    const int tg0 = warp % tgs, sg = warp / tgs;
-    for (int pass = 0; pass < ntg; pass += kWarps) {
-        const int tile = (pass + tg0) * 32 + lane;
-        const bool live = tile < ntiles && sg < ns;
-        const int col0 = (tile % ntc) * 8, row0 = ty0 + (tile / ntc) * 8;
-        float2 acc[8][4];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[j][c] = make_float2(0.f, 0.f);
-        for (int want = kStarWide; want <= (COV ? kStarMid : kStarWide); ++want)
-            for (int q0 = 0; q0 < n; q0 += kStampThreads) {
-                const int nw = list_chunk(S, st, s0, n, q0, g, cov, ty0, ty0 + tyn - 1, want);
-                for (int b0 = 0; b0 < nw; b0 += kBatch) {
-                    const int nb = min(kBatch, nw - b0);
-                    const int k = threadIdx.x >> 4, e = threadIdx.x & 15;
-                    if (b0) __syncthreads();  // the previous batch is done with its records
-                    if (k < nb && e == 0) load_record(S.rec[k], st, s0 + S.list[b0 + k], g, cov);
-                    __syncthreads();
-                    if (COV) {
-                        if (k < nb) {
-                            const float dj = (float)(e >> 1) - kTileMid;
-                            const float c = -2.f * S.rec[k].p[0] * S.rec[k].p[1] * dj;
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                S.T[k][4 * e + i] = ex2f(c * ((float)((e & 1) * 4 + i) - kTileMid));
-                        }
-                        __syncthreads();
-                    }
-                    if (sg < ns && pass + tg0 < ntg)
-                        for (int k2 = sg; k2 < nb; k2 += ns) {
-                            if (!COV || want == kStarWide)
-                                wide_tile<COV>(acc, S.rec[k2], S.T[k2], col0, row0, live);
-                            else
-                                mid_tile(acc, S.rec[k2], S.T[k2], col0, row0, live);
-                        }
-                }
-            }
-        if (live) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (row0 + j - ty0 >= tyn) break;
-                float *row = band + (int64_t)(row0 + j - ty0) * g.nx + col0;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    if (col0 + 2 * c < g.nx) atomicAdd(row + 2 * c, acc[j][c].x);
-                    if (col0 + 2 * c + 1 < g.nx) atomicAdd(row + 2 * c + 1, acc[j][c].y);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < bandn; k += kStampThreads) dst[k] = band[k];
-}
-
-__global__ void __launch_bounds__(kStampThreads, 2)
-k_stamps(StampStars st, Grid2 g, int TY, float *__restrict__ out) {
-    extern __shared__ float smem[];
-    __shared__ StampShared S;
-    const int t = blockIdx.y, ty0 = blockIdx.x * TY;
-    float *dst = out + (int64_t)t * ((int64_t)g.nx * g.ny) + (int64_t)ty0 * g.nx;
-    if (st.cov[t] != 0) stamp_band<true>(smem, S, st, t, g, ty0, TY, dst);
-    else stamp_band<false>(smem, S, st, t, g, ty0, TY, dst);
-}
-
-// One band of one template per CTA from a flattened tile list: templates with their own
-// Hess grids (ragged galaxies).
-struct StampTile {
-    int32_t t, ty0, ty;  // template, first row, band height of this template
+struct WarpStars {
+    StarRec rec[32];  // the warp's current stars
+    float T[64];      // and shear table
 };
 
-__global__ void __launch_bounds__(kStampThreads, 2)
-k_stamps_ragged(StampStars st, const StampTile *__restrict__ tiles,
-                const Grid2 *__restrict__ grids, const int64_t *__restrict__ out_off,
-                float *__restrict__ out) {
+// A warp's walk through a template's stars (first star s0, n of them), of which it takes sg,
+// sg + ns, ...: 32 at a time, one per lane, those wanted are compacted into its slots in
+// order.  Wanted: wide or mid, with a window that reaches rows ty0 .. ty1; of the wide stars
+// those that have (NODES) or lack (else) one of the strips.
+template <bool NODES, bool REC>
+__device__ __forceinline__ int next_stars(StarRec *slot, const StampStars &st, int64_t s0, int n,
+                                          int q0, int sg, int ns, const Grid2 &g, int cov, int ty0,
+                                          int ty1, unsigned long long strips) {
+    const int lane = threadIdx.x & 31, q = (q0 + lane) * ns + sg;
+    bool take = false;
+    StarRec tmp;
+    const StarRec *r = &tmp;
+    if (q < n) {
+        if (REC) r = st.rec + s0 + q;
+        else star_record(tmp, g, st.x[s0 + q], st.y[s0 + q], st.sx[s0 + q], st.sy[s0 + q], st.w[s0 + q], cov);
+        take = (r->cls == kStarWide || (!NODES && r->cls == kStarMid)) && r->ylo <= ty1 && r->yhi >= ty0;
+        if (take && r->cls == kStarWide)
+            take = ((NODES ? star_strips(*r) : ~star_strips(*r)) & strips) != 0ull;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (take) {
+        const float4 *from = reinterpret_cast<const float4 *>(r);
+        float4 *to = reinterpret_cast<float4 *>(slot + __popc(m & ((1u << lane) - 1u)));
+#pragma unroll
+        for (int k = 0; k < (int)(sizeof(StarRec) / sizeof(float4)); ++k) to[k] = from[k];
+    }
+    __syncwarp();
+    return __popc(m);
+}
+
+// Adds the warp's wide (and mid) stars to the lane's tile.  The warp makes each star's shear
+// table, two entries a lane.
+template <bool COV, bool NODES, bool REC>
+__device__ __forceinline__ void add_stars(float2 (&acc)[8][4], WarpStars &W, const StampStars &st,
+                                          int64_t s0, int n, int sg, int ns, const Grid2 &g, int cov,
+                                          int ty0, int ty1, unsigned long long strips, const Tile &tl) {
+    float *T = W.T;
+    // lane: row l / 4 of T, columns 2 (l % 4) and the next; nodes are odd about the middle
+    const int lane = threadIdx.x & 31, jr = lane >> 2, jp = jr < 4 ? 3 - jr : jr - 4, ic = lane & 3;
+    float tj = jp == 0 ? tile_node(NODES, 4) : jp == 1 ? tile_node(NODES, 5)
+               : jp == 2 ? tile_node(NODES, 6) : tile_node(NODES, 7);
+    if (jr < 4) tj = -tj;
+    if (NODES) tj *= tl.xh * tl.yh;
+    const float ti0 = ic == 0 ? tile_node(NODES, 0) : ic == 1 ? tile_node(NODES, 2)
+                      : ic == 2 ? tile_node(NODES, 4) : tile_node(NODES, 6);
+    const float ti1 = ic == 0 ? tile_node(NODES, 1) : ic == 1 ? tile_node(NODES, 3)
+                      : ic == 2 ? tile_node(NODES, 5) : tile_node(NODES, 7);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[j][c] = make_float2(0.f, 0.f);
+    for (int q0 = 0; q0 * ns + sg < n; q0 += 32) {
+        const int nw = next_stars<NODES, REC>(W.rec, st, s0, n, q0, sg, ns, g, cov, ty0, ty1, strips);
+#pragma unroll 1
+        for (int k = 0; k < nw; ++k) {
+            const StarRec &r = W.rec[k];
+            if (COV) {
+                const float c = -2.f * r.p[0] * r.p[1] * tj;
+                const float2 t = make_float2(ex2f(c * ti0), ex2f(c * ti1));
+                __syncwarp();  // the previous star's table is no longer read
+                *reinterpret_cast<float2 *>(T + 2 * lane) = t;
+                __syncwarp();
+            }
+            if (COV && !NODES && r.cls == kStarMid) mid_tile(acc, r, T, tl);
+            else wide_tile<COV, NODES>(acc, r, T, tl);
+        }
+        __syncwarp();  // the slots are done with
+    }
+}
+
+// Sums the warps' accumulators in warp order into sum[value][lane] (8 KB).
+__device__ __forceinline__ void sum_warps(float *sum, const float2 (&acc)[8][4], int warps) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int w = 0; w < warps; ++w) {
+        if (w == warp) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float *v = sum + (8 * j + 2 * c) * 32 + lane;
+                    v[0] = w ? v[0] + acc[j][c].x : acc[j][c].x;
+                    v[32] = w ? v[32] + acc[j][c].y : acc[j][c].y;
+                }
+        }
+        __syncthreads();
+    }
+}
+
+// The 8 Chebyshev-node Lagrange weights at x in (-1, 1), nodes ascending:
+// (1 + 2 sum_k T_k(c_m) T_k(x)) / 8.
+__device__ __forceinline__ void lagrange8(float x, float (&L)[8]) {
+    constexpr float c16[9] = {1.f, 0.9807852804032304f, 0.9238795325112867f, 0.8314696123025452f,
+                              0.7071067811865476f, 0.5555702330196022f, 0.3826834323650898f,
+                              0.19509032201612825f, 0.f};
+    float T[8];
+    T[0] = 1.f;
+    T[1] = x;
+#pragma unroll
+    for (int k = 2; k < 8; ++k) T[k] = fmaf(2.f * x, T[k - 1], -T[k - 2]);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        float a = 0.125f;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) {
+            const int n = (k * (2 * (7 - m) + 1)) & 31;  // T_k(c_m) = cos(n pi / 16)
+            const int f = n <= 16 ? n : 32 - n;
+            a = fmaf(0.25f * (f <= 8 ? c16[f] : -c16[16 - f]), T[k], a);
+        }
+        L[m] = a;
+    }
+}
+
+// Grid: x -> group of 32 Chebyshev tiles, y -> template; the CTA's warps share the stars.
+// node: the tiles' 64 values each, rows of 8.  Most updates come from stars far below the
+// detection limit whose errors span the whole diagram (of 5.6e10 updates of the 1,200-template
+// build about seven eighths): on these tiles 64 values stand for 640 bins.
+__global__ void __launch_bounds__(kNodeWarps * 32, 2)
+k_stamp_nodes(StampStars st, Grid2 g0, const Grid2 *__restrict__ grids,
+              const int64_t *__restrict__ node_off, int t0, float *__restrict__ node) {
+    __shared__ __align__(16) WarpStars W[kNodeWarps];
+    __shared__ float sum[2048];
+    const int t = t0 + blockIdx.y, group = blockIdx.x;
+    const Grid2 g = grids ? grids[t] : g0;
+    const Smooth sm = smooth_tiling(g, true);
+    if (!sm.on || group >= sm.groups()) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = group * 32 + lane, last = min(group * 32 + 31, sm.tiles() - 1);
+    Tile tl{};
+    tl.live = tile <= last;
+    tl.strip = min(tile, last) / sm.nwc;
+    tl.xh = 0.5f * (float)sm.wx;
+    tl.yh = 0.5f * (float)sm.wy;
+    tl.xc = (float)((tile % sm.nwc) * sm.wx) + tl.xh - 0.5f;
+    tl.yc = (float)(tl.strip * sm.wy) + tl.yh - 0.5f;
+    const int sa = group * 32 / sm.nwc, sb = last / sm.nwc, cov = st.cov[t];
+    float2 acc[8][4];
+    if (cov != 0)
+        add_stars<true, true, true>(acc, W[warp], st, st.start[t], st.count[t], warp, kNodeWarps, g, cov,
+                                    sa * sm.wy, (sb + 1) * sm.wy - 1, strip_bits(sa, sb), tl);
+    else
+        add_stars<false, true, true>(acc, W[warp], st, st.start[t], st.count[t], warp, kNodeWarps, g, cov,
+                                     sa * sm.wy, (sb + 1) * sm.wy - 1, strip_bits(sa, sb), tl);
+    sum_warps(sum, acc, kNodeWarps);
+    float *out = node + (node_off ? node_off[t] : (int64_t)t * 64 * sm.tiles()) + (int64_t)group * 2048;
+    for (int k = threadIdx.x; k < 64 * (last - group * 32 + 1); k += kNodeWarps * 32)
+        out[k] = sum[(k & 63) * 32 + (k >> 6)];
+}
+
+// One group of 32 tiles of one template per CTA; its ns warps share the stars.  Adds the
+// interpolated node values and writes the tiles.
+struct StampGroup {
+    int32_t t, group;
+};
+
+__host__ __device__ inline int tile_groups(int64_t nx, int64_t ny) {
+    return (int)((((nx + 7) / 8) * ((ny + 7) / 8) + 31) / 32);
+}
+
+template <bool REC>
+__global__ void __launch_bounds__(kTileWarpsMax * 32, 1)
+k_stamp_tiles(StampStars st, Grid2 g0, const StampGroup *__restrict__ groups,
+              const Grid2 *__restrict__ grids, const int64_t *__restrict__ out_off,
+              const int64_t *__restrict__ node_off, const float *__restrict__ node,
+              float *__restrict__ out) {
+    extern __shared__ __align__(16) float smem[];  // [2048] node rows, [ns > 1: 2048] sums, warps
+    const int ns = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const StampGroup gr = groups ? groups[blockIdx.x] : StampGroup{(int)blockIdx.y, (int)blockIdx.x};
+    const int t = gr.t, cov = st.cov[t];
+    const Grid2 g = grids ? grids[t] : g0;
+    float *mid = smem, *sum = smem + 2048;
+    WarpStars &W = reinterpret_cast<WarpStars *>(smem + (ns > 1 ? 4096 : 2048))[warp];
+    const Smooth sm = smooth_tiling(g, node != nullptr);
+    const int ntc = (g.nx + 7) >> 3, ntiles = ntc * ((g.ny + 7) >> 3);
+    const int tile = gr.group * 32 + lane, last = min(gr.group * 32 + 31, ntiles - 1);
+    Tile tl{};
+    tl.live = tile <= last;
+    tl.col0 = (tile % ntc) * 8;
+    tl.row0 = (tile / ntc) * 8;
+    tl.strip = tl.live ? tl.row0 / sm.wy : 0;
+    const int wa = gr.group * 32 / ntc * 8, wb = min(last / ntc * 8 + 7, g.ny - 1);
+    const unsigned long long strips = strip_bits(wa / sm.wy, wb / sm.wy);
+    float2 acc[8][4];
+    if (cov != 0)
+        add_stars<true, false, REC>(acc, W, st, st.start[t], st.count[t], warp, ns, g, cov, wa, wb, strips, tl);
+    else
+        add_stars<false, false, REC>(acc, W, st, st.start[t], st.count[t], warp, ns, g, cov, wa, wb, strips, tl);
+    if (ns > 1) sum_warps(sum, acc, ns);
+    if (sm.on) {
+        // the tile's 8 columns of its Chebyshev tile's 8 node rows: mid[8 n + i][lane]
+        const float *f = node + (node_off ? node_off[t] : (int64_t)t * 64 * sm.tiles()) +
+                         64 * (tl.live ? tl.strip * sm.nwc + tl.col0 / sm.wx : 0);
+        const float xh = 0.5f * (float)sm.wx;
+        for (int i = warp; i < 8; i += ns) {
+            float L[8];
+            lagrange8(((float)(tl.col0 % sm.wx + i) + 0.5f - xh) / xh, L);
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(f + 8 * n));
+                const float4 c = __ldg(reinterpret_cast<const float4 *>(f + 8 * n + 4));
+                mid[(8 * n + i) * 32 + lane] =
+                    fmaf(L[0], a.x, fmaf(L[1], a.y, fmaf(L[2], a.z, fmaf(L[3], a.w,
+                    fmaf(L[4], c.x, fmaf(L[5], c.y, fmaf(L[6], c.z, L[7] * c.w)))))));
+            }
+        }
+        if (ns > 1) __syncthreads();
+        else __syncwarp();
+    }
+    if (!tl.live) return;
+    float *dst = out + (out_off ? out_off[t] : (int64_t)t * g.nx * g.ny) + (int64_t)tl.row0 * g.nx + tl.col0;
+    const bool wide = (g.nx & 7) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if ((ns > 1 && j % ns != warp) || tl.row0 + j >= g.ny) continue;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[i] = ns > 1 ? sum[(8 * j + i) * 32 + lane] : i & 1 ? acc[j][i >> 1].y : acc[j][i >> 1].x;
+        if (sm.on) {
+            const float yh = 0.5f * (float)sm.wy;
+            float L[8];
+            lagrange8(((float)(tl.row0 % sm.wy + j) + 0.5f - yh) / yh, L);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float a = 0.f;
+#pragma unroll
+                for (int n = 0; n < 8; ++n) a = fmaf(L[n], mid[(8 * n + i) * 32 + lane], a);
+                v[i] += a;
+            }
+        }
+        float *row = dst + (int64_t)j * g.nx;
+        if (wide) {
+            reinterpret_cast<float4 *>(row)[0] = make_float4(v[0], v[1], v[2], v[3]);
+            reinterpret_cast<float4 *>(row)[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (tl.col0 + i < g.nx) row[i] = v[i];
+        }
+    }
+}
+
+// The narrow stars of all templates (REC: from k_star_prep's list, dealt out star by star; else
+// grid y -> template, every star looked at), added to the templates.
+template <bool REC>
+__global__ void __launch_bounds__(kNarrowWarps * 32)
+k_stamp_narrow(StampStars st, Grid2 g0, const Grid2 *__restrict__ grids,
+               const int64_t *__restrict__ out_off, const StarId *__restrict__ narrow,
+               const int *__restrict__ n_narrow, int buf, float *__restrict__ out) {
     extern __shared__ float smem[];
-    __shared__ StampShared S;
-    const StampTile tile = tiles[blockIdx.x];
-    const Grid2 g = grids[tile.t];
-    float *dst = out + out_off[tile.t] + (int64_t)tile.ty0 * g.nx;
-    if (st.cov[tile.t] != 0) stamp_band<true>(smem, S, st, tile.t, g, tile.ty0, tile.ty, dst);
-    else stamp_band<false>(smem, S, st, tile.t, g, tile.ty0, tile.ty, dst);
+    __shared__ __align__(16) StarRec s_rec[kNarrowWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float *bx_buf = smem + (size_t)warp * buf, *by_buf = bx_buf + buf - kNarrowRows;
+    const int n = REC ? *n_narrow : st.count[blockIdx.y];
+    for (int k = blockIdx.x * kNarrowWarps + warp; k < n; k += gridDim.x * kNarrowWarps) {
+        const StarId id = REC ? narrow[k] : StarId{(int)blockIdx.y, k};
+        const Grid2 g = grids ? grids[id.t] : g0;
+        const int64_t s = st.start[id.t] + id.q;
+        __syncwarp();  // the previous star is done with
+        if (REC) {
+            if (lane < (int)(sizeof(StarRec) / 4))
+                reinterpret_cast<int *>(&s_rec[warp])[lane] = reinterpret_cast<const int *>(st.rec + s)[lane];
+        } else if (lane == 0) {
+            StarRec r;
+            star_record(r, g, st.x[s], st.y[s], st.sx[s], st.sy[s], st.w[s], st.cov[id.t]);
+            s_rec[warp] = r;
+        }
+        __syncwarp();
+        const StarRec &r = s_rec[warp];
+        if (!REC && r.cls != kStarNarrow) continue;
+        float *dst = out + (out_off ? out_off[id.t] : (int64_t)id.t * g.nx * g.ny);
+        if (r.cov != 0) star_cov(dst, r, g.nx, lane);
+        else star_asym(dst, bx_buf, by_buf, r, g.nx, lane);
+    }
 }
 
 __global__ void k_offsets_to_counts(const int64_t *__restrict__ off, int64_t n,
@@ -874,80 +1126,113 @@ k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
     }
 }
 
-// Dynamic shared memory of one stamp CTA: the FP32 band (TY x nx) plus per-warp buffers of
-// the narrow stars (nx + TY floats: the x/y factor tables of the separable kernel).
-size_t stamp_smem(int64_t nx, int64_t TY) {
-    return ((size_t)TY * nx + (size_t)kWarps * (nx + TY)) * sizeof(float);
+// The widest accepted grid: a separable narrow star's x table of four warps in shared memory.
+constexpr int64_t kMaxColumns = 3123;
+
+// Warps per tile group: as many as the stars can be dealt to while all groups together stay
+// within four waves of 16 warps (128 registers) per SM: a group in the dense part of a diagram takes
+// several times the mean, and one warp of it would be the tail (60 binary templates: 1.50 ms with
+// one warp per group, 0.59 ms with four).
+int tile_warps(int64_t groups, int sm_count) {
+    int ns = 1;
+    while (ns < kTileWarpsMax && groups * 2 * ns <= 64 * (int64_t)sm_count) ns *= 2;
+    return ns;
 }
 
-// The widest accepted grid, 3,123 columns: its one tile row takes 201 KB.
-bool stamp_grid_ok(int64_t nx) { return nx <= 3123; }
+size_t tile_smem(int ns) { return (ns > 1 ? 16384 : 8192) + ns * sizeof(WarpStars); }
 
-// Rows per band (a multiple of the 8-row tile): the number of tile rows with the least
-// estimated time.  A CTA of 8 warps takes one unit per 8 groups of 32 tiles; with fewer
-// groups the warps share the stars of each group, so a band of 5 tiles costs an eighth of a
-// unit even though 27 of 32 lanes idle: few templates get short bands, many get full ones.
-// 0.15 units stand for staging the star list.  Two CTAs per SM (registers, kBandBudget);
-// one row of tiles is always taken, whatever its shared memory.
-int band_rows(int64_t nx, int64_t ny, int64_t ntempl, int sm_count) {
-    const int64_t ntc = (nx + 7) / 8, ntr = (ny + 7) / 8;
-    int64_t best = 1;
-    double best_cost = 0.0;
-    for (int64_t R = 1; R <= ntr; ++R) {
-        if (R > 1 && stamp_smem(nx, 8 * R) + sizeof(StampShared) > kBandBudget) break;
-        const int64_t bands = (ntr + R - 1) / R;
-        if (R > 1 && bands == (ntr + R - 2) / (R - 1)) continue;  // same bands, less even
-        const int64_t ntg = (ntc * R + 31) / 32;
-        const double unit = ntg >= kWarps ? (double)((ntg + kWarps - 1) / kWarps)
-                                          : 1.0 / (double)(kWarps / ntg);
-        const int64_t slots = 2 * (int64_t)sm_count;
-        const double waves = (double)((ntempl * bands + slots - 1) / slots);
-        const double cost = waves * (unit + 0.15);
-        if (R == 1 || cost < best_cost * 0.999) {
-            best = R;
-            best_cost = cost;
-        }
+// Bytes of the node values of ntempl templates on one grid.
+size_t node_bytes(const Grid2 &g, int64_t ntempl) {
+    const Smooth sm = smooth_tiling(g, true);
+    return sm.on ? (size_t)ntempl * 64 * sm.tiles() * sizeof(float) : 0;
+}
+
+// Device workspace of the stamps, where the star counts are known to the host.
+struct StampWork {
+    StarRec *rec = nullptr;    // one per star, indexed as the star arrays
+    StarId *narrow = nullptr;  // room for every star
+    int *n_narrow = nullptr;
+    float *node = nullptr;     // node_bytes() / the ragged batch's nodes
+    int64_t maxcount = 0;      // largest star count of a template
+    static size_t bytes(int64_t stars, size_t node) {
+        const size_t n = (size_t)std::max<int64_t>(stars, 1);
+        return 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarId)) + sfh_align256(node);
     }
-    return (int)(8 * best);
-}
+    StampWork() = default;
+    StampWork(char *b, int64_t stars, int64_t maxcount_) : maxcount(maxcount_) {
+        const size_t n = (size_t)std::max<int64_t>(stars, 1);
+        n_narrow = (int *)b;
+        rec = (StarRec *)(b + 256);
+        narrow = (StarId *)(b + 256 + sfh_align256(n * sizeof(StarRec)));
+        node = (float *)(b + 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarId)));
+    }
+};
 
-int stamp_attributes(sfh_ctx *ctx) {
+// Per-template grids of a ragged batch on the device.
+struct StampGrids {
+    const Grid2 *grids;
+    const int64_t *out_off, *node_off;
+    const StampGroup *groups;
+    int64_t ngroups;
+    int max_node_groups;
+    int64_t max_nx;
+};
+
+// Stamps of ntempl templates, on one grid g or (rg) each on its own.  Without work->rec (the
+// caller does not know the star counts) every kernel makes the records it needs and no strips
+// are smooth.
+int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const StampGrids *rg,
+                  const StampWork &w, float *d_out) {
+    const int64_t nx = rg ? rg->max_nx : g.nx;
+    if (!rg && (g.nx < 1 || g.ny < 1 || g.nx > (1 << 20) || g.ny > (1 << 20) || ntempl < 1 || ntempl > 65535))
+        return sfh_set_error(ctx, SFH_ERR_ARG, "stamp grid or template count out of range");
+    if (nx > kMaxColumns)
+        return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
+    const bool have = w.rec != nullptr;
+    st.rec = w.rec;
+    const Smooth sm = smooth_tiling(g, have && !rg);
+    const int node_groups = rg ? rg->max_node_groups : sm.on ? sm.groups() : 0;
+    cudaStream_t s = ctx->stream;
     static thread_local bool attr_set = false;
     if (!attr_set) {
-        SFH_CK(ctx, cudaFuncSetAttribute(k_stamps, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         216 * 1024));
-        SFH_CK(ctx, cudaFuncSetAttribute(k_stamps_ragged,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
+        for (auto k : {k_stamp_tiles<true>, k_stamp_tiles<false>})
+            SFH_CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)tile_smem(kTileWarpsMax)));
+        for (auto k : {k_stamp_narrow<true>, k_stamp_narrow<false>})
+            SFH_CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(kNarrowWarps * (kMaxColumns + kNarrowRows) * 4)));
         attr_set = true;
     }
-    return SFH_OK;
-}
-
-// Stamps of ntempl templates on one grid.  d_rec: room for one record per star (indexed as
-// the star arrays) with maxcount the largest star count, or NULL when the caller does not
-// know the counts: the records are then made by each band.
-int launch_stamps(sfh_ctx *ctx, const double *d_x, const double *d_y, const double *d_sx,
-                  const double *d_sy, const double *d_w, const int64_t *d_start,
-                  const int32_t *d_count, const int32_t *d_cov, int64_t ntempl, double xf,
-                  double xs, int64_t nx, double yf, double ys, int64_t ny, float *d_out,
-                  StarRec *d_rec, int64_t maxcount) {
-    if (nx < 1 || ny < 1 || nx > (1 << 20) || ny > (1 << 20) || ntempl < 1 || ntempl > 65535)
-        return sfh_set_error(ctx, SFH_ERR_ARG, "stamp grid or template count out of range");
-    if (!stamp_grid_ok(nx))
-        return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
-    int rc = stamp_attributes(ctx);
-    if (rc) return rc;
-    const int TY = band_rows(nx, ny, ntempl, ctx->sm_count);
-    Grid2 g{xf, xs, yf, ys, (int)nx, (int)ny};
-    if (d_rec && maxcount > 0) {
-        k_star_prep<<<dim3((unsigned)((maxcount + kPrepThreads - 1) / kPrepThreads), (unsigned)ntempl),
-                      kPrepThreads, 0, ctx->stream>>>(d_x, d_y, d_sx, d_sy, d_w, d_start, d_count,
-                                                      d_cov, g, nullptr, 0, d_rec);
-        SFH_LAUNCHED(ctx);
+    if (have) SFH_CK(ctx, cudaMemsetAsync(w.n_narrow, 0, sizeof(int), s));
+    for (int64_t t0 = 0; have && t0 < ntempl; t0 += 65535) {
+        const unsigned nt = (unsigned)std::min<int64_t>(65535, ntempl - t0);
+        if (w.maxcount > 0) {
+            k_star_prep<<<dim3((unsigned)((w.maxcount + kPrepThreads - 1) / kPrepThreads), nt),
+                          kPrepThreads, 0, s>>>(st.x, st.y, st.sx, st.sy, st.w, st.start, st.count,
+                                                st.cov, g, rg ? rg->grids : nullptr, (int)t0, w.rec,
+                                                w.narrow, w.n_narrow);
+            SFH_LAUNCHED(ctx);
+        }
+        if (node_groups > 0) {
+            k_stamp_nodes<<<dim3((unsigned)node_groups, nt), kNodeWarps * 32, 0, s>>>(
+                st, g, rg ? rg->grids : nullptr, rg ? rg->node_off : nullptr, (int)t0, w.node);
+            SFH_LAUNCHED(ctx);
+        }
     }
-    dim3 grid((unsigned)((ny + TY - 1) / TY), (unsigned)ntempl);
-    k_stamps<<<grid, kStampThreads, stamp_smem(nx, TY), ctx->stream>>>(
-        StampStars{d_x, d_y, d_sx, d_sy, d_w, d_rec, d_start, d_count, d_cov}, g, TY, d_out);
+    const int64_t groups = rg ? rg->ngroups : ntempl * tile_groups(g.nx, g.ny);
+    const int ns = tile_warps(groups, ctx->sm_count);
+    const dim3 grid = rg ? dim3((unsigned)groups) : dim3((unsigned)tile_groups(g.nx, g.ny), (unsigned)ntempl);
+    auto tiles = have ? k_stamp_tiles<true> : k_stamp_tiles<false>;
+    tiles<<<grid, 32 * ns, tile_smem(ns), s>>>(st, g, rg ? rg->groups : nullptr, rg ? rg->grids : nullptr,
+                                               rg ? rg->out_off : nullptr, rg ? rg->node_off : nullptr,
+                                               node_groups > 0 ? w.node : nullptr, d_out);
+    SFH_LAUNCHED(ctx);
+    const int buf = (int)nx + kNarrowRows;
+    const unsigned blocks = 8u * (unsigned)ctx->sm_count;
+    const dim3 ngrid = have ? dim3(blocks) : dim3(std::max(1u, blocks / (unsigned)ntempl), (unsigned)ntempl);
+    auto narrow = have ? k_stamp_narrow<true> : k_stamp_narrow<false>;
+    narrow<<<ngrid, kNarrowWarps * 32, kNarrowWarps * buf * sizeof(float), s>>>(
+        st, g, rg ? rg->grids : nullptr, rg ? rg->out_off : nullptr, w.narrow, w.n_narrow, buf, d_out);
     SFH_LAUNCHED(ctx);
     return SFH_OK;
 }
@@ -975,8 +1260,9 @@ extern "C" int sfh_bin_cmd_smooth_batch_dev(sfh_ctx *ctx, const double *d_x, con
     k_offsets_to_counts<<<(int)((ntempl + 255) / 256), 256, 0, ctx->stream>>>(d_offsets, ntempl,
                                                                                 d_cnt);
     SFH_LAUNCHED(ctx);
-    return launch_stamps(ctx, d_x, d_y, d_sx, d_sy, d_w, d_offsets, d_cnt, d_cov, ntempl, xf, xs,
-                         nx, yf, ys, ny, d_models, nullptr, 0);
+    const Grid2 g{xf, xs, yf, ys, (int)std::min<int64_t>(nx, INT32_MAX), (int)std::min<int64_t>(ny, INT32_MAX)};
+    return launch_stamps(ctx, StampStars{d_x, d_y, d_sx, d_sy, d_w, nullptr, d_offsets, d_cnt, d_cov},
+                         ntempl, g, nullptr, StampWork(), d_models);
 }
 
 extern "C" int sfh_bin_cmd_smooth(sfh_ctx *ctx, const double *x, const double *y,
@@ -993,8 +1279,11 @@ extern "C" int sfh_bin_cmd_smooth(sfh_ctx *ctx, const double *x, const double *y
     SFH_CK(ctx, cudaSetDevice(ctx->device));
     const int64_t nbins = nx * ny;
     const size_t a5 = sfh_align256((size_t)(npts > 0 ? npts : 1) * 8);
-    const size_t o_out = 5 * a5, o_meta = o_out + sfh_align256(nbins * 4), o_rec = o_meta + 256;
-    int rc = sfh_stage_reserve(ctx, o_rec + (size_t)(npts > 0 ? npts : 1) * sizeof(StarRec));
+    const size_t o_out = 5 * a5, o_meta = o_out + sfh_align256(nbins * 4), o_work = o_meta + 256;
+    if (nx > (1 << 20) || ny > (1 << 20))
+        return sfh_set_error(ctx, SFH_ERR_ARG, "stamp grid or template count out of range");
+    const Grid2 g{xf, xs, yf, ys, (int)nx, (int)ny};
+    int rc = sfh_stage_reserve(ctx, o_work + StampWork::bytes(npts, node_bytes(g, 1)));
     if (rc) return rc;
     char *b = (char *)ctx->stage;
     const double *src[5] = {x, y, sx, sy, w};
@@ -1003,11 +1292,12 @@ extern "C" int sfh_bin_cmd_smooth(sfh_ctx *ctx, const double *x, const double *y
     struct { int64_t start; int32_t count; int32_t cov; } meta{0, (int32_t)npts, cov_mult};
     SFH_CK(ctx, cudaMemcpyAsync(b + o_meta, &meta, sizeof(meta), cudaMemcpyHostToDevice, ctx->stream));
     float *d_out = (float *)(b + o_out);
-    rc = launch_stamps(ctx, (const double *)b, (const double *)(b + a5),
-                       (const double *)(b + 2 * a5), (const double *)(b + 3 * a5),
-                       (const double *)(b + 4 * a5), (const int64_t *)(b + o_meta),
-                       (const int32_t *)(b + o_meta + 8), (const int32_t *)(b + o_meta + 12), 1, xf,
-                       xs, nx, yf, ys, ny, d_out, (StarRec *)(b + o_rec), npts);
+    rc = launch_stamps(ctx, StampStars{(const double *)b, (const double *)(b + a5),
+                                       (const double *)(b + 2 * a5), (const double *)(b + 3 * a5),
+                                       (const double *)(b + 4 * a5), nullptr,
+                                       (const int64_t *)(b + o_meta), (const int32_t *)(b + o_meta + 8),
+                                       (const int32_t *)(b + o_meta + 12)},
+                       1, g, nullptr, StampWork(b + o_work, npts, npts), d_out);
     if (rc) return rc;
     std::vector<float> tmp((size_t)nbins);
     SFH_CK(ctx, cudaMemcpyAsync(tmp.data(), d_out, nbins * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1084,10 +1374,12 @@ namespace {
 // Host-side description of per-template Hess grids (ragged galaxies).
 struct RaggedSpec {
     std::vector<Grid2> grids;
-    std::vector<int64_t> out_off;
+    std::vector<int64_t> out_off, node_off;
+    int64_t nodes = 0;   // node values of all templates
+    int max_node_groups = 0;  // largest template's groups of 32 Chebyshev tiles
     std::vector<double> dmag;
-    std::vector<StampTile> tiles;
-    size_t smem = 0;
+    std::vector<StampGroup> groups;  // every template's groups of 32 tiles
+    int64_t max_nx = 0;
 };
 
 // The two device passes of partial_cmd_smooth for a batch of isochrones (resampled star
@@ -1136,11 +1428,15 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     const int64_t nstar_total = soff[(size_t)ntempl] > 0 ? soff[(size_t)ntempl] : 1;
     // Pass 2: star records, then the stamps.
     const size_t a8 = sfh_align256((size_t)nstar_total * 8);
-    const size_t o_rec = o_stars + 5 * a8;
-    const size_t o_grid = o_rec + (size_t)nstar_total * sizeof(StarRec);
+    const Grid2 g{xf, xs, yf, ys, (int)std::min<int64_t>(nx, INT32_MAX), (int)std::min<int64_t>(ny, INT32_MAX)};
+    const size_t nodes = rg ? (size_t)rg->nodes * sizeof(float)
+                            : nx <= kMaxColumns && ny <= (1 << 20) ? node_bytes(g, ntempl) : 0;
+    const size_t o_work = o_stars + 5 * a8;
+    const size_t o_grid = o_work + StampWork::bytes(nstar_total, nodes);
     const size_t o_oof = o_grid + (rg ? sfh_align256(ntempl * sizeof(Grid2)) : 0);
-    const size_t o_tiles = o_oof + (rg ? sfh_align256(ntempl * 8) : 0);
-    const size_t o_end = o_tiles + (rg ? sfh_align256(rg->tiles.size() * sizeof(StampTile)) : 0);
+    const size_t o_noff = o_oof + (rg ? sfh_align256(ntempl * 8) : 0);
+    const size_t o_tiles = o_noff + (rg ? sfh_align256(ntempl * 8) : 0);
+    const size_t o_end = o_tiles + (rg ? sfh_align256(rg->groups.size() * sizeof(StampGroup)) : 0);
     rc = sfh_scratch_reserve(ctx, o_end);
     if (rc) return rc;
     b = (char *)ctx->scratch;  // may have moved
@@ -1158,7 +1454,8 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
         SFH_CK(ctx, cudaMemcpyAsync(b + o_grid, rg->grids.data(), ntempl * sizeof(Grid2),
                                     cudaMemcpyHostToDevice, st));
         SFH_CK(ctx, cudaMemcpyAsync(b + o_oof, rg->out_off.data(), ntempl * 8, cudaMemcpyHostToDevice, st));
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_tiles, rg->tiles.data(), rg->tiles.size() * sizeof(StampTile),
+        SFH_CK(ctx, cudaMemcpyAsync(b + o_noff, rg->node_off.data(), ntempl * 8, cudaMemcpyHostToDevice, st));
+        SFH_CK(ctx, cudaMemcpyAsync(b + o_tiles, rg->groups.data(), rg->groups.size() * sizeof(StampGroup),
                                     cudaMemcpyHostToDevice, st));
     }
     double *sxp = (double *)(b + o_stars), *syp = (double *)(b + o_stars + a8);
@@ -1170,28 +1467,16 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
         (const int64_t *)(b + o_soff), sxp, syp, ssxp, ssyp, swp, (int32_t *)(b + o_cnt),
         (int *)(b + o_err));
     SFH_LAUNCHED(ctx);
-    if (rg) {
-        if ((rc = stamp_attributes(ctx))) return rc;
-        const Grid2 *d_grids = (const Grid2 *)(b + o_grid);
-        StarRec *rec = (StarRec *)(b + o_rec);
-        const StampStars ss{sxp, syp, ssxp, ssyp, swp, rec, (const int64_t *)(b + o_soff),
-                            (const int32_t *)(b + o_cnt), (const int32_t *)(b + o_cov)};
-        for (int64_t t0 = 0; t0 < ntempl && maxcount > 0; t0 += 65535) {
-            k_star_prep<<<dim3((unsigned)((maxcount + kPrepThreads - 1) / kPrepThreads),
-                               (unsigned)std::min<int64_t>(65535, ntempl - t0)),
-                          kPrepThreads, 0, st>>>(sxp, syp, ssxp, ssyp, swp, ss.start, ss.count,
-                                                 ss.cov, Grid2{}, d_grids, (int)t0, rec);
-            SFH_LAUNCHED(ctx);
-        }
-        k_stamps_ragged<<<(unsigned)rg->tiles.size(), kStampThreads, rg->smem, st>>>(
-            ss, (const StampTile *)(b + o_tiles), d_grids, (const int64_t *)(b + o_oof), d_models);
-        SFH_LAUNCHED(ctx);
-    } else {
-        rc = launch_stamps(ctx, sxp, syp, ssxp, ssyp, swp, (const int64_t *)(b + o_soff),
-                           (const int32_t *)(b + o_cnt), (const int32_t *)(b + o_cov), ntempl, xf,
-                           xs, nx, yf, ys, ny, d_models, (StarRec *)(b + o_rec), maxcount);
-        if (rc) return rc;
-    }
+    StampGrids sg{};
+    if (rg)
+        sg = StampGrids{(const Grid2 *)(b + o_grid), (const int64_t *)(b + o_oof),
+                        (const int64_t *)(b + o_noff), (const StampGroup *)(b + o_tiles),
+                        (int64_t)rg->groups.size(), rg->max_node_groups, rg->max_nx};
+    rc = launch_stamps(ctx, StampStars{sxp, syp, ssxp, ssyp, swp, nullptr, (const int64_t *)(b + o_soff),
+                                       (const int32_t *)(b + o_cnt), (const int32_t *)(b + o_cov)},
+                       ntempl, g, rg ? &sg : nullptr, StampWork(b + o_work, nstar_total, maxcount),
+                       d_models);
+    if (rc) return rc;
     SFH_CK(ctx, cudaMemcpyAsync(&flag, b + o_err, 4, cudaMemcpyDeviceToHost, st));
     SFH_CK(ctx, cudaStreamSynchronize(st));
     if (flag) return sfh_set_error(ctx, SFH_ERR_CUDA, "resampled star count changed between passes");
@@ -1236,6 +1521,7 @@ extern "C" int sfh_partial_cmd_smooth_ragged_dev(
     RaggedSpec rg;
     rg.grids.resize((size_t)ntempl);
     rg.out_off.resize((size_t)ntempl);
+    rg.node_off.resize((size_t)ntempl);
     rg.dmag.resize((size_t)ntempl);
     for (int64_t t = 0; t < ntempl; ++t) {
         const sfh_hess_grid &h = h_grids[t];
@@ -1244,17 +1530,21 @@ extern "C" int sfh_partial_cmd_smooth_ragged_dev(
             return sfh_set_error(ctx, SFH_ERR_ARG, "Hess grid out of range");
         if (h.out_offset < 0 || h.out_offset + h.nx * h.ny > models_len)
             return sfh_set_error(ctx, SFH_ERR_ARG, "template output outside d_models");
-        const int TY = band_rows(h.nx, h.ny, ntempl, ctx->sm_count);
-        if (!stamp_grid_ok(h.nx))
+        if (h.nx > kMaxColumns)
             return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
         rg.grids[(size_t)t] = Grid2{h.x_first, h.x_step, h.y_first, h.y_step, (int)h.nx, (int)h.ny};
         rg.out_off[(size_t)t] = h.out_offset;
+        rg.node_off[(size_t)t] = rg.nodes;
+        const Smooth sm = smooth_tiling(rg.grids[(size_t)t], true);
+        if (sm.on) {
+            rg.nodes += 64 * (int64_t)sm.tiles();
+            rg.max_node_groups = std::max(rg.max_node_groups, sm.groups());
+        }
         rg.dmag[(size_t)t] = std::fmin(std::fabs(h.x_step), std::fabs(h.y_step));  // :851
-        rg.smem = std::max(rg.smem, stamp_smem(h.nx, TY));
-        for (int64_t y0 = 0; y0 < h.ny; y0 += TY)
-            rg.tiles.push_back(StampTile{(int32_t)t, (int32_t)y0, (int32_t)TY});
+        rg.max_nx = std::max(rg.max_nx, h.nx);
+        for (int k = 0; k < tile_groups(h.nx, h.ny); ++k) rg.groups.push_back(StampGroup{(int32_t)t, k});
     }
-    if (rg.tiles.size() > 0x7fffffffu)
+    if (rg.groups.size() > 0x7fffffffu)
         return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "too many stamp tiles");
     P.dmag = rg.dmag[0];
     return partial_run(ctx, d_m_ini, d_mags, h_iso_off, h_iso_len, ntempl, P, y_index, c1, h_dmod,
@@ -1491,22 +1781,23 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
         for (int64_t q = 0; q < nc; ++q) { hstart[(size_t)q] = tot; tot += hcnt[(size_t)q]; }
         int64_t maxcount = 0;
         for (int64_t q = 0; q < nc; ++q) maxcount = std::max<int64_t>(maxcount, hcnt[(size_t)q]);
-        const size_t need = (size_t)std::max<int64_t>(tot, 1) * (5 * 8 + sizeof(StarRec));
+        const int64_t np = std::max<int64_t>(tot, 1);
+        const size_t a8 = sfh_align256((size_t)np * 8);
+        const size_t need = 5 * a8 + StampWork::bytes(tot, node_bytes(g, nc));
         if (need > pts_cap) {
             if (pts) cudaFree(pts);
             pts = nullptr;
             if ((e = cudaMalloc(&pts, need))) { rc = sfh_cuda_error(ctx, e, "binary_hess points"); break; }
             pts_cap = need;
         }
-        const int64_t np = std::max<int64_t>(tot, 1);
-        StarRec *rec = (StarRec *)pts;  // first: records are 16-byte aligned
-        double *px = (double *)(rec + np), *py = px + np, *psx = py + np, *psy = psx + np,
-               *pw = psy + np;
+        char *pb = (char *)pts;
+        double *px = pts, *py = (double *)(pb + a8), *psx = (double *)(pb + 2 * a8),
+               *psy = (double *)(pb + 3 * a8), *pw = (double *)(pb + 4 * a8);
         cudaMemcpyAsync(d_start, hstart.data(), nc * 8, cudaMemcpyHostToDevice, st);
         k_bin_points<<<(unsigned)nc, kPairThreads, 0, st>>>(P, hist, g, d_start, px, py, psx, psy, pw);
         ctx->launches++;
-        rc = launch_stamps(ctx, px, py, psx, psy, pw, d_start, d_cnt, d_cov, nc, x_first, x_step, nx,
-                           y_first, y_step, ny, d_models + t0 * nbins, rec, maxcount);
+        rc = launch_stamps(ctx, StampStars{px, py, psx, psy, pw, nullptr, d_start, d_cnt, d_cov}, nc, g,
+                           nullptr, StampWork(pb + 5 * a8, tot, maxcount), d_models + t0 * nbins);
         if (rc == SFH_OK && (e = cudaStreamSynchronize(st))) rc = sfh_cuda_error(ctx, e, "binary_hess");
     }
     cleanup();
