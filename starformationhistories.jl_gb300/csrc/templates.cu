@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "sfh_internal.cuh"
@@ -38,7 +39,13 @@ constexpr int kNarrowRows = 64;   // rows of a separable star's y table at a tim
 struct Grid2 {
     double xf, xs, yf, ys;
     int nx, ny;
+    double ixs, iys;  // 1 / xs, 1 / ys
 };
+
+Grid2 make_grid(double xf, double xs, int64_t nx, double yf, double ys, int64_t ny) {
+    return Grid2{xf, xs, yf, ys, (int)std::min<int64_t>(nx, INT32_MAX), (int)std::min<int64_t>(ny, INT32_MAX),
+                 1.0 / xs, 1.0 / ys};
+}
 
 // Signed erfc table entry: |value| = erfc(|t|), sign bit = sign of t.
 __device__ __forceinline__ float erfc_signed(float t) { return copysignf(erfcf(fabsf(t)), t); }
@@ -165,6 +172,30 @@ constexpr float kRoot2G = 1.1774100225154747f;  // sqrt 2 / g: u in units of sig
 // 2.5e-3 so that one correction serves the three nodes (y step up to 4): within 1e-8 of the peak and 1.5e-6
 // of a bin's own value down to 1e-4 of the peak.  The rest (a few bins per sigma) is integrated
 // bin by bin with erfc differences.
+//
+// FP64 throughput bounds this: divisions and square roots in full were three quarters of it.
+// Quantities that only need FP32 results take one Newton step from an FP32 seed (2^-44); pixel
+// numbers and window sizes take the product with the grid's inverse step, and the exact
+// division only within 1e-9 of a rounding boundary.
+__device__ __forceinline__ double rsqrt_nr(double v) {
+    if (!(v > 1.0e-30 && v < 1.0e30)) return 1.0 / sqrt(v);
+    const double y = (double)rsqrtf((float)v);
+    return fma(0.5 * y, fma(-(v * y), y, 1.0), y);
+}
+__device__ __forceinline__ double rcp_nr(double v) {
+    const double a = fabs(v);
+    if (!(a > 1.0e-30 && a < 1.0e30)) return 1.0 / v;
+    const double y = (double)__frcp_rn((float)v);
+    return fma(y, fma(-v, y, 1.0), y);
+}
+// z, or exact() when z is within 1e-9 of half way between integers (half) / of an integer.
+template <bool HALF, typename F>
+__device__ __forceinline__ double near_exact(double z, F exact) {
+    const double d = fabs(z - rint(z)), tol = fma(1.0e-9, fabs(z), 1.0e-9);
+    const bool safe = HALF ? d < 0.5 - tol : d > tol;
+    return safe ? z : exact();
+}
+
 __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x, double y,
                                             double sx, double sy, double A, int cov) {
     r.cls = kStarNone;
@@ -172,20 +203,26 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     r.xlo = r.ylo = 0;
     r.xhi = r.yhi = -1;
     if (!(sx >= 0.0 && sy >= 0.0)) return;
-    const double x0 = (x - g.xf) / g.xs + 1.0, y0 = (y - g.yf) / g.ys + 1.0;  // histogram_pix, :502
+    // histogram_pix, :502
+    const double x0 = near_exact<true>(fma(x - g.xf, g.ixs, 1.0), [&] { return (x - g.xf) / g.xs + 1.0; });
+    const double y0 = near_exact<true>(fma(y - g.yf, g.iys, 1.0), [&] { return (y - g.yf) / g.ys + 1.0; });
     if (!(fabs(x0) < 4.0e15 && fabs(y0) < 4.0e15)) return;
     const int64_t xc = __double2ll_rn(x0), yc = __double2ll_rn(y0);  // round(Int, ·): ties to even
-    const double ssx = sx / g.xs, ssy = sy / g.ys;
+    const double ssx = sx * g.ixs, ssy = sy * g.iys;
     int64_t xoff, yoff;
     if (cov == 0) {
         // size(GaussianPSFAsymmetric) = (ceil(Int, 10σx), ceil(Int, 10σy)), :247
         if (!(ssx >= 0.0 && ssy >= 0.0)) return;
-        xoff = max((int64_t)1, clamp_cut(ceil(ssx * 10.0)) / 2);
-        yoff = max((int64_t)1, clamp_cut(ceil(ssy * 10.0)) / 2);
+        const double cx = near_exact<false>(10.0 * ssx, [&] { return sx / g.xs * 10.0; });
+        const double cy = near_exact<false>(10.0 * ssy, [&] { return sy / g.ys * 10.0; });
+        xoff = max((int64_t)1, clamp_cut(ceil(cx)) / 2);
+        yoff = max((int64_t)1, clamp_cut(ceil(cy)) / 2);
     } else {
         // size(GaussianPSFCovariant) = (15σx, 10σy), :293; half widths, :383-384
-        xoff = max((int64_t)1, (int64_t)__double2ll_rn(fmin(15.0 * sx / g.xs / 2.0, 4.0e9)));
-        yoff = max((int64_t)1, (int64_t)__double2ll_rn(fmin(10.0 * sy / g.ys / 2.0, 4.0e9)));
+        const double cx = near_exact<true>(7.5 * ssx, [&] { return 15.0 * sx / g.xs / 2.0; });
+        const double cy = near_exact<true>(5.0 * ssy, [&] { return 10.0 * sy / g.ys / 2.0; });
+        xoff = max((int64_t)1, (int64_t)__double2ll_rn(fmin(cx, 4.0e9)));
+        yoff = max((int64_t)1, (int64_t)__double2ll_rn(fmin(cy, 4.0e9)));
     }
     const int64_t xlo = max((int64_t)1, xc - xoff), xhi = min((int64_t)g.nx, xc + xoff);
     const int64_t ylo = max((int64_t)1, yc - yoff), yhi = min((int64_t)g.ny, yc + yoff);
@@ -195,101 +232,91 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     r.ylo = (int)ylo - 1;
     r.yhi = (int)yhi - 1;
     r.cls = kStarNarrow;
-    const double isx = 1.0 / sx, isy = 1.0 / sy;
-    const double hx = 0.7071067811865476 * g.xs * isx, by = 0.7071067811865476 * g.ys * isy;
-    const double bx = cov ? 0.7071067811865476 * g.ys * isx : 0.0;
+    const float xsf = (float)g.xs, ysf = (float)g.ys;
+    const float hx = 0.70710678f * xsf / (float)sx, by = 0.70710678f * ysf / (float)sy;
+    const float bx = cov ? 0.70710678f * ysf / (float)sx : 0.f;
     // (a weight that is not a finite float stays bin by bin: 0 * inf must not leave the window)
-    const bool fine = fabs(A) <= 1.0e30 && hx > 0.0 && by > 0.0;
-    const bool wide = fine && (cov ? hx <= 0.045 && bx * bx + by * by <= 0.08 * 0.08
-                                   : hx <= 0.1 && by <= 0.1);
-    const bool mid = fine && cov != 0 && !wide && hx <= 0.1 && hx * hx * bx <= 2.5e-3 && by <= 4.0;
+    const bool fine = fabs(A) <= 1.0e30 && hx > 0.f && by > 0.f;
+    const bool wide = fine && (cov ? hx <= 0.045f && bx * bx + by * by <= 0.08f * 0.08f
+                                   : hx <= 0.1f && by <= 0.1f);
+    const bool mid = fine && cov != 0 && !wide && hx <= 0.1f && hx * hx * bx <= 2.5e-3f && by <= 4.f;
+    const double c = (double)cov, gs = 1.2011224087864498;  // sqrt(log2 e)
+    // the star's offset from its reference bin: its own, moved into its window
+    const int irl = (int)min(max(xc, xlo), xhi), jrl = (int)min(max(yc, ylo), yhi);
+    const double X = fma((double)irl - 0.5, g.xs, g.xf - x), Y = fma((double)jrl - 0.5, g.ys, g.yf - y);
+    r.ir = (float)(irl - 1);
+    r.jr = (float)(jrl - 1);
     if (wide || mid) {
-        const double gs = 1.2011224087864498;  // sqrt(log2 e)
-        const double c = (double)cov;
-        const double Syy = sy * sy + (wide ? g.ys * g.ys / 12.0 : 0.0);
-        const double m = -c * sy * sy / Syy;
-        const double vx = sx * sx + g.xs * g.xs / 12.0 + (c * c + c * m) * sy * sy;
-        const double ivx = 1.0 / vx, iSyy = 1.0 / Syy;
-        const double qx = 0.7071067811865476 * sqrt(ivx), qy = 0.7071067811865476 * sqrt(iSyy);
-        // reference bin: the star's own, moved into its window
-        const int64_t irl = min(max(xc, xlo), xhi), jrl = min(max(yc, ylo), yhi);
-        const double X = ((double)irl - 0.5) * g.xs + g.xf - x;
-        const double Y = ((double)jrl - 0.5) * g.ys + g.yf - y;
-        const double wx = g.xs * qx * gs, wsh = -m * g.ys * qx * gs, wy = g.ys * qy * gs;
-        const double uref = (X - m * Y) * qx * gs, vref = Y * qy * gs;
+        const double sy2 = sy * sy, Syy = wide ? fma(g.ys * (1.0 / 12.0), g.ys, sy2) : sy2;
+        const double ry = rsqrt_nr(Syy), m = wide ? -c * sy2 * (ry * ry) : -c;
+        const double vx = fma(sx, sx, fma(g.xs * (1.0 / 12.0), g.xs, wide ? (c * c + c * m) * sy2 : 0.0));
+        const double rx = rsqrt_nr(vx), qx = 0.8493218002880191 * rx, qy = 0.8493218002880191 * ry;  // g / √2
+        const double wsh = -m * g.ys * qx;
+        const float wxf = (float)(g.xs * qx), wshf = (float)wsh, wyf = (float)(g.ys * qy);
+        const float uref = (float)((X - m * Y) * qx), vref = (float)(Y * qy);
         // 2^(exponents relative to a tile's centre) stays in range over the window
-        const double eu = (double)(xhi - xlo + 1) * wx + (double)(yhi - ylo + 1) * fabs(wsh) + fabs(uref);
-        const double ev = (double)(yhi - ylo) * wy + fabs(vref);
-        if (eu * wx <= 10.0 && (mid ? fabs(wsh) * wx <= 1.0 : eu * fabs(wsh) + ev * wy <= 10.0)) {
-            const double k4x = g.xs * g.xs * ivx;
-            const double amp = A * g.xs * g.ys * qx * qy * 0.3183098861837907;  // A dx dy / (2π √(vx Syy))
+        const float eu = (float)(xhi - xlo + 1) * wxf + (float)(yhi - ylo + 1) * fabsf(wshf) + fabsf(uref);
+        const float ev = (float)(yhi - ylo) * wyf + fabsf(vref);
+        if (eu * wxf <= 10.f && (mid ? fabsf(wshf) * wxf <= 1.f : eu * fabsf(wshf) + ev * wyf <= 10.f)) {
+            const float rxf = (float)rx, k4x = xsf * rxf * (xsf * rxf);
+            const double amp = A * (g.xs * rx) * (g.ys * ry) * 0.15915494309189535;  // A dx dy / (2π √(vx Syy))
             r.cls = wide ? kStarWide : kStarMid;
-            r.p[0] = (float)wx;
-            r.p[1] = (float)wsh;
-            r.p[2] = (float)wy;
-            r.p[4] = (float)uref;
-            r.p[5] = (float)vref;
-            r.ir = (float)(irl - 1);
-            r.jr = (float)(jrl - 1);
+            r.p[0] = wxf;
+            r.p[1] = wshf;
+            r.p[2] = wyf;
+            r.p[4] = uref;
+            r.p[5] = vref;
+            r.p[6] = k4x * k4x * (1.f / 2880.f);
             if (wide) {
-                const double P = iSyy + m * m * ivx, s = 1.0 / sqrt(P), k4y = g.ys * g.ys * P;
+                const float ryf = (float)ry, mf = (float)m, P = fmaf(mf * rxf, mf * rxf, ryf * ryf);
+                const float s = rsqrtf(P), k4y = ysf * ysf * P;
                 r.p[3] = (float)amp;
-                r.p[6] = (float)(k4x * k4x / 2880.0);
-                r.p[7] = (float)(k4y * k4y / 2880.0);
-                r.p[8] = (float)(-2.0 * s * m * qx / gs);
-                r.p[9] = (float)(2.0 * s * qy / gs);
+                r.p[7] = k4y * k4y * (1.f / 2880.f);
+                r.p[8] = -1.1774100225f * s * mf * rxf;  // sqrt 2 / g
+                r.p[9] = 1.1774100225f * s * ryf;
                 r.p[10] = r.p[11] = 0.f;  // no smooth strips
             } else {
                 r.p[3] = (float)(amp * 0.4444444444444444);  // weight 8/9 of the middle node, halved
-                r.p[6] = (float)(k4x * k4x / 2880.0);
                 r.p[7] = (float)(0.3872983346207417 * wsh);  // sqrt(3/5) / 2 row
-                r.p[8] = (float)(0.3872983346207417 * wy);
+                r.p[8] = (float)(0.3872983346207417 * (g.ys * qy));
             }
             return;
         }
     }
     if (cov == 0) {
         // Bin i spans pixel coordinates [i, i+1]: evaluate at i + 1/2 with half width 1/2.
-        r.p[0] = (float)(0.7071067811865476 / ssx);
-        r.p[1] = (float)(0.7071067811865476 / ssy);
+        r.p[0] = (float)(0.7071067811865476 * g.xs * rcp_nr(sx));
+        r.p[1] = (float)(0.7071067811865476 * g.ys * rcp_nr(sy));
         r.p[2] = (float)((double)xlo - x0);
         r.p[3] = (float)((double)ylo - y0);
         r.p[4] = (float)(A * 0.25);
         return;
     }
-    // Bin centres: range(histogram_data(first + 1/2), histogram_data(last + 1/2); length), :390-393
-    const double xr0 = ((double)xlo - 0.5) * g.xs + g.xf, xr1 = ((double)xhi - 0.5) * g.xs + g.xf;
-    const double yr0 = ((double)ylo - 0.5) * g.ys + g.yf, yr1 = ((double)yhi - 0.5) * g.ys + g.yf;
-    const double xrs = (xr1 - xr0) / (double)(xhi - xlo), yrs = (yr1 - yr0) / (double)(yhi - ylo);
-    const int64_t irl = min(max(xc, xlo), xhi), jrl = min(max(yc, ylo), yhi);
-    const double X = xr0 + (double)(irl - xlo) * xrs - x, Y = yr0 + (double)(jrl - ylo) * yrs - y;
-    const double c = (double)cov;
     // A few bins per sigma (x step up to 0.25 sqrt 2 sigma): a bin's x integral as the Gaussian
     // with the box's variance, corrected through its sixth cumulant (He8 terms below 3e-9);
     // u at bin centres, base-2 scale.  Else erfc differences, u = t at the bins' lower edges.
-    const bool gauss = hx > 0.0 && hx <= 0.25;
-    const double vx = gauss ? sx * sx + xrs * xrs / 12.0 : sx * sx;
+    const bool gauss = hx > 0.f && hx <= 0.25f;
+    const double rx = rsqrt_nr(gauss ? fma(sx, sx, g.xs * g.xs * (1.0 / 12.0)) : sx * sx);
     // (a vanishing error: far edges at a large finite t, a hard histogram)
-    const double scale = fmin(0.7071067811865476 / sqrt(vx) * (gauss ? 1.2011224087864498 : 1.0), 1.0e30);
-    const double bxs = c * yrs * scale, sxs = xrs * scale, k = xrs * xrs / vx;
-    r.ir = (float)(irl - 1);
-    r.jr = (float)(jrl - 1);
-    r.p[0] = (float)((X + c * Y - (gauss ? 0.0 : xrs / 2.0)) * scale);
+    const double scale = fmin(0.7071067811865476 * rx * (gauss ? gs : 1.0), 1.0e30);
+    const double bxs = c * g.ys * scale, sxs = g.xs * scale;
+    r.p[0] = (float)((X + c * Y - (gauss ? 0.0 : g.xs * 0.5)) * scale);
     r.p[1] = (float)bxs;
     r.p[2] = (float)(bxs - (double)r.p[1]);
     r.p[3] = (float)sxs;
     r.p[4] = (float)(sxs - (double)r.p[3]);
-    const double vref = Y * isy * 0.8493218002880191, bys = yrs * isy * 0.8493218002880191;  // g / √2
+    const double isy = rcp_nr(sy) * 0.8493218002880191, vref = Y * isy, bys = g.ys * isy;
     r.p[5] = (float)vref;
     r.p[6] = (float)bys;
     r.p[10] = (float)(vref - (double)r.p[5]);
     r.p[11] = (float)(bys - (double)r.p[6]);
-    // prefac = A / 2 / sqrt(2π) / σy (:320) times the scale hy = yrs / 2 of the GL weights
-    // (:325), and the unit Gaussian's integral 2/√π xrs / (√2 √vx)
-    r.p[7] = (float)(A / 2.0 / 2.5066282746310002 * isy * (yrs / 2.0) *
-                     (gauss ? 0.7978845608028654 * sqrt(k) : 1.0));
-    r.p[8] = gauss ? (float)(k * k / 2880.0) : -1.f;
-    r.p[9] = (float)(k * k * k / 181440.0);
+    // prefac = A / 2 / sqrt(2π) / σy (:320) times the scale hy = dy / 2 of the GL weights
+    // (:325), and the unit Gaussian's integral 2/√π dx / (√2 √vx)
+    const double k = g.xs * rx;
+    r.p[7] = (float)(A * bys * 0.11742965983745643 * (gauss ? 0.7978845608028654 * k : 1.0));
+    const float k2 = (float)(k * k);
+    r.p[8] = gauss ? k2 * k2 * (1.f / 2880.f) : -1.f;
+    r.p[9] = k2 * k2 * k2 * (1.f / 181440.f);
 }
 
 // The strips over which a wide star's contribution can be interpolated from 8 x 8 Chebyshev
@@ -320,6 +347,27 @@ __device__ __forceinline__ unsigned long long smooth_strips(const StarRec &r, co
     return m;
 }
 
+// Completes a star's record with its smooth strips, stores it, and lists it when it is narrow:
+// the narrow stars of all templates are in one list (one atomic per warp).
+__device__ __forceinline__ void store_record(StarRec &r, const Grid2 &g, StarId id, StarRec *to,
+                                             StarId *narrow, int *n_narrow) {
+    if (r.cls == kStarWide) {
+        const Smooth sm = smooth_tiling(g, true);
+        const unsigned long long m = sm.on ? smooth_strips(r, g, sm) : 0ull;
+        r.p[10] = __uint_as_float((unsigned int)m);
+        r.p[11] = __uint_as_float((unsigned int)(m >> 32));
+    }
+    const unsigned act = __activemask(), nar = __ballot_sync(act, r.cls == kStarNarrow);
+    if (r.cls == kStarNarrow) {
+        const int lane = threadIdx.x & 31, lead = __ffs(nar) - 1;
+        int at = 0;
+        if (lane == lead) at = atomicAdd(n_narrow, __popc(nar));
+        at = __shfl_sync(nar, at, lead);
+        narrow[at + __popc(nar & ((1u << lane) - 1u))] = id;
+    }
+    *to = r;
+}
+
 constexpr int kPrepThreads = 64;  // small blocks: a few hundred stars already spread over the SMs
 
 __global__ void __launch_bounds__(kPrepThreads)
@@ -336,22 +384,7 @@ k_star_prep(const double *__restrict__ xs, const double *__restrict__ ys,
     StarRec r{};
     const Grid2 g = grids ? grids[t] : g0;
     star_record(r, g, xs[s], ys[s], sxs[s], sys[s], ws[s], covs[t]);
-    if (r.cls == kStarWide) {
-        const Smooth sm = smooth_tiling(g, true);
-        const unsigned long long m = sm.on ? smooth_strips(r, g, sm) : 0ull;
-        r.p[10] = __uint_as_float((unsigned int)m);
-        r.p[11] = __uint_as_float((unsigned int)(m >> 32));
-    }
-    // the narrow stars of all templates in one list (one atomic per warp)
-    const unsigned act = __activemask(), nar = __ballot_sync(act, r.cls == kStarNarrow);
-    if (r.cls == kStarNarrow) {
-        const int lane = threadIdx.x & 31, lead = __ffs(nar) - 1;
-        int at = 0;
-        if (lane == lead) at = atomicAdd(n_narrow, __popc(nar));
-        at = __shfl_sync(nar, at, lead);
-        narrow[at + __popc(nar & ((1u << lane) - 1u))] = StarId{t, q};
-    }
-    rec[s] = r;
+    store_record(r, g, StarId{t, q}, rec + s, narrow, n_narrow);
 }
 
 // ---------------------------------------------------------------- narrow stars
@@ -475,6 +508,11 @@ __device__ __forceinline__ float tile_node(bool nodes, int i) {  // ascending, i
     return i < 4 ? -c : c;
 }
 
+// The bits of 0 .. 7 from lo to hi (any two ints, lo <= hi).
+__device__ __forceinline__ unsigned window_bits(int lo, int hi) {
+    return (0xffu << min(max(lo, 0), 8)) & (0xffu >> (7 - min(max(hi, -1), 7))) & 0xffu;
+}
+
 struct Tile {
     int col0, row0;          // first bin (plain tiles)
     float xc, yc, xh, yh;    // centre in 0-based bins, half widths (NODES)
@@ -538,12 +576,14 @@ __device__ __forceinline__ void wide_tile(float2 (&acc)[8][4], const StarRec &r,
             X[i] = ex2f(-fmaf(2.f * u * hx, d, hx * hx * (d * d))) * fmaf(-r.p[6], fmaf(a2, a2 - 6.f, 3.f), 1.f);
         }
     }
-    if (__any_sync(0xffffffffu, part)) {
+    unsigned rows = 0xffu;  // the tile's rows in the window
+    if (!NODES && __any_sync(0xffffffffu, part)) {
+        const unsigned cols = window_bits(r.xlo - col0, r.xhi - col0);
+        rows = window_bits(r.ylo - row0, r.yhi - row0);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            if (col0 + i < r.xlo || col0 + i > r.xhi) X[i] = 0.f;
+            if (!(cols >> i & 1u)) X[i] = 0.f;
     }
-    const int ylo = NODES ? row0 : r.ylo, yhi = NODES ? row0 + 7 : r.yhi;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float d = tile_node(NODES, j);
@@ -552,7 +592,7 @@ __device__ __forceinline__ void wide_tile(float2 (&acc)[8][4], const StarRec &r,
             const float b = fmaf(kRoot2G * by, d, zy), b2 = b * b;
             y *= fmaf(-r.p[7], fmaf(b2, b2 - 6.f, 3.f), 1.f);
         }
-        if (row0 + j < ylo || row0 + j > yhi) y = 0.f;
+        if (!NODES && !(rows >> j & 1u)) y = 0.f;
         const float2 y2 = make_float2(y, y);
         if (COV) {
             const float4 t0 = *reinterpret_cast<const float4 *>(T + 8 * j);
@@ -586,6 +626,8 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
     const float2 c0 = make_float2(fmaf(-3.f, r.p[6], 1.f), fmaf(-3.f, r.p[6], 1.f));
     const float c1f = 8.317766166719343f * r.p[6], c2f = -1.9218120556728056f * r.p[6];
     const float2 c1 = make_float2(c1f, c1f), c2 = make_float2(c2f, c2f);
+    const unsigned cols = window_bits(r.xlo - col0, r.xhi - col0);
+    const unsigned rows = window_bits(r.ylo - row0, r.yhi - row0);
     float2 X0[4], Xm[4], Xp[4], hd[4];
     const float hx2 = hx * hx, g0 = -2.f * hx * u, gd = -2.f * hx * dn;
 #pragma unroll
@@ -594,10 +636,10 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const float d = tile_node(false, 2 * c + q), cx = hx2 * d * d;
-            const bool in = col0 + 2 * c + q >= r.xlo && col0 + 2 * c + q <= r.xhi;
-            x0[q] = in ? ex2f(fmaf(g0, d, -cx)) : 0.f;
-            xm[q] = in ? ex2f(fmaf(g0 - gd, d, -cx)) : 0.f;
-            xp[q] = in ? ex2f(fmaf(g0 + gd, d, -cx)) : 0.f;
+            x0[q] = ex2f(fmaf(g0, d, -cx));
+            xm[q] = ex2f(fmaf(g0 - gd, d, -cx));
+            xp[q] = ex2f(fmaf(g0 + gd, d, -cx));
+            if (!(cols >> (2 * c + q) & 1u)) x0[q] = xm[q] = xp[q] = 0.f;
             h2[q] = hx * d;
         }
         X0[c] = make_float2(x0[0], x0[1]);
@@ -608,7 +650,7 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float d = tile_node(false, j), uj = fmaf(bx, d, u), vj = fmaf(by, d, v);
-        const float a = row0 + j >= r.ylo && row0 + j <= r.yhi ? amp : 0.f;
+        const float a = rows >> j & 1u ? amp : 0.f;
         const float um = uj - dn, vm = vj - en, up = uj + dn, vp = vj + en;
         const float y0 = a * ex2f(-fmaf(uj, uj, vj * vj));
         const float ym = 0.625f * a * ex2f(-fmaf(um, um, vm * vm));
@@ -949,7 +991,7 @@ struct IsoParams {
 };
 
 struct IsoPoint {
-    double mass, xcol, ymag, cerr, yerr, compl_;
+    double mass, xcol, ymag, cerr, yerr, compl_, pdf;
 };
 
 __device__ __forceinline__ double imf_pdf(const IsoParams &P, double m) {
@@ -966,7 +1008,7 @@ __device__ __forceinline__ double err_eval(const IsoParams &P, int f, double m) 
 }
 
 __device__ __forceinline__ double compl_eval(const IsoParams &P, int f, double m) {
-    return P.cA[f] / (1.0 + (double)__expf((float)((m - P.cm50[f]) * P.crho_inv[f])));
+    return P.cA[f] * rcp_nr(1.0 + (double)__expf((float)((m - P.cm50[f]) * P.crho_inv[f])));
 }
 
 // Resampled point q of the isochrone (mini_spacing + interpolate_mini + callables).
@@ -991,8 +1033,8 @@ __device__ IsoPoint iso_point(const IsoParams &P, const double *m, const double 
             mass = m[k + 1];
             frac = 1.0;
         } else {
-            mass = m[k] + (m[k + 1] - m[k]) / (double)c * (double)j;
-            frac = (mass - m[k]) / (m[k + 1] - m[k]);
+            frac = (double)j * rcp_nr((double)c);
+            mass = fma(m[k + 1] - m[k], frac, m[k]);
         }
     }
     const int kk = (q == 0) ? 0 : k;
@@ -1090,10 +1132,10 @@ __global__ void __launch_bounds__(kIsoThreads)
 k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
             const int64_t *__restrict__ iso_off, const int32_t *__restrict__ iso_len,
             const double *__restrict__ dmods, const double *__restrict__ norms, IsoParams P,
-            const double *__restrict__ dmag_t, const int64_t *__restrict__ star_off,
-            double *__restrict__ sx_,
-            double *__restrict__ sy_, double *__restrict__ ssx, double *__restrict__ ssy,
-            double *__restrict__ sw, int32_t *__restrict__ count, int *__restrict__ err_flag) {
+            const double *__restrict__ dmag_t, const int64_t *__restrict__ star_off, Grid2 g0,
+            const Grid2 *__restrict__ grids, StarRec *__restrict__ rec, StarId *__restrict__ narrow,
+            int *__restrict__ n_narrow, int32_t *__restrict__ count, int *__restrict__ err_flag) {
+    __shared__ IsoPoint s_pt[kIsoThreads];
     __shared__ int s_cnt[kIsoMaxPts];
     __shared__ int s_pos[kIsoMaxPts];
     __shared__ int s_warp[kIsoThreads / 32];
@@ -1112,17 +1154,28 @@ k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
     const double dmod = dmods[t];
     const double wscale = norms[t] * P.inv_mean_mass;
     const int64_t so = star_off[t];
-    // One thread per star: endpoints q and q+1, midpoints and weight, :765-776, :884-888.
-    for (int q = threadIdx.x; q < nstars; q += blockDim.x) {
-        const IsoPoint a = iso_point(P, m, mg, n, s_pos, s_cnt, dmod, q);
-        const IsoPoint b = iso_point(P, m, mg, n, s_pos, s_cnt, dmod, q + 1);
-        const double w = (b.mass - a.mass) * (imf_pdf(P, a.mass) + imf_pdf(P, b.mass)) / 2.0 *
-                         a.compl_ * wscale;
-        sx_[so + q] = a.xcol + (b.xcol - a.xcol) / 2.0;
-        sy_[so + q] = a.ymag + (b.ymag - a.ymag) / 2.0;
-        ssx[so + q] = a.cerr + (b.cerr - a.cerr) / 2.0;
-        ssy[so + q] = a.yerr + (b.yerr - a.yerr) / 2.0;
-        sw[so + q] = w;
+    // A thread per point, blocks of points overlapping by one: a star is a point and its right
+    // neighbour (midpoints and weight, :765-776, :884-888).
+    const Grid2 g = grids ? grids[t] : g0;
+    const int cov = P.covariant ? (P.y_index == P.c1 ? -1 : 1) : 0;
+    for (int base = 0; base < nstars; base += kIsoThreads - 1) {
+        const int q = base + (int)threadIdx.x;
+        IsoPoint a;
+        if (q < npts) {
+            a = iso_point(P, m, mg, n, s_pos, s_cnt, dmod, q);
+            a.pdf = imf_pdf(P, a.mass);
+        }
+        __syncthreads();  // the previous block's points are no longer read
+        if (q < npts) s_pt[threadIdx.x] = a;
+        __syncthreads();
+        if (threadIdx.x < kIsoThreads - 1 && q < nstars) {
+            const IsoPoint &b = s_pt[threadIdx.x + 1];
+            const double w = (b.mass - a.mass) * (a.pdf + b.pdf) * 0.5 * a.compl_ * wscale;
+            StarRec r{};
+            star_record(r, g, a.xcol + (b.xcol - a.xcol) * 0.5, a.ymag + (b.ymag - a.ymag) * 0.5,
+                        a.cerr + (b.cerr - a.cerr) * 0.5, a.yerr + (b.yerr - a.yerr) * 0.5, w, cov);
+            store_record(r, g, StarId{t, q}, rec + so + q, narrow, n_narrow);
+        }
     }
 }
 
@@ -1154,6 +1207,7 @@ struct StampWork {
     int *n_narrow = nullptr;
     float *node = nullptr;     // node_bytes() / the ragged batch's nodes
     int64_t maxcount = 0;      // largest star count of a template
+    bool made = false;         // the records are there already (k_iso_stars)
     static size_t bytes(int64_t stars, size_t node) {
         const size_t n = (size_t)std::max<int64_t>(stars, 1);
         return 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarId)) + sfh_align256(node);
@@ -1203,10 +1257,10 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
                                              (int)(kNarrowWarps * (kMaxColumns + kNarrowRows) * 4)));
         attr_set = true;
     }
-    if (have) SFH_CK(ctx, cudaMemsetAsync(w.n_narrow, 0, sizeof(int), s));
+    if (have && !w.made) SFH_CK(ctx, cudaMemsetAsync(w.n_narrow, 0, sizeof(int), s));
     for (int64_t t0 = 0; have && t0 < ntempl; t0 += 65535) {
         const unsigned nt = (unsigned)std::min<int64_t>(65535, ntempl - t0);
-        if (w.maxcount > 0) {
+        if (w.maxcount > 0 && !w.made) {
             k_star_prep<<<dim3((unsigned)((w.maxcount + kPrepThreads - 1) / kPrepThreads), nt),
                           kPrepThreads, 0, s>>>(st.x, st.y, st.sx, st.sy, st.w, st.start, st.count,
                                                 st.cov, g, rg ? rg->grids : nullptr, (int)t0, w.rec,
@@ -1260,7 +1314,7 @@ extern "C" int sfh_bin_cmd_smooth_batch_dev(sfh_ctx *ctx, const double *d_x, con
     k_offsets_to_counts<<<(int)((ntempl + 255) / 256), 256, 0, ctx->stream>>>(d_offsets, ntempl,
                                                                                 d_cnt);
     SFH_LAUNCHED(ctx);
-    const Grid2 g{xf, xs, yf, ys, (int)std::min<int64_t>(nx, INT32_MAX), (int)std::min<int64_t>(ny, INT32_MAX)};
+    const Grid2 g = make_grid(xf, xs, nx, yf, ys, ny);
     return launch_stamps(ctx, StampStars{d_x, d_y, d_sx, d_sy, d_w, nullptr, d_offsets, d_cnt, d_cov},
                          ntempl, g, nullptr, StampWork(), d_models);
 }
@@ -1282,7 +1336,7 @@ extern "C" int sfh_bin_cmd_smooth(sfh_ctx *ctx, const double *x, const double *y
     const size_t o_out = 5 * a5, o_meta = o_out + sfh_align256(nbins * 4), o_work = o_meta + 256;
     if (nx > (1 << 20) || ny > (1 << 20))
         return sfh_set_error(ctx, SFH_ERR_ARG, "stamp grid or template count out of range");
-    const Grid2 g{xf, xs, yf, ys, (int)nx, (int)ny};
+    const Grid2 g = make_grid(xf, xs, nx, yf, ys, ny);
     int rc = sfh_stage_reserve(ctx, o_work + StampWork::bytes(npts, node_bytes(g, 1)));
     if (rc) return rc;
     char *b = (char *)ctx->stage;
@@ -1391,91 +1445,79 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
                 const double *h_norm, const RaggedSpec *rg, double xf, double xs, int64_t nx,
                 double yf, double ys, int64_t ny, float *d_models) {
     cudaStream_t st = ctx->stream;
+    // What the host knows, in one upload: star offsets (known after pass 1) first, then the
+    // per-template inputs and the zeroed counters; the star counts follow the counters, so
+    // that pass 1 is read back in one copy.
+    std::vector<char> head;
+    auto add = [&](const void *src, size_t bytes) {
+        const size_t at = head.size();
+        head.resize(at + sfh_align256(bytes), 0);
+        if (src) std::memcpy(head.data() + at, src, bytes);
+        return at;
+    };
+    const size_t n8 = (size_t)ntempl * 8, n4 = (size_t)ntempl * 4;
+    const std::vector<int32_t> cov((size_t)ntempl, P.covariant ? (y_index == c1 ? -1 : 1) : 0);
+    const size_t o_soff = add(nullptr, n8 + 8);
+    const size_t o_off = add(h_iso_off, n8), o_len = add(h_iso_len, n4), o_dm = add(h_dmod, n8);
+    const size_t o_nm = add(h_norm, n8), o_cov = add(cov.data(), n4);
+    const size_t o_dmag = rg ? add(rg->dmag.data(), n8) : 0;
+    const size_t o_grid = rg ? add(rg->grids.data(), ntempl * sizeof(Grid2)) : 0;
+    const size_t o_oof = rg ? add(rg->out_off.data(), n8) : 0, o_noff = rg ? add(rg->node_off.data(), n8) : 0;
+    const size_t o_groups = rg ? add(rg->groups.data(), rg->groups.size() * sizeof(StampGroup)) : 0;
+    const size_t o_err = add(nullptr, 8), o_cnt64 = head.size();  // error flag, narrow stars
+    const size_t o_cnt = o_cnt64 + sfh_align256(n8), o_work = o_cnt + sfh_align256(n4);
     // Pass 1: resampled star count per template (one read-back), exact offsets.
-    const size_t o_off = 0, o_len = sfh_align256(ntempl * 8), o_dm = o_len + sfh_align256(ntempl * 4);
-    const size_t o_nm = o_dm + sfh_align256(ntempl * 8), o_err = o_nm + sfh_align256(ntempl * 8);
-    const size_t o_cnt64 = o_err + 256, o_soff = o_cnt64 + sfh_align256(ntempl * 8);
-    const size_t o_cnt = o_soff + sfh_align256((ntempl + 1) * 8), o_cov = o_cnt + sfh_align256(ntempl * 4);
-    const size_t o_dmag = o_cov + sfh_align256(ntempl * 4);
-    const size_t o_stars = o_dmag + sfh_align256(ntempl * 8);
-    const double *d_dmag = nullptr;  // per-template Δmag (ragged grids), set once uploaded
-    int rc = sfh_scratch_reserve(ctx, o_stars);
+    int rc = sfh_scratch_reserve(ctx, o_work);
     if (rc) return rc;
     char *b = (char *)ctx->scratch;
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_off, h_iso_off, ntempl * 8, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_len, h_iso_len, ntempl * 4, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemsetAsync(b + o_err, 0, 4, st));
-    if (rg) {
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_dmag, rg->dmag.data(), ntempl * 8, cudaMemcpyHostToDevice, st));
-        d_dmag = (const double *)(b + o_dmag);
-    }
+    SFH_CK(ctx, cudaMemcpyAsync(b + o_off, head.data() + o_off, head.size() - o_off,
+                                cudaMemcpyHostToDevice, st));
+    const auto dmag = [&] { return rg ? (const double *)(b + o_dmag) : nullptr; };  // per-template Δmag
     k_iso_count<<<(unsigned)ntempl, kIsoThreads, 0, st>>>(
-        d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len), P, d_dmag,
+        d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len), P, dmag(),
         (int64_t *)(b + o_cnt64), (int *)(b + o_err));
     SFH_LAUNCHED(ctx);
-    std::vector<int64_t> nst((size_t)ntempl);
-    int flag = 0;
-    SFH_CK(ctx, cudaMemcpyAsync(nst.data(), b + o_cnt64, ntempl * 8, cudaMemcpyDeviceToHost, st));
-    SFH_CK(ctx, cudaMemcpyAsync(&flag, b + o_err, 4, cudaMemcpyDeviceToHost, st));
+    std::vector<int64_t> back((o_cnt64 - o_err) / 8 + (size_t)ntempl);
+    SFH_CK(ctx, cudaMemcpyAsync(back.data(), b + o_err, back.size() * 8, cudaMemcpyDeviceToHost, st));
     SFH_CK(ctx, cudaStreamSynchronize(st));
+    int flag = 0;
+    std::memcpy(&flag, back.data(), 4);
     if (flag == 2) return sfh_set_error(ctx, SFH_ERR_ARG, "isochrone masses must be strictly increasing");
-    std::vector<int64_t> soff((size_t)ntempl + 1, 0);
+    const int64_t *nst = back.data() + (o_cnt64 - o_err) / 8;
+    int64_t *soff = (int64_t *)(head.data() + o_soff);
     int64_t maxcount = 0;
     for (int64_t t = 0; t < ntempl; ++t) {
-        soff[(size_t)t + 1] = soff[(size_t)t] + nst[(size_t)t];
-        maxcount = std::max(maxcount, nst[(size_t)t]);
+        soff[t + 1] = soff[t] + nst[t];
+        maxcount = std::max(maxcount, nst[t]);
     }
-    const int64_t nstar_total = soff[(size_t)ntempl] > 0 ? soff[(size_t)ntempl] : 1;
+    const int64_t nstar_total = std::max<int64_t>(soff[ntempl], 1);
     // Pass 2: star records, then the stamps.
-    const size_t a8 = sfh_align256((size_t)nstar_total * 8);
-    const Grid2 g{xf, xs, yf, ys, (int)std::min<int64_t>(nx, INT32_MAX), (int)std::min<int64_t>(ny, INT32_MAX)};
+    const Grid2 g = make_grid(xf, xs, nx, yf, ys, ny);
     const size_t nodes = rg ? (size_t)rg->nodes * sizeof(float)
                             : nx <= kMaxColumns && ny <= (1 << 20) ? node_bytes(g, ntempl) : 0;
-    const size_t o_work = o_stars + 5 * a8;
-    const size_t o_grid = o_work + StampWork::bytes(nstar_total, nodes);
-    const size_t o_oof = o_grid + (rg ? sfh_align256(ntempl * sizeof(Grid2)) : 0);
-    const size_t o_noff = o_oof + (rg ? sfh_align256(ntempl * 8) : 0);
-    const size_t o_tiles = o_noff + (rg ? sfh_align256(ntempl * 8) : 0);
-    const size_t o_end = o_tiles + (rg ? sfh_align256(rg->groups.size() * sizeof(StampGroup)) : 0);
-    rc = sfh_scratch_reserve(ctx, o_end);
+    rc = sfh_scratch_reserve(ctx, o_work + StampWork::bytes(nstar_total, nodes));
     if (rc) return rc;
-    b = (char *)ctx->scratch;  // may have moved
-    std::vector<int32_t> cov((size_t)ntempl, P.covariant ? (y_index == c1 ? -1 : 1) : 0);
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_off, h_iso_off, ntempl * 8, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_len, h_iso_len, ntempl * 4, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_dm, h_dmod, ntempl * 8, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_nm, h_norm, ntempl * 8, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_soff, soff.data(), (ntempl + 1) * 8, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_cov, cov.data(), ntempl * 4, cudaMemcpyHostToDevice, st));
-    SFH_CK(ctx, cudaMemsetAsync(b + o_err, 0, 4, st));
-    if (rg) {
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_dmag, rg->dmag.data(), ntempl * 8, cudaMemcpyHostToDevice, st));
-        d_dmag = (const double *)(b + o_dmag);
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_grid, rg->grids.data(), ntempl * sizeof(Grid2),
-                                    cudaMemcpyHostToDevice, st));
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_oof, rg->out_off.data(), ntempl * 8, cudaMemcpyHostToDevice, st));
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_noff, rg->node_off.data(), ntempl * 8, cudaMemcpyHostToDevice, st));
-        SFH_CK(ctx, cudaMemcpyAsync(b + o_tiles, rg->groups.data(), rg->groups.size() * sizeof(StampGroup),
-                                    cudaMemcpyHostToDevice, st));
-    }
-    double *sxp = (double *)(b + o_stars), *syp = (double *)(b + o_stars + a8);
-    double *ssxp = (double *)(b + o_stars + 2 * a8), *ssyp = (double *)(b + o_stars + 3 * a8);
-    double *swp = (double *)(b + o_stars + 4 * a8);
+    const bool moved = b != (char *)ctx->scratch;
+    b = (char *)ctx->scratch;
+    SFH_CK(ctx, cudaMemcpyAsync(b, head.data(), moved ? head.size() : o_off, cudaMemcpyHostToDevice, st));
+    StampWork work(b + o_work, nstar_total, maxcount);
+    work.made = true;
+    work.n_narrow = (int *)(b + o_err) + 1;
     k_iso_stars<<<(unsigned)ntempl, kIsoThreads, 0, st>>>(
         d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len),
-        (const double *)(b + o_dm), (const double *)(b + o_nm), P, d_dmag,
-        (const int64_t *)(b + o_soff), sxp, syp, ssxp, ssyp, swp, (int32_t *)(b + o_cnt),
-        (int *)(b + o_err));
+        (const double *)(b + o_dm), (const double *)(b + o_nm), P, dmag(),
+        (const int64_t *)(b + o_soff), g, rg ? (const Grid2 *)(b + o_grid) : nullptr, work.rec,
+        work.narrow, work.n_narrow, (int32_t *)(b + o_cnt), (int *)(b + o_err));
     SFH_LAUNCHED(ctx);
     StampGrids sg{};
     if (rg)
         sg = StampGrids{(const Grid2 *)(b + o_grid), (const int64_t *)(b + o_oof),
-                        (const int64_t *)(b + o_noff), (const StampGroup *)(b + o_tiles),
+                        (const int64_t *)(b + o_noff), (const StampGroup *)(b + o_groups),
                         (int64_t)rg->groups.size(), rg->max_node_groups, rg->max_nx};
-    rc = launch_stamps(ctx, StampStars{sxp, syp, ssxp, ssyp, swp, nullptr, (const int64_t *)(b + o_soff),
-                                       (const int32_t *)(b + o_cnt), (const int32_t *)(b + o_cov)},
-                       ntempl, g, rg ? &sg : nullptr, StampWork(b + o_work, nstar_total, maxcount),
-                       d_models);
+    rc = launch_stamps(ctx, StampStars{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                       (const int64_t *)(b + o_soff), (const int32_t *)(b + o_cnt),
+                                       (const int32_t *)(b + o_cov)},
+                       ntempl, g, rg ? &sg : nullptr, work, d_models);
     if (rc) return rc;
     SFH_CK(ctx, cudaMemcpyAsync(&flag, b + o_err, 4, cudaMemcpyDeviceToHost, st));
     SFH_CK(ctx, cudaStreamSynchronize(st));
@@ -1532,7 +1574,7 @@ extern "C" int sfh_partial_cmd_smooth_ragged_dev(
             return sfh_set_error(ctx, SFH_ERR_ARG, "template output outside d_models");
         if (h.nx > kMaxColumns)
             return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
-        rg.grids[(size_t)t] = Grid2{h.x_first, h.x_step, h.y_first, h.y_step, (int)h.nx, (int)h.ny};
+        rg.grids[(size_t)t] = make_grid(h.x_first, h.x_step, h.nx, h.y_first, h.y_step, h.ny);
         rg.out_off[(size_t)t] = h.out_offset;
         rg.node_off[(size_t)t] = rg.nodes;
         const Smooth sm = smooth_tiling(rg.grids[(size_t)t], true);
@@ -1763,7 +1805,7 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
                                                                     fl, imfv);
     k_bin_prefac<<<(unsigned)ntempl, kPairThreads, 0, st>>>(P, d_m_ini, d_off, d_len, d_norm, prefac);
     ctx->launches += 2;
-    Grid2 g{x_first, x_step, y_first, y_step, (int)nx, (int)ny};
+    const Grid2 g = make_grid(x_first, x_step, nx, y_first, y_step, ny);
     std::vector<int32_t> hcnt((size_t)chunk);
     std::vector<int64_t> hstart((size_t)chunk);
     size_t pts_cap = 0;
