@@ -288,7 +288,8 @@ def _range(e):
     if e.ndim != 1 or e.size < 2:
         raise ValueError("edges must be evenly spaced vectors of length >= 2")
     step = (e[-1] - e[0]) / (e.size - 1)
-    if not np.allclose(np.diff(e), step, rtol=1e-9, atol=0.0):
+    d = e[1:] - e[:-1]
+    if not np.all((np.abs(d - step) <= 1e-9 * abs(step)) | (d == step)):
         raise ValueError("edges must be AbstractRange-like (evenly spaced)")
     if jstep is not None and jstep != 0.0:
         step = jstep
@@ -717,6 +718,9 @@ class HessGrid(C.Structure):
                 ("out_offset", C.c_int64)]
 
 
+_GRID = np.dtype([(n, np.int64 if t is C.c_int64 else np.float64) for n, t in HessGrid._fields_])
+
+
 def partial_cmd_smooth_ragged(m_ini, mags, iso_off, iso_len, y_index, color_indices, err_models,
                               compl_models, imf, dmod, normalize_value, edges, mean_mass=None,
                               bias=None, out=None, ctx=None):
@@ -734,12 +738,20 @@ def partial_cmd_smooth_ragged(m_ini, mags, iso_off, iso_len, y_index, color_indi
         raise ValueError("one (xedges, yedges) pair per template is required")
     dm = np.ascontiguousarray(np.broadcast_to(np.asarray(dmod, dtype=np.float64), (nt,)))
     nm = np.ascontiguousarray(np.broadcast_to(np.asarray(normalize_value, dtype=np.float64), (nt,)))
-    grids = (HessGrid * nt)()
-    offsets = np.zeros(nt + 1, dtype=np.int64)
+    # one row per template; a galaxy's templates usually share its edge vectors, which this
+    # call then looks at once (`seen` holds them, so no other object takes their id)
+    seen = {}
+    rows = np.empty((nt, 6))
     for t, (xe, ye) in enumerate(edges):
-        (xf, xs, nx), (yf, ys, ny) = _range(xe), _range(ye)
-        grids[t] = HessGrid(xf, xs, nx, yf, ys, ny, int(offsets[t]))
-        offsets[t + 1] = offsets[t] + nx * ny
+        got = seen.get((id(xe), id(ye)))
+        if got is None:
+            got = seen[(id(xe), id(ye))] = (_range(xe) + _range(ye), xe, ye)
+        rows[t] = got[0]
+    grids = np.zeros(nt, dtype=_GRID)
+    for k, name in enumerate(("x_first", "x_step", "nx", "y_first", "y_step", "ny")):
+        grids[name] = rows[:, k]
+    offsets = np.concatenate([[0], np.cumsum(grids["nx"] * grids["ny"])]).astype(np.int64)
+    grids["out_offset"] = offsets[:-1]
     if out is None:
         out = torch.empty(int(offsets[-1]), dtype=torch.float32, device=m_ini.device)
     elif out.numel() < offsets[-1]:
@@ -758,6 +770,6 @@ def partial_cmd_smooth_ragged(m_ini, mags, iso_off, iso_len, y_index, color_indi
     check(load().sfh_partial_cmd_smooth_ragged_dev(
         ctx.handle, m_ini.data_ptr(), mags.data_ptr(), int(total), iso_off.ctypes.data,
         iso_len.ctypes.data, nt, nf, int(y_index), int(color_indices[0]), int(color_indices[1]),
-        E, Cm, b, C.byref(ip), mm, dm.ctypes.data, nm.ctypes.data, grids, int(out.numel()),
+        E, Cm, b, C.byref(ip), mm, dm.ctypes.data, nm.ctypes.data, grids.ctypes.data, int(out.numel()),
         out.data_ptr()), ctx.handle, "partial_cmd_smooth_ragged")
     return out, offsets
