@@ -335,6 +335,128 @@ __global__ void k_reduce_g(const double *__restrict__ partG, int nchunks, int64_
 }
 
 
+// ---------------------------------------------------------------- fg! in one launch (FP64 storage)
+// A matrix whose 64-bin tiles all fit the GPU at once (one tile per CTA): every CTA keeps its
+// tile of M in shared memory, forms m, the Poisson terms and w for its bins, then its share
+// of G = M^T w; the last CTA to finish adds the CTAs' shares in CTA order.  Launches, the host
+// link and the FP64 pipe's latency bound a matrix of this size, not bytes: the four kernels
+// below read M twice; a host-array call of 50 templates x 7,500 bins took 49 us with them and takes
+// 28 us with this one (16 us in the kernel).
+constexpr int kTile64 = 64, kPad64 = kTile64 + 1;  // padded: templates fall on different banks
+
+size_t tile64_smem(int64_t nt) { return ((size_t)nt * (kPad64 + 1) + 6 * kTile64) * sizeof(double); }
+
+// Two CTAs of 256 threads fit an SM up to 106 KB each, one up to 213 KB.
+bool tile64_fits(const sfh_ctx *ctx, int64_t nbins, int64_t nt) {
+    const size_t smem = tile64_smem(nt);
+    const int per_sm = smem <= 106 * 1024 ? 2 : smem <= 213 * 1024 ? 1 : 0;
+    return (nbins + kTile64 - 1) / kTile64 <= (int64_t)per_sm * ctx->sm_count;
+}
+
+struct Tile64Args {
+    const double *M;
+    int64_t nbins;
+    int nt;
+    const double *r, *data;
+    double eps;
+    double *composite, *G, *negLogL;  // negLogL may be NULL
+    double gsign;
+    double *part;  // [CTAs][nt + 1]: G shares, logL share
+    unsigned int *counter;
+};
+
+__global__ void __launch_bounds__(kThreads) k_fg_tile_f64(Tile64Args a) {
+    extern __shared__ double s_t[];
+    double *s_m = s_t, *s_r = s_m + (size_t)a.nt * kPad64, *s_q = s_r + a.nt, *s_w = s_q + 5 * kTile64;
+    __shared__ bool s_last;
+    const int tid = threadIdx.x, b = tid & (kTile64 - 1), part = tid / kTile64;  // 4 template shares
+    const int64_t i = (int64_t)blockIdx.x * kTile64 + b;
+    const bool live = i < a.nbins;
+    // the thread's own elements of M (its bin, every fourth template), r and the counts, all
+    // in flight together
+    for (int j = part; j < a.nt; j += 4) {
+        if (live) {
+            const unsigned to = (unsigned)__cvta_generic_to_shared(s_m + j * kPad64 + b);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(a.M + (int64_t)j * a.nbins + i)
+                         : "memory");
+        } else {
+            s_m[j * kPad64 + b] = 0.0;
+        }
+    }
+    const double n = live && part == 0 ? a.data[i] : 0.0;
+    for (int j = tid; j < a.nt; j += kThreads) s_r[j] = a.r[j];
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    double m = 0.0;
+    for (int j = part; j < a.nt; j += 4) m = fma(s_m[j * kPad64 + b], s_r[j], m);
+    s_q[part * kTile64 + b] = m;
+    __syncthreads();
+    if (part == 0) {
+        double w = 0.0, term = 0.0;
+        if (live) {
+            m = (s_q[b] + s_q[kTile64 + b]) + (s_q[2 * kTile64 + b] + s_q[3 * kTile64 + b]);
+            const double c = m > a.eps ? m : a.eps;
+            w = 1.0 - n / c;
+            a.composite[i] = w;
+            if (a.negLogL) term = n > 0.0 ? n - c - n * log(n / c) : -c;
+        }
+        s_w[b] = w;
+        s_q[b] = term;
+    }
+    __syncthreads();
+    // G shares: thread (template j, segment sg of the bins); then the segments in order
+    const int segs = min(kThreads / min(a.nt, kThreads), kTile64);
+    double *mine = a.part + (int64_t)blockIdx.x * (a.nt + 1);
+    const int sg = tid / a.nt;
+    for (int j = tid % a.nt; sg < segs && j < a.nt; j += kThreads) {
+        const int k0 = kTile64 * sg / segs, k1 = kTile64 * (sg + 1) / segs;
+        double g = 0.0;
+        for (int k = k0; k < k1; ++k) g = fma(s_m[j * kPad64 + k], s_w[k], g);
+        if (segs > 1) s_q[kTile64 + sg * a.nt + j] = g;  // behind the terms; segs * nt <= 256
+        else mine[j] = g;
+    }
+    __syncthreads();
+    if (segs > 1 && tid < a.nt) {
+        double g = 0.0;
+        for (int k = 0; k < segs; ++k) g += s_q[kTile64 + k * a.nt + tid];
+        mine[tid] = g;
+    }
+    if (tid < 32) {  // a warp: the terms in a fixed tree
+        double v = s_q[tid] + s_q[tid + 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (tid == 0) mine[a.nt] = v;
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // the CTAs' shares: entry j (logL last) by `ways` threads, each every ways-th CTA
+    const int ne = a.nt + 1, ways = max(1, kThreads / ne), way = tid / ne;
+    for (int j = tid % ne; way < ways && j < ne; j += kThreads) {
+        double g0 = 0.0, g1 = 0.0, g2 = 0.0, g3 = 0.0;
+        int c = way;
+        for (; c + 3 * ways < (int)gridDim.x; c += 4 * ways) {
+            g0 += __ldcg(a.part + (int64_t)c * ne + j);
+            g1 += __ldcg(a.part + (int64_t)(c + ways) * ne + j);
+            g2 += __ldcg(a.part + (int64_t)(c + 2 * ways) * ne + j);
+            g3 += __ldcg(a.part + (int64_t)(c + 3 * ways) * ne + j);
+        }
+        for (; c < (int)gridDim.x; c += ways) g0 += __ldcg(a.part + (int64_t)c * ne + j);
+        s_m[way * ne + j] = (g0 + g1) + (g2 + g3);
+    }
+    __syncthreads();
+    for (int j = tid; j < ne; j += kThreads) {
+        double g = 0.0;
+        for (int k = 0; k < ways; ++k) g += s_m[k * ne + j];
+        if (j < a.nt) a.G[j] = a.gsign * g;
+        else if (a.negLogL) *a.negLogL = -((g != 0.0) ? g : -INFINITY);  // fitting_base.jl:95
+    }
+    if (tid == 0) *a.counter = 0u;  // re-arm for the next launch on this stream
+}
+
 // ---------------------------------------------------------------- fused pass 1 (FP32 storage)
 // m partials over template splits (register double-buffered loads).  The last split
 // block to finish a row tile sums its rows' partials in split order, forms the FP64
@@ -740,6 +862,24 @@ int sfh_launch_fg(sfh_ctx *ctx, const sfh_models *m, const FgArgs &a, cudaEvent_
         return sfh_launch_fg_onepass(ctx, const_cast<sfh_models *>(m), a.coeffs, a.data,
                                      a.composite, a.G, a.negLogL, a.eps, a.gsign, ctx->scratch, ev,
                                      a.skip, a.occ_key);
+    }
+    if (f64 && a.mode == FG_MODE_FG && a.G && a.data && tile64_fits(ctx, nbins, nt)) {
+        const int grid = (int)((nbins + kTile64 - 1) / kTile64);
+        int rc = sfh_scratch_reserve(ctx, (size_t)grid * (nt + 1) * sizeof(double));
+        if (rc) return rc;
+        static thread_local bool attr_set = false;
+        if (!attr_set) {
+            SFH_CK(ctx, cudaFuncSetAttribute(k_fg_tile_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             213 * 1024));
+            attr_set = true;
+        }
+        if (ev) SFH_CK(ctx, cudaEventRecord(ev[0], ctx->stream));
+        k_fg_tile_f64<<<grid, kThreads, tile64_smem(nt), ctx->stream>>>(
+            Tile64Args{(const double *)Mptr, nbins, (int)nt, a.coeffs, a.data, a.eps, a.composite, a.G,
+                       a.negLogL, a.gsign, (double *)ctx->scratch, ctx->d_counters + SFH_CNT_LOGL});
+        SFH_LAUNCHED(ctx);
+        for (int k = 1; ev && k < 5; ++k) SFH_CK(ctx, cudaEventRecord(ev[k], ctx->stream));
+        return SFH_OK;
     }
     const bool fused_path = !f64 && (a.mode == FG_MODE_FG || a.mode == FG_MODE_COMPOSITE);
     const Plan p = make_plan(ctx, nbins, nt, f64, fused_path, m);
