@@ -33,6 +33,7 @@ struct sfh_galaxies {
     int64_t n_fused_tiles;  // tiles of galaxies with <= kFuseMax templates
     int64_t n_fused_gal, n_big_gal, max_fused_nt;
     int64_t n_fused_class[3];  // fused tiles with nt <= 8, <= 16, <= 32 (in that order)
+    int64_t max_nt_class[3];   // largest nt of each
     void *d_desc;       // GalDesc[ngal]
     void *d_rows;       // RowTile[n_row_tiles] (two-pass galaxies)
     void *d_cols;       // ColTile[n_col_tiles] (two-pass galaxies)
@@ -80,8 +81,7 @@ __device__ __forceinline__ void block_sum(double v, double *s_red, double *out) 
 // One bin's share of fg!: the model m = ah + al (compensated), the Poisson term in
 // double-float (sfh_dfloat.cuh) and w = 1 - n / max(m, eps) (fitting_base.jl:90-93,
 // 274-280); composite receives w when the gradient is wanted, the model otherwise.
-__device__ __forceinline__ void bin_terms(float ah, float al, const double *__restrict__ data,
-                                          int64_t ii, float eps_f, int want_logl, int want_w,
+__device__ __forceinline__ void bin_terms(float ah, float al, double n, int64_t ii, float eps_f, int want_logl, int want_w,
                                           const sfh_df *s_tab, double *__restrict__ composite,
                                           sfh_df &term, float &w) {
     sfh_df c = df_fast_two_sum(ah, al);
@@ -90,7 +90,7 @@ __device__ __forceinline__ void bin_terms(float ah, float al, const double *__re
     // max(composite, eps(T)); eps(T) is a power of two, exact in FP32
     if (c.h < eps_f || (c.h == eps_f && c.l < 0.f)) c = sfh_df{eps_f, 0.f};
     float nh, nl;
-    sfh_split_double(data[ii], nh, nl);
+    sfh_split_double(n, nh, nl);
     if (want_logl)
         term = df_add(term, sfh_bin_term(c, nh, nl, s_tab));
     if (want_w) {
@@ -152,7 +152,8 @@ k_ragged_pass1(const float *__restrict__ M, const GalDesc *__restrict__ gals,
     if (live) {
         const int64_t ii = G.boff + i;
         float w = 0.f;
-        bin_terms(ah, al, data, ii, eps, want_logl, want_w, s_tab, composite, term, w);
+        const double n = want_logl || want_w ? data[ii] : 0.0;
+        bin_terms(ah, al, n, ii, eps, want_logl, want_w, s_tab, composite, term, w);
         if (want_w) w32[ii] = w;
     }
     if (want_logl) {
@@ -206,6 +207,32 @@ k_ragged_pass2(const float *__restrict__ M, const GalDesc *__restrict__ gals,
 // tile's partial G = Mᵀ w (gpart, kFuseMax doubles per tile).  Tiles tile_base + blockIdx.x
 // of the fused list; each thread takes kFuseRows bins (rows row0 + r * kRT + tid), so the
 // table load, the block reduction and the transpose are paid once per kFuseRows * kRT bins.
+//
+// HBM and instruction issue bound it.  The loads of a row of M are asynchronous copies into
+// shared memory, kept fused_depth(NT) rows ahead (each thread copies and reads only its own
+// elements, so no barrier; bins past the end and templates up to a multiple of four are
+// zeroed).  256 galaxies of 12 templates (431 MB): 210 us with the rows loaded as they were
+// needed, 181 us now (2.4 TB/s; the arithmetic of a bin, about 600 instructions, is the rest).
+__host__ __device__ constexpr int fused_depth(int NT) { return NT <= 16 ? kFuseRows : 2; }
+__host__ __device__ inline int64_t fused_pad(int64_t nt) { return (nt + 3) / 4 * 4; }
+size_t fused_smem(int NT, int64_t nt) {  // counts, then rows of M: [depth][pad][kRT]
+    return (size_t)fused_depth(NT) * kRT * (8 + 4 * (size_t)fused_pad(nt));
+}
+
+// `bytes` (0 or the size) are read, the rest of the element is zeroed.
+__device__ __forceinline__ void copy4_async(void *smem, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(smem)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void copy8_async(void *smem, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(smem)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+
 template <int NT>
 __global__ void __launch_bounds__(kRT, NT <= 8 ? 4 : NT <= 16 ? 3 : 2)
 k_ragged_fused(const float *__restrict__ M, const GalDesc *__restrict__ gals,
@@ -213,20 +240,40 @@ k_ragged_fused(const float *__restrict__ M, const GalDesc *__restrict__ gals,
                const double *__restrict__ data, double *__restrict__ composite,
                double *__restrict__ tile_logl, double *__restrict__ gpart, float eps,
                int want_logl, int want_g, const sfh_df *__restrict__ tab, int tile_base) {
-    __shared__ float rhi[NT], rlo[NT];
+    __shared__ float2 s_r[NT];  // coefficients, hi and lo
     __shared__ double s_red[kRT / 32];
     __shared__ float s_g[kRT / 32][NT];
     __shared__ sfh_df s_tab[SFH_DF_TAB_ALL];
-    for (int k = threadIdx.x; k < SFH_DF_TAB_ALL; k += kRT) s_tab[k] = tab[k];
+    constexpr int D = fused_depth(NT);
+    extern __shared__ double s_n[];                            // [D][kRT]
+    float *s_m = reinterpret_cast<float *>(s_n + D * kRT);     // [D][pad][kRT]
     const int64_t t = (int64_t)tile_base + blockIdx.x;
     const RowTile tile = tiles[t];
     const GalDesc G = gals[tile.g];
-    const int nt = (int)G.nt;
+    const int nt = (int)G.nt, pad = (int)fused_pad(nt);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const auto fetch = [&](int r) {  // row r of the thread's bins; an empty group past the end
+        if (r < kFuseRows && (int64_t)tile.row0 + r * kRT < G.nbins) {
+            const int64_t i = (int64_t)tile.row0 + r * kRT + threadIdx.x;
+            const int have = i < G.nbins;
+            float *to = s_m + (size_t)(r % D) * pad * kRT + threadIdx.x;
+            const float *col = have ? M + G.moff + i : M;
+            const int64_t step = have ? G.nbins : 0;
+#pragma unroll 4
+            for (int j = 0; j < nt; ++j, col += step) copy4_async(to + j * kRT, col, 4 * have);
+            if (data) copy8_async(s_n + (r % D) * kRT + threadIdx.x, have ? data + G.boff + i : data, 8 * have);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int r = 0; r < D; ++r) fetch(r);
+    for (int r = 0; r < D; ++r)
+        for (int j = nt; j < pad; ++j) s_m[((size_t)r * pad + j) * kRT + threadIdx.x] = 0.f;
+    for (int k = threadIdx.x; k < SFH_DF_TAB_ALL; k += kRT) s_tab[k] = tab[k];
     if (threadIdx.x < NT) {
         const double v = threadIdx.x < nt ? coeffs[G.toff + threadIdx.x] : 0.0;
         const float h = __double2float_rn(v);
-        rhi[threadIdx.x] = h;
-        rlo[threadIdx.x] = __double2float_rn(v - (double)h);
+        s_r[threadIdx.x] = make_float2(h, __double2float_rn(v - (double)h));
     }
     __syncthreads();
     sfh_df term{0.f, 0.f};
@@ -238,16 +285,17 @@ k_ragged_fused(const float *__restrict__ M, const GalDesc *__restrict__ gals,
         if ((int64_t)tile.row0 + r * kRT >= G.nbins) break;  // uniform over the CTA
         const int64_t i = (int64_t)tile.row0 + r * kRT + threadIdx.x;
         const bool live = i < G.nbins;
-        const float *col = M + G.moff + i;
+        asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");  // row r has landed
+        const float *own = s_m + (size_t)(r % D) * pad * kRT + threadIdx.x;
         // templates in groups of four behind branches that are uniform over the CTA (one
         // galaxy per tile): a galaxy with nt < NT issues no loads or products for the rest
         float m[NT];
 #pragma unroll
         for (int j0 = 0; j0 < NT; j0 += 4)
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                m[j0 + u] = (j0 < nt && live && j0 + u < nt)
-                                ? __ldg(col + (int64_t)(j0 + u) * G.nbins) : 0.f;
+            for (int u = 0; u < 4; ++u) m[j0 + u] = j0 < nt ? own[(j0 + u) * kRT] : 0.f;
+        const double n_i = data ? s_n[(r % D) * kRT + threadIdx.x] : 0.0;
+        fetch(r + D);
         // the bin's products summed error-free against a power-of-two anchor from the bin's
         // own bound sum_j |M_ij| |r_j| (sfh_anc_acc)
         float b = 0.f;
@@ -255,7 +303,7 @@ k_ragged_fused(const float *__restrict__ M, const GalDesc *__restrict__ gals,
         for (int j0 = 0; j0 < NT; j0 += 4) {
             if (j0 >= nt) break;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) b = fmaf(fabsf(m[j0 + u]), fabsf(rhi[j0 + u]), b);
+            for (int u = 0; u < 4; ++u) b = fmaf(fabsf(m[j0 + u]), fabsf(s_r[j0 + u].x), b);
         }
         const float sg = sfh_anchor(b * 1.0009765625f);
         float aa = sg, lo = 0.f;
@@ -263,12 +311,14 @@ k_ragged_fused(const float *__restrict__ M, const GalDesc *__restrict__ gals,
         for (int j0 = 0; j0 < NT; j0 += 4) {
             if (j0 >= nt) break;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) sfh_anc_acc(aa, lo, m[j0 + u], rhi[j0 + u], rlo[j0 + u]);
+            for (int u = 0; u < 4; ++u) {
+                const float2 c = s_r[j0 + u];
+                sfh_anc_acc(aa, lo, m[j0 + u], c.x, c.y);
+            }
         }
         const sfh_df cm = sfh_anc_result(aa, lo, sg);
-        const float ah = cm.h, al = cm.l;
         float w = 0.f;
-        if (live) bin_terms(ah, al, data, G.boff + i, eps, want_logl, want_g, s_tab, composite, term, w);
+        if (live) bin_terms(cm.h, cm.l, n_i, G.boff + i, eps, want_logl, want_g, s_tab, composite, term, w);
         __syncwarp();  // reconverge after the lane-dependent tail
 #pragma unroll
         for (int j0 = 0; j0 < NT; j0 += 4) {
@@ -286,7 +336,6 @@ k_ragged_fused(const float *__restrict__ M, const GalDesc *__restrict__ gals,
     // warp transpose-reduce over NT templates: after the step with offset o (o < NT)
     // each lane keeps o partial column sums; lanes that differ only in bits >= log2(NT)
     // hold the same columns and are folded first.  Lane l then holds template l % NT.
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o >= NT; o >>= 1)
 #pragma unroll
@@ -387,12 +436,13 @@ extern "C" int sfh_galaxies_create(sfh_ctx *ctx, const float *d_models, int64_t 
         maxnt = std::max(maxnt, h.ntempl);
     }
     // fused tiles grouped by register class (nt <= 8, <= 16, <= 32): one launch per class
-    int64_t ncls[3] = {0, 0, 0};
+    int64_t ncls[3] = {0, 0, 0}, maxnt_cls[3] = {0, 0, 0};
     for (int c = 0; c < 3; ++c) {
         const int64_t before = (int64_t)fused.size();
         for (int32_t g : fused_ids) {
             GalDesc &d = desc[(size_t)g];
             if (fused_class(d.nt) != c) continue;
+            maxnt_cls[c] = std::max(maxnt_cls[c], d.nt);
             d.tile0 = (int64_t)fused.size();
             for (int64_t r0 = 0; r0 < d.nbins; r0 += kFuseStep)
                 fused.push_back(RowTile{(int32_t)g, (int32_t)r0});
@@ -421,7 +471,10 @@ extern "C" int sfh_galaxies_create(sfh_ctx *ctx, const float *d_models, int64_t 
     G->n_big_gal = (int64_t)big_ids.size();
     G->max_nt = maxnt;
     G->max_fused_nt = maxfnt;
-    for (int c = 0; c < 3; ++c) G->n_fused_class[c] = ncls[c];
+    for (int c = 0; c < 3; ++c) {
+        G->n_fused_class[c] = ncls[c];
+        G->max_nt_class[c] = maxnt_cls[c];
+    }
     G->d_models = d_models;
     void **bufs[] = {&G->d_desc, &G->d_rows, &G->d_cols, &G->d_fused, &G->d_fused_ids, &G->d_big_ids};
     const void *src[] = {desc.data(), rows.data(), cols.data(), fused.data(), fused_ids.data(),
@@ -489,11 +542,15 @@ extern "C" int sfh_fg_ragged_dev(sfh_ctx *ctx, const sfh_galaxies *gal, const do
     if (gal->n_fused_gal) {
         decltype(&k_ragged_fused<8>) kerns[3] = {k_ragged_fused<8>, k_ragged_fused<16>,
                                                  k_ragged_fused<32>};
+        const int width[3] = {8, 16, 32};
         int64_t base = 0;
         for (int c = 0; c < 3; ++c) {
             const int64_t n = gal->n_fused_class[c];
             if (!n) continue;
-            kerns[c]<<<(unsigned)n, kRT, 0, st>>>(
+            const size_t smem = fused_smem(width[c], gal->max_nt_class[c]);
+            SFH_CK(ctx, cudaFuncSetAttribute(kerns[c], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)fused_smem(width[c], width[c])));
+            kerns[c]<<<(unsigned)n, kRT, smem, st>>>(
                 gal->d_models, desc, (const RowTile *)gal->d_fused, d_coeffs, d_data, d_composite,
                 tf, gp, (float)eps, want_logl ? 1 : 0, want_w ? 1 : 0, ctx->d_df_tab, (int)base);
             SFH_LAUNCHED(ctx);
