@@ -1628,59 +1628,101 @@ k_bin_prefac(IsoParams P, const double *__restrict__ m, const int64_t *__restric
     }
 }
 
-// fluxes of the two colour filters and the magnitude filter (:644), and IMF values.
+// fluxes of the two colour filters, of which one is the magnitude filter (:644, :700), and
+// IMF values.
 __global__ void k_bin_flux(IsoParams P, const double *__restrict__ m, const double *__restrict__ mags,
                            int64_t total, double *__restrict__ fl, double *__restrict__ imfv) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    const int fs[3] = {P.c1, P.c2, P.y_index};
+    const int fs[2] = {P.c1, P.c2};
 #pragma unroll
-    for (int q = 0; q < 3; ++q) fl[q * total + i] = exp10(-0.4 * mags[(int64_t)fs[q] * total + i]);
+    for (int q = 0; q < 2; ++q) fl[q * total + i] = exp10(-0.4 * mags[(int64_t)fs[q] * total + i]);
     imfv[i] = imf_pdf(P, m[i]);
 }
 
-// left-closed histogram bin of v (edges first + k step, step > 0), -1 outside
-__device__ __forceinline__ int hist_bin(double v, double first, double step, int n) {
-    if (!(v >= first)) return -1;
-    int k = (int)floor((v - first) / step);
-    if (k > 0 && v < first + (double)k * step) --k;
-    if (v >= first + (double)(k + 1) * step) ++k;
+// left-closed histogram bin of v (edges first + k step, step > 0), -1 outside: the product with
+// the inverse step, and the edges themselves only within 1e-6 bins of one
+__device__ __forceinline__ int hist_bin(double v, double first, double step, double inv, int n) {
+    const double q = (v - first) * inv;
+    if (!(q >= -1.0 && q <= (double)n)) return -1;
+    int k = __double2int_rd(q);
+    const float frac = (float)(q - (double)k);
+    if (frac < 1e-6f || frac > 1.f - 1e-6f) {
+        if (!(v >= first)) return -1;
+        k = max(k, 0);
+        if (k > 0 && v < first + (double)k * step) --k;
+        if (v >= first + (double)(k + 1) * step) ++k;
+    }
     return (k >= 0 && k < n) ? k : -1;
 }
 
-// Grid: x -> j blocks, y -> i, z -> template (chunk-relative).  hist is [chunk][nx*ny].
+// Natural logarithm by a table (Tang, 1990): x = 2^e c_j (1 + r), c_j = 1 + j / 128, and the
+// series of log1p(r) to r^7 (|r| < 2^-7: the rest is below 2e-18).  About a dozen FP64
+// operations; s_log[j] = (1 / c_j, log c_j).
+__device__ __forceinline__ double log_table(double x, const double2 *s_log) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)(b >> 52) - 1023, j = (int)(b >> 45) & 127;
+    if (e < -1000 || e > 1000) return log(x);  // negative, subnormal, huge, inf or NaN
+    const double m = __longlong_as_double((long long)((b & 0xfffffffffffffull) | 0x3ff0000000000000ull));
+    const double c = __longlong_as_double((long long)((b & 0xfe00000000000ull) | 0x3ff0000000000000ull));
+    const double2 t = s_log[j];
+    const double r = (m - c) * t.x;
+    double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
+    p = fma(r, p, 1.0 / 5.0);
+    p = fma(r, p, -1.0 / 4.0);
+    p = fma(r, p, 1.0 / 3.0);
+    p = fma(r, p, -1.0 / 2.0);
+    return fma((double)e, 0.6931471805599453, t.y) + fma(r * r, p, r);
+}
+
+// Grid: x -> left points i (a warp each), y -> template (chunk-relative); the lanes take the
+// pairs' right points j.  hist is [chunk][nx*ny].  FP64 throughput bounds it: with three library
+// log10 and two divisions a pair, 60 templates of 300 points took 946 us, now 480 us.
 __global__ void __launch_bounds__(kPairThreads)
 k_bin_pairs(IsoParams P, const double *__restrict__ m, const double *__restrict__ fl,
             const double *__restrict__ imfv, int64_t total, const int64_t *__restrict__ off,
             const int32_t *__restrict__ len, const double *__restrict__ prefac, Grid2 g,
-            int t0, double *__restrict__ hist) {
-    const int t = t0 + blockIdx.z, n = len[t], ns = n - 1;
-    const int i = blockIdx.y, j = i + 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ns || j >= ns) return;
+            const sfh_df *__restrict__ tab, int t0, double *__restrict__ hist) {
+    __shared__ double2 s_log[128];
+    if (threadIdx.x < 128)
+        s_log[threadIdx.x] = make_double2(128.0 / (128.0 + (double)threadIdx.x),
+                                          (double)tab[threadIdx.x].h + (double)tab[threadIdx.x].l);
+    __syncthreads();
+    const int t = t0 + blockIdx.y, ns = len[t] - 1, lane = threadIdx.x & 31;
     const int64_t o = off[t];
     const double *mt = m + o, *iv = imfv + o;
-    const double *f1 = fl + o, *f2 = fl + total + o, *fy = fl + 2 * total + o;
-    // flux2mag(f) = -5 log10(f) / 2 (:656)
-    const double bm1 = -2.5 * log10(f1[i] + f1[j]);
-    const double bm2 = -2.5 * log10(f2[i] + f2[j]);
-    const double bmy = -2.5 * log10(fy[i] + fy[j]);
-    double w = (mt[i + 1] - mt[i]) * (mt[j + 1] - mt[j]) * (iv[i] + iv[i + 1]) * (iv[j] + iv[j + 1]) *
-               prefac[t];
-    w *= compl_eval(P, P.c1, bm1) * compl_eval(P, P.c2, bm2);
-    const double col = (bm1 + P.bias[P.c1]) - (bm2 + P.bias[P.c2]);
-    const double ym = bmy + P.bias[P.y_index];
-    const int ix = hist_bin(col, g.xf, g.xs, g.nx), iy = hist_bin(ym, g.yf, g.ys, g.ny);
-    if (ix >= 0 && iy >= 0)
-        atomicAdd(hist + (int64_t)blockIdx.z * g.nx * g.ny + ix + (int64_t)g.nx * iy, w);
+    const double *f1 = fl + o, *f2 = fl + total + o;
+    double *h = hist + (int64_t)blockIdx.y * g.nx * g.ny;
+    const double k = -1.0857362047581296, pre = prefac[t];  // flux2mag(f) = -2.5 log10 f (:656)
+    for (int i = blockIdx.x * (kPairThreads / 32) + (threadIdx.x >> 5); i < ns;
+         i += gridDim.x * (kPairThreads / 32)) {
+        const double fi1 = f1[i], fi2 = f2[i], wi = (mt[i + 1] - mt[i]) * (iv[i] + iv[i + 1]) * pre;
+        for (int j = i + 1 + lane; j < ns; j += 32) {
+            const double bm1 = k * log_table(fi1 + f1[j], s_log), bm2 = k * log_table(fi2 + f2[j], s_log);
+            double w = wi * ((mt[j + 1] - mt[j]) * (iv[j] + iv[j + 1]));
+            // the product of the two colour filters' completeness (compl_eval) over one division
+            const double e1 = (double)__expf((float)((bm1 - P.cm50[P.c1]) * P.crho_inv[P.c1]));
+            const double e2 = (double)__expf((float)((bm2 - P.cm50[P.c2]) * P.crho_inv[P.c2]));
+            w *= P.cA[P.c1] * P.cA[P.c2] * rcp_nr((1.0 + e1) * (1.0 + e2));
+            const double col = (bm1 + P.bias[P.c1]) - (bm2 + P.bias[P.c2]);
+            // the magnitude is one of the colour's (:700)
+            const double ym = (P.y_index == P.c1 ? bm1 : bm2) + P.bias[P.y_index];
+            const int ix = hist_bin(col, g.xf, g.xs, g.ixs, g.nx), iy = hist_bin(ym, g.yf, g.ys, g.iys, g.ny);
+            if (ix >= 0 && iy >= 0) atomicAdd(h + ix + (int64_t)g.nx * iy, w);
+        }
+    }
 }
 
-// nonzero bins of each template (one block per template of the chunk)
+// Nonzero bins of a segment of kSegBins bins: x -> segment, y -> template of the chunk.
+constexpr int kSegBins = 4096;
+
 __global__ void __launch_bounds__(kPairThreads)
 k_bin_count(const double *__restrict__ hist, int64_t nbins, int32_t *__restrict__ cnt) {
     __shared__ int s_red[kPairThreads / 32];
-    const double *h = hist + (int64_t)blockIdx.x * nbins;
+    const double *h = hist + (int64_t)blockIdx.y * nbins;
+    const int64_t k0 = (int64_t)blockIdx.x * kSegBins, k1 = min(nbins, k0 + kSegBins);
     int c = 0;
-    for (int64_t k = threadIdx.x; k < nbins; k += blockDim.x) c += h[k] != 0.0;
+    for (int64_t k = k0 + threadIdx.x; k < k1; k += kPairThreads) c += h[k] != 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = c;
@@ -1688,35 +1730,52 @@ k_bin_count(const double *__restrict__ hist, int64_t nbins, int32_t *__restrict_
     if (threadIdx.x == 0) {
         int tot = 0;
         for (int w = 0; w < kPairThreads / 32; ++w) tot += s_red[w];
-        cnt[blockIdx.x] = tot;
+        cnt[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
     }
 }
 
-// points of the nonzero bins in bin order (x fastest), at start[t]: thread q takes a
-// contiguous range of bins; a block scan of the range counts gives its first point.
+// Records of the nonzero bins in bin order (x fastest): the segment's first point is number
+// first[] of its template.  The bins are listed first, so that the FP64 work of a record is
+// done by full warps (few bins of a segment hold pairs).
 __global__ void __launch_bounds__(kPairThreads)
 k_bin_points(IsoParams P, const double *__restrict__ hist, Grid2 g, const int64_t *__restrict__ start,
-             double *__restrict__ px, double *__restrict__ py, double *__restrict__ psx,
-             double *__restrict__ psy, double *__restrict__ pw) {
-    __shared__ int s_scan[kPairThreads];
+             const int32_t *__restrict__ first, int cov, StarRec *__restrict__ rec,
+             StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
+    __shared__ int s_list[kSegBins];
+    __shared__ int s_red[kPairThreads / 32];
     const int64_t nbins = (int64_t)g.nx * g.ny;
-    const double *h = hist + (int64_t)blockIdx.x * nbins;
-    const int64_t per = (nbins + kPairThreads - 1) / kPairThreads;
-    const int64_t k0 = (int64_t)threadIdx.x * per, k1 = k0 + per < nbins ? k0 + per : nbins;
-    int c = 0;
-    for (int64_t k = k0; k < k1; ++k) c += h[k] != 0.0;
-    s_scan[threadIdx.x] = c;
-    __syncthreads();
-    for (int o = 1; o < kPairThreads; o <<= 1) {  // inclusive scan (Hillis-Steele)
-        const int v = threadIdx.x >= o ? s_scan[threadIdx.x - o] : 0;
-        __syncthreads();
-        s_scan[threadIdx.x] += v;
-        __syncthreads();
+    const double *h = hist + (int64_t)blockIdx.y * nbins;
+    const int64_t k0 = (int64_t)blockIdx.x * kSegBins;
+    const int len = (int)min(nbins - k0, (int64_t)kSegBins);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // a warp's share: consecutive bins, 32 at a time
+    constexpr int kShare = kSegBins / (kPairThreads / 32);
+    unsigned masks[kShare / 32];
+    int mine = 0;
+#pragma unroll
+    for (int c = 0; c < kShare / 32; ++c) {
+        const int k = warp * kShare + c * 32 + lane;
+        masks[c] = __ballot_sync(0xffffffffu, k < len && h[k0 + k] != 0.0);
+        mine += __popc(masks[c]);
     }
-    int64_t q = start[blockIdx.x] + s_scan[threadIdx.x] - c;
+    if (lane == 0) s_red[warp] = mine;
+    __syncthreads();
+    int at = 0, all = 0;
+#pragma unroll
+    for (int v = 0; v < kPairThreads / 32; ++v) {
+        at += v < warp ? s_red[v] : 0;
+        all += s_red[v];
+    }
+#pragma unroll
+    for (int c = 0; c < kShare / 32; ++c) {
+        if (masks[c] >> lane & 1u) s_list[at + __popc(masks[c] & ((1u << lane) - 1u))] = warp * kShare + c * 32 + lane;
+        at += __popc(masks[c]);
+    }
+    __syncthreads();
+    const int q0 = first[(int64_t)blockIdx.y * gridDim.x + blockIdx.x];
     const int xc = (P.c1 != P.y_index) ? P.c1 : P.c2;
-    for (int64_t k = k0; k < k1; ++k) {
-        if (h[k] == 0.0) continue;
+    for (int p = threadIdx.x; p < all; p += kPairThreads) {
+        const int64_t k = k0 + s_list[p];
         const int ix = (int)(k % g.nx), iy = (int)(k / g.nx);
         // edges[k] + step / 2 (:688-689) with the edge correctly rounded by one fma and no
         // further contraction: the centre is a rounding tie of the stamp's pixel
@@ -1724,12 +1783,9 @@ k_bin_points(IsoParams P, const double *__restrict__ hist, Grid2 g, const int64_
         const double cx = __dadd_rn(__fma_rn((double)ix, g.xs, g.xf), g.xs / 2.0);
         const double cy = __dadd_rn(__fma_rn((double)iy, g.ys, g.yf), g.ys / 2.0);
         const double xmag = (P.y_index == P.c1) ? cy - cx : cy + cx;  // :692-695
-        px[q] = cx;
-        py[q] = cy;
-        psx[q] = err_eval(P, xc, xmag);
-        psy[q] = err_eval(P, P.y_index, cy);
-        pw[q] = h[k];
-        ++q;
+        StarRec r{};
+        star_record(r, g, cx, cy, err_eval(P, xc, xmag), err_eval(P, P.y_index, cy), h[k], cov);
+        store_record(r, g, StarId{(int)blockIdx.y, q0 + p}, rec + start[blockIdx.y] + q0 + p, narrow, n_narrow);
     }
 }
 
@@ -1774,76 +1830,93 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
     SFH_CK(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const int64_t nbins = nx * ny;
-    // per-call buffers (template builds are not latency critical)
     const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(ntempl, (256ll << 20) / (nbins * 8)));
-    double *fl = nullptr, *imfv = nullptr, *prefac = nullptr, *hist = nullptr, *d_norm = nullptr;
-    int64_t *d_off = nullptr, *d_start = nullptr;
-    int32_t *d_len = nullptr, *d_cnt = nullptr, *d_cov = nullptr;
-    double *pts = nullptr;
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(st);
-        for (void *p : {(void *)fl, (void *)imfv, (void *)prefac, (void *)hist, (void *)d_norm,
-                        (void *)d_off, (void *)d_start, (void *)d_len, (void *)d_cnt, (void *)d_cov,
-                        (void *)pts})
-            if (p) cudaFree(p);
+    const int64_t nseg = (nbins + kSegBins - 1) / kSegBins;
+    const int cov = y_index == c1 ? -1 : 1;  // :698
+    // scratch: per-template inputs (one upload), fluxes, IMF values, prefactors, then the
+    // chunk's starts, counts and firsts (one upload) and pair histograms; the records, whose
+    // number is known after the count, go into the staging buffer
+    std::vector<char> head;
+    auto add = [&](const void *src, size_t bytes) {
+        const size_t at = head.size();
+        head.resize(at + sfh_align256(bytes), 0);
+        if (src) std::memcpy(head.data() + at, src, bytes);
+        return at;
     };
-    cudaError_t e = cudaSuccess;
-    if ((e = cudaMalloc(&fl, 3 * total_points * 8)) || (e = cudaMalloc(&imfv, total_points * 8)) ||
-        (e = cudaMalloc(&prefac, ntempl * 8)) || (e = cudaMalloc(&hist, chunk * nbins * 8)) ||
-        (e = cudaMalloc(&d_norm, ntempl * 8)) || (e = cudaMalloc(&d_off, ntempl * 8)) ||
-        (e = cudaMalloc(&d_start, chunk * 8)) || (e = cudaMalloc(&d_len, ntempl * 4)) ||
-        (e = cudaMalloc(&d_cnt, chunk * 4)) || (e = cudaMalloc(&d_cov, chunk * 4))) {
-        cleanup();
-        return sfh_cuda_error(ctx, e, "binary_hess buffers");
-    }
-    cudaMemcpyAsync(d_norm, h_norm, ntempl * 8, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(d_off, h_off, ntempl * 8, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(d_len, h_len, ntempl * 4, cudaMemcpyHostToDevice, st);
-    std::vector<int32_t> hcov((size_t)chunk, y_index == c1 ? -1 : 1);  // :698
-    cudaMemcpyAsync(d_cov, hcov.data(), chunk * 4, cudaMemcpyHostToDevice, st);
+    const std::vector<int32_t> hcov((size_t)chunk, cov);
+    const size_t o_norm = add(h_norm, ntempl * 8), o_off = add(h_off, ntempl * 8);
+    const size_t o_len = add(h_len, ntempl * 4), o_cov = add(hcov.data(), chunk * 4);
+    size_t at = head.size();
+    auto carve = [&](size_t bytes) {
+        const size_t o = at;
+        at += sfh_align256(bytes);
+        return o;
+    };
+    const size_t o_fl = carve(2 * total_points * 8), o_imf = carve(total_points * 8), o_pre = carve(ntempl * 8);
+    const size_t up = sfh_align256(256) + sfh_align256(chunk * 8) + sfh_align256(chunk * 4);
+    const size_t o_up = carve(up + chunk * nseg * 4);  // narrow counter, starts, counts, firsts
+    const size_t o_seg = carve(chunk * nseg * 4), o_hist = carve(chunk * nbins * 8);
+    if ((rc = sfh_scratch_reserve(ctx, at))) return rc;
+    char *b = (char *)ctx->scratch;
+    const int64_t *d_off = (const int64_t *)(b + o_off);
+    const int32_t *d_len = (const int32_t *)(b + o_len);
+    double *fl = (double *)(b + o_fl), *imfv = (double *)(b + o_imf), *prefac = (double *)(b + o_pre);
+    double *hist = (double *)(b + o_hist);
+    SFH_CK(ctx, cudaMemcpyAsync(b, head.data(), head.size(), cudaMemcpyHostToDevice, st));
     k_bin_flux<<<(unsigned)((total_points + 255) / 256), 256, 0, st>>>(P, d_m_ini, d_mags, total_points,
                                                                     fl, imfv);
-    k_bin_prefac<<<(unsigned)ntempl, kPairThreads, 0, st>>>(P, d_m_ini, d_off, d_len, d_norm, prefac);
-    ctx->launches += 2;
+    SFH_LAUNCHED(ctx);
+    k_bin_prefac<<<(unsigned)ntempl, kPairThreads, 0, st>>>(P, d_m_ini, d_off, d_len,
+                                                            (const double *)(b + o_norm), prefac);
+    SFH_LAUNCHED(ctx);
     const Grid2 g = make_grid(x_first, x_step, nx, y_first, y_step, ny);
-    std::vector<int32_t> hcnt((size_t)chunk);
-    std::vector<int64_t> hstart((size_t)chunk);
-    size_t pts_cap = 0;
-    for (int64_t t0 = 0; t0 < ntempl && rc == SFH_OK; t0 += chunk) {
+    std::vector<int32_t> seg((size_t)(chunk * nseg));
+    std::vector<char> hup(up + (size_t)(chunk * nseg) * 4, 0);
+    int64_t *starts = (int64_t *)(hup.data() + 256);
+    int32_t *counts = (int32_t *)(hup.data() + 256 + sfh_align256(chunk * 8));
+    int32_t *firsts = (int32_t *)(hup.data() + up);
+    for (int64_t t0 = 0; t0 < ntempl; t0 += chunk) {
         const int64_t nc = std::min(chunk, ntempl - t0);
-        if ((e = cudaMemsetAsync(hist, 0, nc * nbins * 8, st))) { rc = sfh_cuda_error(ctx, e, "memset"); break; }
-        dim3 grid((unsigned)((nmax + kPairThreads - 1) / kPairThreads), (unsigned)(nmax - 1), (unsigned)nc);
+        SFH_CK(ctx, cudaMemsetAsync(hist, 0, nc * nbins * 8, st));
+        const dim3 grid((unsigned)((nmax - 1 + kPairThreads / 32 - 1) / (kPairThreads / 32)), (unsigned)nc);
         k_bin_pairs<<<grid, kPairThreads, 0, st>>>(P, d_m_ini, fl, imfv, total_points, d_off, d_len,
-                                                    prefac, g, (int)t0, hist);
-        k_bin_count<<<(unsigned)nc, kPairThreads, 0, st>>>(hist, nbins, d_cnt);
-        ctx->launches += 2;
-        if ((e = cudaMemcpyAsync(hcnt.data(), d_cnt, nc * 4, cudaMemcpyDeviceToHost, st)) ||
-            (e = cudaStreamSynchronize(st))) { rc = sfh_cuda_error(ctx, e, "binary_hess counts"); break; }
-        int64_t tot = 0;
-        for (int64_t q = 0; q < nc; ++q) { hstart[(size_t)q] = tot; tot += hcnt[(size_t)q]; }
-        int64_t maxcount = 0;
-        for (int64_t q = 0; q < nc; ++q) maxcount = std::max<int64_t>(maxcount, hcnt[(size_t)q]);
-        const int64_t np = std::max<int64_t>(tot, 1);
-        const size_t a8 = sfh_align256((size_t)np * 8);
-        const size_t need = 5 * a8 + StampWork::bytes(tot, node_bytes(g, nc));
-        if (need > pts_cap) {
-            if (pts) cudaFree(pts);
-            pts = nullptr;
-            if ((e = cudaMalloc(&pts, need))) { rc = sfh_cuda_error(ctx, e, "binary_hess points"); break; }
-            pts_cap = need;
+                                                    prefac, g, ctx->d_df_tab, (int)t0, hist);
+        SFH_LAUNCHED(ctx);
+        k_bin_count<<<dim3((unsigned)nseg, (unsigned)nc), kPairThreads, 0, st>>>(hist, nbins,
+                                                                                 (int32_t *)(b + o_seg));
+        SFH_LAUNCHED(ctx);
+        SFH_CK(ctx, cudaMemcpyAsync(seg.data(), b + o_seg, nc * nseg * 4, cudaMemcpyDeviceToHost, st));
+        SFH_CK(ctx, cudaStreamSynchronize(st));
+        int64_t tot = 0, maxcount = 0;
+        for (int64_t q = 0; q < nc; ++q) {
+            int32_t c = 0;
+            for (int64_t k = 0; k < nseg; ++k) {
+                firsts[q * nseg + k] = c;
+                c += seg[(size_t)(q * nseg + k)];
+            }
+            starts[q] = tot;
+            counts[q] = c;
+            tot += c;
+            maxcount = std::max<int64_t>(maxcount, c);
         }
-        char *pb = (char *)pts;
-        double *px = pts, *py = (double *)(pb + a8), *psx = (double *)(pb + 2 * a8),
-               *psy = (double *)(pb + 3 * a8), *pw = (double *)(pb + 4 * a8);
-        cudaMemcpyAsync(d_start, hstart.data(), nc * 8, cudaMemcpyHostToDevice, st);
-        k_bin_points<<<(unsigned)nc, kPairThreads, 0, st>>>(P, hist, g, d_start, px, py, psx, psy, pw);
-        ctx->launches++;
-        rc = launch_stamps(ctx, StampStars{px, py, psx, psy, pw, nullptr, d_start, d_cnt, d_cov}, nc, g,
-                           nullptr, StampWork(pb + 5 * a8, tot, maxcount), d_models + t0 * nbins);
-        if (rc == SFH_OK && (e = cudaStreamSynchronize(st))) rc = sfh_cuda_error(ctx, e, "binary_hess");
+        const size_t nodes = nx <= kMaxColumns && ny <= (1 << 20) ? node_bytes(g, nc) : 0;
+        if ((rc = sfh_stage_reserve(ctx, StampWork::bytes(tot, nodes)))) return rc;
+        SFH_CK(ctx, cudaMemcpyAsync(b + o_up, hup.data(), hup.size(), cudaMemcpyHostToDevice, st));
+        StampWork work((char *)ctx->stage, tot, maxcount);
+        work.made = true;
+        work.n_narrow = (int *)(b + o_up);
+        const int64_t *d_start = (const int64_t *)(b + o_up + 256);
+        const int32_t *d_cnt = (const int32_t *)(b + o_up + 256 + sfh_align256(chunk * 8));
+        k_bin_points<<<dim3((unsigned)nseg, (unsigned)nc), kPairThreads, 0, st>>>(
+            P, hist, g, d_start, (const int32_t *)(b + o_up + up), cov, work.rec, work.narrow, work.n_narrow);
+        SFH_LAUNCHED(ctx);
+        rc = launch_stamps(ctx, StampStars{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d_start,
+                                           d_cnt, (const int32_t *)(b + o_cov)},
+                           nc, g, nullptr, work, d_models + t0 * nbins);
+        if (rc) return rc;
+        SFH_CK(ctx, cudaStreamSynchronize(st));
     }
-    cleanup();
-    return rc;
+    return SFH_OK;
 }
 
 extern "C" int sfh_mix_binary_templates_dev(sfh_ctx *ctx, const float *d_single,
