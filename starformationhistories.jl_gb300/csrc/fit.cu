@@ -30,7 +30,7 @@
 namespace {
 
 constexpr int kVecThreads = 1024;
-constexpr int kRowWarps = 8;
+constexpr int kRowWarps = 8;  // most rows of H per CTA of k_fit_hgemv / k_fit_hupdate
 constexpr int kMaxBacktracks = 40;
 constexpr int kMaxExpand = 10;
 constexpr double kArmijo = 1e-4;
@@ -54,29 +54,44 @@ struct FitVecs {
     double g_abstol, f_reltol, x_abstol;
 };
 
+// Maximum of two values that are >= 0 or NaN, by their bits: a NaN is the largest.
 __device__ __forceinline__ double nanmax(double a, double b) {
-    return (a != a || b != b) ? __longlong_as_double(0x7ff8000000000000LL) : fmax(a, b);
+    return __longlong_as_double(max(__double_as_longlong(fabs(a)), __double_as_longlong(fabs(b))));
 }
 
-// Sum (or NaN-propagating max) over the block; every thread gets the result.
-template <bool MAX>
-__device__ double block_reduce(double v, double *sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = MAX ? nanmax(v, u) : v + u;
-    }
+// Sums (or NaN-propagating maxima of magnitudes) of N values over the block; every thread gets
+// the results.  A butterfly per warp, then one warp per value over the warps' results: FP64
+// retires two operations per SM clock, so the second step is not repeated in every warp and
+// the block is no larger than the vectors (eval_threads).  The order of a sum does not depend on
+// the block's size while a thread holds one element.
+template <int N, bool MAX>
+__device__ __forceinline__ void block_reduce(double (&v)[N], double *sh) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncthreads();
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    double t = l < nw ? sh[l] : 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double u = __shfl_xor_sync(0xffffffffu, t, o);
-        t = MAX ? nanmax(t, u) : t + u;
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const double u = __shfl_xor_sync(0xffffffffu, v[k], o);
+            v[k] = MAX ? nanmax(v[k], u) : v[k] + u;
+        }
+    __syncthreads();
+    if (l == 0)
+#pragma unroll
+        for (int k = 0; k < N; ++k) sh[32 * k + w] = v[k];
+    __syncthreads();
+    for (int k = w; k < N; k += nw) {
+        double t = l < nw ? sh[32 * k + l] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double u = __shfl_xor_sync(0xffffffffu, t, o);
+            t = MAX ? nanmax(t, u) : t + u;
+        }
+        __syncwarp();
+        if (l == 0) sh[32 * k] = t;
     }
-    return t;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = sh[32 * k];
 }
 
 __device__ __forceinline__ double to_coeff(int transform, double th) {
@@ -96,7 +111,7 @@ __global__ void k_fit_init(FitState *S, FitVecs V) {
 }
 
 __global__ void __launch_bounds__(kVecThreads) k_fit_trial(FitState *S, FitVecs V) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     const int64_t nt = V.nt;
     if (S->done) {
         if (threadIdx.x == 0) S->skip = 1;
@@ -110,22 +125,22 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_trial(FitState *S, FitVecs 
         for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) V.theta_t[i] = V.theta[i];
     } else {
         if (newdir) {
-            double dg = 0.0, dd = 0.0;
+            double sums[2] = {0.0, 0.0};
             for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
-                dg += V.g[i] * V.d[i];
-                dd += V.d[i] * V.d[i];
+                sums[0] += V.g[i] * V.d[i];
+                sums[1] += V.d[i] * V.d[i];
             }
-            dg = block_reduce<false>(dg, sh);
-            dd = block_reduce<false>(dd, sh);
+            block_reduce<2, false>(sums, sh);
+            double dg = sums[0], dd = sums[1];
             if (!(dg < 0.0)) {  // not a descent direction: steepest descent, H restarts at I
-                double gg = 0.0;
+                double gg[1] = {0.0};
                 for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
                     V.d[i] = -V.g[i];
-                    gg += V.g[i] * V.g[i];
+                    gg[0] += V.g[i] * V.g[i];
                 }
-                gg = block_reduce<false>(gg, sh);
-                dg = -gg;
-                dd = gg;
+                block_reduce<1, false>(gg, sh);
+                dg = -gg[0];
+                dd = gg[0];
                 reset = 1;
             }
             const double nd = sqrt(dd);
@@ -154,14 +169,14 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_trial(FitState *S, FitVecs 
 }
 
 __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     const int64_t nt = V.nt;
     if (S->done) return;
     const int first = S->first, nexp = S->expansions, have_best = S->best_valid;
     const double f0 = S->f, alpha = S->alpha, dg0 = S->dg0, f_b = S->f_b, alpha_b = S->alpha_b;
     __syncthreads();
     // transformed gradient at θt, in place of the raw one, and the slope φ'(α) = gtᵀd
-    double sumth = 0.0, dgt = 0.0;
+    double sums[2] = {0.0, 0.0};  // Σθ, gtᵀd
     for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
         const double th = V.theta_t[i], G = V.Graw[i];
         double gt;
@@ -171,16 +186,16 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V
             gt = G * 2.0 * th;
         } else {
             gt = V.transform == SFH_FIT_LOG_MAP ? G * V.r[i] - 1.0 : G * V.r[i];
-            sumth += th;
+            sums[0] += th;
         }
         V.Graw[i] = gt;
-        if (!first) dgt += gt * V.d[i];
+        if (!first) sums[1] += gt * V.d[i];
     }
-    if (V.transform == SFH_FIT_LOG_MAP) sumth = block_reduce<false>(sumth, sh);
+    block_reduce<2, false>(sums, sh);
+    const double sumth = sums[0], dgt = sums[1];
     const double ft = *V.negLogL - (V.transform == SFH_FIT_LOG_MAP ? sumth : 0.0);
     bool use_best = false;
     if (!first) {
-        dgt = block_reduce<false>(dgt, sh);
         const bool finite = fabs(ft) < INFINITY && fabs(dgt) < INFINITY;
         // sufficient decrease, or Hager-Zhang's approximate Wolfe conditions (slope reduced
         // to within [σ φ'(0), (2δ - 1) φ'(0)], σ = 0.9, δ = 0.1, and f at most ε |f| higher,
@@ -234,7 +249,7 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V
     const double *th_src = use_best ? V.theta_b : V.theta_t;
     const double *g_src = use_best ? V.g_b : V.Graw;
     const double a_acc = use_best ? alpha_b : alpha, f_acc = use_best ? f_b : ft;
-    double gmax = 0.0, smax = 0.0;
+    double most[2] = {0.0, 0.0};  // |g|, |s|
     for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
         const double gt = g_src[i];
         if (first) {
@@ -243,14 +258,14 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V
             const double s = a_acc * V.d[i];
             V.s[i] = s;
             V.y[i] = gt - V.g[i];
-            smax = nanmax(smax, fabs(s));
+            most[1] = nanmax(most[1], s);
         }
         V.theta[i] = th_src[i];
         V.g[i] = gt;
-        gmax = nanmax(gmax, fabs(gt));
+        most[0] = nanmax(most[0], gt);
     }
-    gmax = block_reduce<true>(gmax, sh);
-    smax = block_reduce<true>(smax, sh);
+    block_reduce<2, true>(most, sh);
+    const double gmax = most[0], smax = most[1];
     if (threadIdx.x == 0) {
         S->f_prev = first ? f_acc : f0;
         S->f = f_acc;
@@ -282,7 +297,7 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V
 __global__ void __launch_bounds__(kRowWarps * 32) k_fit_hgemv(const FitState *S, FitVecs V) {
     if (!S->accept) return;
     const int64_t nt = V.nt;
-    const int64_t i = (int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= nt) return;
     if (S->reset_h) {
@@ -294,6 +309,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_fit_hgemv(const FitState *S,
     }
     const double *row = V.H + i * nt;
     double a = 0.0, b = 0.0;
+#pragma unroll 8
     for (int64_t j = lane; j < nt; j += 32) {
         const double h = row[j];
         a = fma(h, V.y[j], a);
@@ -313,37 +329,54 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_fit_hgemv(const FitState *S,
 // H += c1 s sᵀ - c2 (Hy sᵀ + s Hyᵀ) with c1 = (sᵀy + yᵀHy) / (sᵀy)², c2 = 1 / sᵀy when
 // sᵀy > 0 (Optim's BFGS update_h!), and d = -H_new g from the same vectors.  Every CTA
 // forms the four dot products in the same order, so all see the same scalars.
-__global__ void __launch_bounds__(kRowWarps * 32) k_fit_hupdate(const FitState *S, FitVecs V) {
-    __shared__ double sh[32];
+// A CTA takes `rows` rows; its threads share their elements.
+__global__ void __launch_bounds__(kRowWarps * 32) k_fit_hupdate(const FitState *S, FitVecs V, int rows) {
+    __shared__ double sh[128];
     if (!S->accept) return;
     const int64_t nt = V.nt;
     const int reset = S->reset_h;
-    double sty = 0.0, yhy = 0.0, sg = 0.0, hyg = 0.0;
+    double dots[4] = {0.0, 0.0, 0.0, 0.0};  // sᵀy, yᵀHy, sᵀg, (Hy)ᵀg
     for (int64_t j = threadIdx.x; j < nt; j += blockDim.x) {
         const double s = V.s[j], hy = V.Hy[j], g = V.g[j];
-        sty += s * V.y[j];
-        yhy += V.y[j] * hy;
-        sg += s * g;
-        hyg += hy * g;
+        dots[0] += s * V.y[j];
+        dots[1] += V.y[j] * hy;
+        dots[2] += s * g;
+        dots[3] += hy * g;
     }
-    sty = block_reduce<false>(sty, sh);
-    yhy = block_reduce<false>(yhy, sh);
-    sg = block_reduce<false>(sg, sh);
-    hyg = block_reduce<false>(hyg, sh);
+    block_reduce<4, false>(dots, sh);
+    const double sty = dots[0], yhy = dots[1], sg = dots[2], hyg = dots[3];
     const bool upd = sty > 0.0 && sty < INFINITY && fabs(yhy) < INFINITY;
     const double c1 = upd ? (sty + yhy) / (sty * sty) : 0.0, c2 = upd ? 1.0 / sty : 0.0;
-    const int64_t i = (int64_t)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (i >= nt) return;
-    const double si = V.s[i], hyi = V.Hy[i];
-    double *row = V.H + i * nt;
+    const int64_t i0 = (int64_t)blockIdx.x * rows;
+    const int nr = (int)min((int64_t)rows, nt - i0);
+    double *H = V.H + i0 * nt;
+    const double *vs = V.s, *vhy = V.Hy;
     if (upd || reset) {
-        for (int64_t j = lane; j < nt; j += 32) {
-            const double base = reset ? (j == i ? 1.0 : 0.0) : row[j];
-            row[j] = base + c1 * si * V.s[j] - c2 * (hyi * V.s[j] + si * V.Hy[j]);
+        const int total = nr * (int)nt, step = kRowWarps * 32;  // rows <= 8, nt < 2^27
+        for (int k0 = threadIdx.x; k0 < total; k0 += 4 * step) {
+            double h[4], sj[4], hyj[4], si[4], hyi[4];  // four elements' loads before their stores
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = k0 + u * step;
+                if (k >= total) break;
+                const int r = k / (int)nt, j = k - r * (int)nt;
+                h[u] = reset ? (j == i0 + r ? 1.0 : 0.0) : H[k];
+                sj[u] = vs[j];
+                hyj[u] = vhy[j];
+                si[u] = vs[i0 + r];
+                hyi[u] = vhy[i0 + r];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k0 + u * step < total)
+                    H[k0 + u * step] = h[u] + c1 * si[u] * sj[u] - c2 * (hyi[u] * sj[u] + si[u] * hyj[u]);
         }
     }
-    if (lane == 0) V.d[i] = -(V.Hg[i] + c1 * si * sg - c2 * (hyi * sg + si * hyg));
+    if ((int)threadIdx.x < nr) {
+        const int64_t i = i0 + threadIdx.x;
+        const double si = vs[i], hyi = vhy[i];
+        V.d[i] = -(V.Hg[i] + c1 * si * sg - c2 * (hyi * sg + si * hyg));
+    }
 }
 
 }  // namespace
@@ -375,17 +408,21 @@ int sfh_bfgs_run(sfh_ctx *ctx, int64_t nvar, const double *d_theta0, const sfh_f
     int rc = SFH_OK;
     const int64_t max_evals = opt->max_evals > 0 ? opt->max_evals : 50 * ((int64_t)opt->max_iter + 1);
     const int K = opt->graph_slots > 0 ? opt->graph_slots : 8;
-    const int hgrid = (int)((nt + kRowWarps - 1) / kRowWarps);
+    // rows per CTA: one CTA per SM (every CTA of k_fit_hupdate repeats four dot products), at
+    // most eight rows
+    const int rows = (int)std::max<int64_t>(1, std::min<int64_t>(kRowWarps, (nt + ctx->sm_count - 1) / ctx->sm_count));
+    const int hgrid = (int)((nt + rows - 1) / rows);
+    const int eval_threads = (int)std::min<int64_t>(kVecThreads, (nt + 31) / 32 * 32);
     auto slot = [&]() -> int {
-        k_fit_trial<<<1, kVecThreads, 0, st>>>(S, V);
+        k_fit_trial<<<1, eval_threads, 0, st>>>(S, V);
         SFH_LAUNCHED(ctx);
         int r = objective(V.theta_t, V.r, V.Graw, V.negLogL, &S->skip);
         if (r) return r;
-        k_fit_eval<<<1, kVecThreads, 0, st>>>(S, V);
+        k_fit_eval<<<1, eval_threads, 0, st>>>(S, V);
         SFH_LAUNCHED(ctx);
-        k_fit_hgemv<<<hgrid, kRowWarps * 32, 0, st>>>(S, V);
+        k_fit_hgemv<<<hgrid, rows * 32, 0, st>>>(S, V);
         SFH_LAUNCHED(ctx);
-        k_fit_hupdate<<<hgrid, kRowWarps * 32, 0, st>>>(S, V);
+        k_fit_hupdate<<<hgrid, kRowWarps * 32, 0, st>>>(S, V, rows);
         SFH_LAUNCHED(ctx);
         return SFH_OK;
     };
