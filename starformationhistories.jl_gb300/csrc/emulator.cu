@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -305,6 +306,127 @@ __global__ void k_mlp_rows(const float *__restrict__ P, int64_t pstride, int64_t
     }
 }
 
+// The same network for many rows: rows of one group are taken up to kMlpRows at a time, so a
+// layer's weights are read once per segment instead of once per row, in coalesced tiles.  A
+// thread owns an output and all rows of the segment; every row's sums run over k in order as in
+// k_mlp_rows, so the results are the same bits.  1,200 rows of 64 groups, 3 -> 256 -> 256 -> 64:
+// 335 us a row at a time (each lane walking a weight row of its own), 56 us this way.
+constexpr int kMlpRows = 16;
+constexpr int kMlpTile = 32;       // weights of an output staged at a time
+constexpr int kMlpThreads = 256;
+
+// One layer for the segment's rows: y[j][row] = act(sum_k x[k][row] bf16(W[j][k]) + b[j]).
+template <bool HIDDEN>
+__device__ __forceinline__ void mlp_layer(const float *__restrict__ W, const float *__restrict__ bias,
+                                          const float *x, float *y, float *s_w, int in, int out,
+                                          const int32_t *s_row, int cnt, float *__restrict__ Y) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int j0 = 0; j0 < out; j0 += kMlpThreads) {
+        const int j = j0 + (int)threadIdx.x;
+        float acc[kMlpRows];
+#pragma unroll
+        for (int r = 0; r < kMlpRows; ++r) acc[r] = 0.f;
+        float next[kMlpTile];  // the tile after the one in shared memory: outputs warp + 8 i
+        const auto fetch = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < kMlpTile; ++i) {
+                const int jj = j0 + warp + (kMlpThreads / 32) * i;
+                next[i] = jj < out && k0 + lane < in ? __ldg(W + (int64_t)jj * in + k0 + lane) : 0.f;
+            }
+        };
+        fetch(0);
+        for (int k0 = 0; k0 < in; k0 += kMlpTile) {
+            __syncthreads();  // the tile before is used up
+#pragma unroll
+            for (int i = 0; i < kMlpTile; ++i)
+                s_w[(warp + (kMlpThreads / 32) * i) * (kMlpTile + 1) + lane] = bf16r(next[i]);
+            __syncthreads();
+            if (k0 + kMlpTile < in) fetch(k0 + kMlpTile);
+            const int kn = min(kMlpTile, in - k0);
+            if (j < out)
+                for (int k = 0; k < kn; ++k) {
+                    const float w = s_w[threadIdx.x * (kMlpTile + 1) + k];
+#pragma unroll
+                    for (int r = 0; r < kMlpRows; r += 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(x + (k0 + k) * kMlpRows + r);
+                        acc[r] = fmaf(v.x, w, acc[r]);
+                        acc[r + 1] = fmaf(v.y, w, acc[r + 1]);
+                        acc[r + 2] = fmaf(v.z, w, acc[r + 2]);
+                        acc[r + 3] = fmaf(v.w, w, acc[r + 3]);
+                    }
+                }
+        }
+        if (j < out) {
+            const float b = bias[j];
+#pragma unroll
+            for (int r = 0; r < kMlpRows; ++r) {
+                if (HIDDEN) y[j * kMlpRows + r] = bf16r(gelu(acc[r] + b));
+                else if (r < cnt) Y[(int64_t)s_row[r] * out + j] = acc[r] + b;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kMlpThreads)
+k_mlp_groups(const float *__restrict__ P, int64_t pstride, int64_t ngroups, MlpShape S,
+             const float *__restrict__ X, const int32_t *__restrict__ group, int64_t B,
+             float *__restrict__ Y) {
+    extern __shared__ __align__(16) float sm[];
+    float *s_w = sm, *x = s_w + kMlpThreads * (kMlpTile + 1), *a1 = x + S.in * kMlpRows,
+          *a2 = a1 + S.h1 * kMlpRows;
+    __shared__ int32_t s_row[kMlpRows];
+    __shared__ int s_count[kMlpThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t g = blockIdx.x;
+    const float *p = P + g * pstride;
+    // The block's rows: of the group's rows in order, every gridDim.y-th run of kMlpRows.
+    int64_t at = 0;  // rows of the group before the 256 looked at
+    int have = 0;    // rows gathered for the segment
+    const auto segment = [&](int cnt) {
+        for (int t = threadIdx.x; t < S.in * kMlpRows; t += kMlpThreads) {
+            const int r = t / S.in, k = t - r * S.in;
+            x[k * kMlpRows + r] = r < cnt ? bf16r(X[(int64_t)s_row[r] * S.in + k]) : 0.f;
+        }
+        // (the layers begin with a barrier)
+        mlp_layer<true>(p + S.oW1, p + S.ob1, x, a1, s_w, S.in, S.h1, s_row, cnt, nullptr);
+        mlp_layer<true>(p + S.oW2, p + S.ob2, a1, a2, s_w, S.h1, S.h2, s_row, cnt, nullptr);
+        mlp_layer<false>(p + S.oW3, p + S.ob3, a2, nullptr, s_w, S.h2, S.out, s_row, cnt, Y);
+    };
+    for (int64_t i0 = 0; i0 < B; i0 += kMlpThreads) {
+        const int64_t i = i0 + threadIdx.x;
+        const int64_t gi = i < B ? (group ? (int64_t)group[i] : 0) : ngroups;
+        if (g == 0 && blockIdx.y == 0 && i < B && (gi < 0 || gi >= ngroups))  // invalid group: NaN row
+            for (int j = 0; j < S.out; ++j) Y[i * S.out + j] = __int_as_float(0x7fc00000);
+        const unsigned hit = __ballot_sync(0xffffffffu, gi == g);
+        if (lane == 0) s_count[warp] = __popc(hit);
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kMlpThreads / 32; ++w) {
+            if (w < warp) before += s_count[w];
+            all += s_count[w];
+        }
+        const int64_t rank = at + before + __popc(hit & ((1u << lane) - 1u));
+        // the runs that end or begin among these rows, in order
+        for (int64_t run = at / kMlpRows; run * kMlpRows < at + all; ++run) {
+            if (run % gridDim.y != blockIdx.y) continue;
+            const int64_t r = rank - run * kMlpRows;
+            if (gi == g && r >= 0 && r < kMlpRows) s_row[r] = (int32_t)i;
+            const int64_t upto = at + all - run * kMlpRows;
+            have = upto < kMlpRows ? (int)upto : kMlpRows;
+            __syncthreads();
+            if (have == kMlpRows) {
+                segment(kMlpRows);
+                have = 0;
+            }
+        }
+        at += all;
+        __syncthreads();  // s_count
+    }
+    if (have) segment(have);
+}
+
 // Templates from coefficients with a basis per row's group:
 // out[b, i] = inverse transform of (offset[g, i] + Σ_k coef[b, k] basis[g, k, i]), g = group[b].
 __global__ void k_recon_rows(const float *__restrict__ coef, const int32_t *__restrict__ group,
@@ -336,52 +458,73 @@ __global__ void k_recon_rows(const float *__restrict__ coef, const int32_t *__re
 // thread owns V consecutive bins and R row accumulators; R is the segment's row count
 // rounded up to 4, 8 or 16 (block-uniform).  Coefficients of the segment sit in shared
 // memory, zero past count.
+//
+// What a row of the basis costs is data returned from shared memory and L1 (128 bytes a clock
+// per SM, broadcast or not) beside the FMAs: 16 rows by 4 bins need 20 words a thread for 64
+// FMAs.  So coefficients are read as 16-byte vectors of four rows, whose halves are the packed
+// operands of __ffma2_rn over row pairs, and at V = 4 the basis comes through a ring of kRecDepth
+// rows filled by cp.async, started before the coefficients are gathered.  64 cells x 64
+// components x 60,000 bins, 1,200 rows: 402 us with plain loads four rows ahead and a 4-byte
+// coefficient read for every four FMAs, 285 us this way (1.27 GB: 4.5 TB/s).  Tried at that size:
+// coefficients stored twice to pack over bins 337, eight bins a thread 268-296, three blocks per
+// SM 383 (spills), depth 4 313, depth 16 286, several tiles to a block 371-600.
 constexpr int kRecRows = 16;
 constexpr int kRecThreads = 256;
 
+constexpr int kRecDepth = 8;  // basis rows in flight per thread
+
+// Queues this thread's four values of basis row k (nothing past the last row, but the group of
+// copies is closed all the same, so that every row is one group).
+__device__ __forceinline__ void recon_fetch(float4 *s_b, const float *vb, int64_t nbins, int k, int K) {
+    if (k < K)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(s_b)),
+                     "l"(vb + (int64_t)k * nbins)
+                     : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 template <int R, int V>
-__device__ __forceinline__ void recon_segment(const float *__restrict__ sc, int K,
+__device__ __forceinline__ void recon_segment(const float *__restrict__ sc, float4 *s_b, int K,
                                               const float *__restrict__ vb,
                                               const float *__restrict__ off, int64_t nbins,
                                               int64_t i0, const int32_t *__restrict__ srow,
                                               int cnt, int mode, float *__restrict__ out) {
-    float acc[R][V];
+    float2 acc[R / 2][V];  // rows 2 r and 2 r + 1
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = 0; r < R / 2; ++r)
 #pragma unroll
-        for (int v = 0; v < V; ++v) acc[r][v] = 0.f;
-    if (V == 4) {
-        // four basis rows in flight per thread: one 16-byte load at a time leaves the
-        // kernel latency-bound at the two blocks per SM its registers allow
-#pragma unroll 4
-        for (int k = 0; k < K; ++k) {
-            const float4 b = __ldg(reinterpret_cast<const float4 *>(vb + (int64_t)k * nbins + i0));
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float c = sc[r * K + k];
-                acc[r][0] = fmaf(c, b.x, acc[r][0]);
-                acc[r][1] = fmaf(c, b.y, acc[r][1]);
-                acc[r][2] = fmaf(c, b.z, acc[r][2]);
-                acc[r][3] = fmaf(c, b.w, acc[r][3]);
-            }
+        for (int v = 0; v < V; ++v) acc[r][v] = make_float2(0.f, 0.f);
+    int slot = 0;
+#pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+        float b[V];
+        if constexpr (V == 4) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRecDepth - 1) : "memory");  // row k is here
+            const float4 t = s_b[slot * kRecThreads];
+            recon_fetch(s_b + slot * kRecThreads, vb + i0, nbins, k + kRecDepth, K);
+            slot = (slot + 1) % kRecDepth;
+            b[0] = t.x;
+            b[1] = t.y;
+            b[2] = t.z;
+            b[3] = t.w;
+        } else {
+            b[0] = __ldg(vb + (int64_t)k * nbins + i0);
         }
-    } else {
-        for (int k = 0; k < K; ++k) {
-            float b[V];
 #pragma unroll
-            for (int v = 0; v < V; ++v)
-                b[v] = i0 + v < nbins ? __ldg(vb + (int64_t)k * nbins + i0 + v) : 0.f;
+        for (int r = 0; r < R / 2; r += 2) {
+            const float4 c = *reinterpret_cast<const float4 *>(sc + k * kRecRows + 2 * r);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float c = sc[r * K + k];
-#pragma unroll
-                for (int v = 0; v < V; ++v) acc[r][v] = fmaf(c, b[v], acc[r][v]);
+            for (int v = 0; v < V; ++v) {
+                const float2 bb = make_float2(b[v], b[v]);
+                acc[r][v] = __ffma2_rn(make_float2(c.x, c.y), bb, acc[r][v]);
+                acc[r + 1][v] = __ffma2_rn(make_float2(c.z, c.w), bb, acc[r + 1][v]);
             }
         }
     }
     float o[V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) o[v] = i0 + v < nbins ? __ldg(off + i0 + v) : 0.f;
+    for (int v = 0; v < V; ++v) o[v] = __ldg(off + i0 + v);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         if (r >= cnt) break;
@@ -389,16 +532,11 @@ __device__ __forceinline__ void recon_segment(const float *__restrict__ sc, int 
         float y[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            const float t = fmaxf(acc[r][v] + o[v], 0.f);
+            const float t = fmaxf((r & 1 ? acc[r / 2][v].y : acc[r / 2][v].x) + o[v], 0.f);
             y[v] = mode == 1 ? t * t : t;
         }
-        if (V == 4) {
-            *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);
-        } else {
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-                if (i0 + v < nbins) dst[v] = y[v];
-        }
+        if constexpr (V == 4) *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);
+        else *dst = y[0];
     }
 }
 
@@ -406,18 +544,23 @@ __device__ __forceinline__ void recon_segment(const float *__restrict__ sc, int 
 // of range writes NaN to the rows it can address and nothing else; a row index outside
 // [0, B) ends its segment at that row.
 template <int V>
-__global__ void __launch_bounds__(kRecThreads)
+__global__ void __launch_bounds__(kRecThreads, 2)
 k_recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
                const int32_t *__restrict__ seg, int64_t B, int64_t ngroups,
                const float *__restrict__ basis, const float *__restrict__ offset, int K,
                int64_t nbins, int mode, float *__restrict__ out) {
-    extern __shared__ float sc[];  // kRecRows x K
+    extern __shared__ __align__(16) float s_coef[];  // K x kRecRows; copies of basis rows
     __shared__ int32_t srow[kRecRows];
     const int s = blockIdx.y;
     const int g = seg[3 * s], start = seg[3 * s + 1];
     int cnt = seg[3 * s + 2];
     const bool bad = g < 0 || g >= ngroups || start < 0 || cnt < 1 || cnt > kRecRows ||
                      (int64_t)start + cnt > B;
+    const int64_t i0 = ((int64_t)blockIdx.x * kRecThreads + threadIdx.x) * V;
+    const float *vb = basis + (bad ? 0 : (int64_t)g * K * nbins);
+    float4 *s_b = reinterpret_cast<float4 *>(s_coef + K * kRecRows) + threadIdx.x;
+    if (V == 4 && !bad && i0 < nbins)  // the first rows travel while the coefficients are read
+        for (int k = 0; k < kRecDepth; ++k) recon_fetch(s_b + k * kRecThreads, vb + i0, nbins, k, K);
     if (threadIdx.x < kRecRows) {
         int32_t r = -1;
         if (start >= 0 && (int64_t)start + threadIdx.x < B && (int)threadIdx.x < cnt)
@@ -425,7 +568,6 @@ k_recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
         srow[threadIdx.x] = (r >= 0 && r < B) ? r : -1;
     }
     __syncthreads();
-    const int64_t i0 = ((int64_t)blockIdx.x * kRecThreads + threadIdx.x) * V;
     if (bad) {
         for (int r = 0; r < kRecRows; ++r)
             if (srow[r] >= 0 && i0 < nbins)
@@ -436,19 +578,19 @@ k_recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
     for (int r = 0; r < kRecRows; ++r)
         if (srow[r] < 0 && r < cnt) cnt = r;  // a row index out of range ends the segment
     for (int t = threadIdx.x; t < kRecRows * K; t += kRecThreads) {
-        const int r = t / K;
-        sc[t] = r < cnt ? coef[(int64_t)srow[r] * K + (t - r * K)] : 0.f;
+        const int r = t / K, k = t - r * K;
+        const float c = r < cnt ? coef[(int64_t)srow[r] * K + k] : 0.f;
+        s_coef[k * kRecRows + r] = c;
     }
     __syncthreads();
     if (i0 >= nbins) return;
-    const float *vb = basis + (int64_t)g * K * nbins;
     const float *off = offset + (int64_t)g * nbins;
     if (cnt <= 4)
-        recon_segment<4, V>(sc, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        recon_segment<4, V>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
     else if (cnt <= 8)
-        recon_segment<8, V>(sc, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        recon_segment<8, V>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
     else
-        recon_segment<16, V>(sc, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        recon_segment<16, V>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
 }
 
 struct Acts {  // activations of one batch (G groups x B rows)
@@ -657,6 +799,23 @@ extern "C" int sfh_mlp_forward_rows(sfh_ctx *ctx, int in, int h1, int h2, int ou
         return SFH_ERR_ARG;
     SFH_CK(ctx, cudaSetDevice(ctx->device));
     const MlpShape S = mlp_shape(in, h1, h2, out);
+    // Rows of a group share its weights where a group has two of them on average and the
+    // activations fit shared memory.  Networks of fewer than 24 K weights finish sooner a row
+    // per block while the blocks fit a few waves, both being latency.  us a row per block / in
+    // groups, hidden layers of 256: 1 group x 16 rows 49 / 47, 64 x 2 49 / 37, 64 x 64 1,200 /
+    // 72, 512 x 4 581 / 117; of 64: 64 x 8 16.6 / 14.7, 512 x 2 22.7 / 31.8, 512 x 3 45 / 35;
+    // of 1,024: 1 x 2 660 / 342, 64 x 16 4,590 / 405.
+    const size_t grp_smem = (size_t)(kMlpThreads * (kMlpTile + 1) + kMlpRows * (in + h1 + h2)) * sizeof(float);
+    if (B >= 2 * ngroups && (S.n >= 24 * 1024 || B >= 8 * (int64_t)ctx->sm_count) && grp_smem <= 200 * 1024) {
+        // as many blocks to a group as it has runs of rows, up to four blocks per SM altogether
+        const int64_t runs = (B / ngroups + kMlpRows - 1) / kMlpRows + 1;
+        const int64_t ny = std::min(runs, std::max<int64_t>(1, 4 * ctx->sm_count / ngroups));
+        SFH_CK(ctx, cudaFuncSetAttribute(k_mlp_groups, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        k_mlp_groups<<<dim3((unsigned)ngroups, (unsigned)ny), kMlpThreads, grp_smem, ctx->stream>>>(
+            d_params, S.n, ngroups, S, d_X, d_group, B, d_Y);
+        SFH_LAUNCHED(ctx);
+        return SFH_OK;
+    }
     const size_t smem = (size_t)(in + h1 + h2) * sizeof(float);
     k_mlp_rows<<<(unsigned)B, 256, smem, ctx->stream>>>(d_params, S.n, ngroups, S, d_X, d_group,
                                                         d_Y);
@@ -777,12 +936,13 @@ extern "C" int sfh_emu_reconstruct_groups(sfh_ctx *ctx, const float *d_coef,
         ngroups < 1 || (mode != 0 && mode != 1))
         return SFH_ERR_ARG;
     SFH_CK(ctx, cudaSetDevice(ctx->device));
-    const size_t shm = (size_t)kRecRows * K * sizeof(float);
+    size_t shm = (size_t)kRecRows * K * sizeof(float);
     // float4 rows need every basis, offset and output row on a 16-byte boundary
     const bool vec = nbins % 4 == 0 && ((uintptr_t)d_basis | (uintptr_t)d_offset |
                                         (uintptr_t)d_out) % 16 == 0;
     if (vec) {
-        if (shm > 48 * 1024)
+        shm += (size_t)kRecDepth * kRecThreads * sizeof(float4);
+        if (shm > 40 * 1024)
             SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups<4>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)shm));
@@ -790,7 +950,7 @@ extern "C" int sfh_emu_reconstruct_groups(sfh_ctx *ctx, const float *d_coef,
         k_recon_groups<4><<<grid, kRecThreads, shm, ctx->stream>>>(
             d_coef, d_rows, d_seg, B, ngroups, d_basis, d_offset, K, nbins, mode, d_out);
     } else {
-        if (shm > 48 * 1024)
+        if (shm > 40 * 1024)
             SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups<1>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)shm));
