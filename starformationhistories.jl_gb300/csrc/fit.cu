@@ -59,39 +59,81 @@ __device__ __forceinline__ double nanmax(double a, double b) {
     return __longlong_as_double(max(__double_as_longlong(fabs(a)), __double_as_longlong(fabs(b))));
 }
 
-// Sums (or NaN-propagating maxima of magnitudes) of N values over the block; every thread gets
-// the results.  A butterfly per warp, then one warp per value over the warps' results: FP64
-// retires two operations per SM clock, so the second step is not repeated in every warp and
-// the block is no larger than the vectors (eval_threads).  The order of a sum does not depend on
-// the block's size while a thread holds one element.
-template <int N, bool MAX>
-__device__ __forceinline__ void block_reduce(double (&v)[N], double *sh) {
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+// What bounds the vector kernels is the serial chain of FP64: two operations retire per SM clock, a
+// warp's instruction holds its scheduler's FP64 pipe for 64 clocks and eight warps take 128.  So
+// sums of several values share their instructions, scalars are formed by one warp, comparisons of
+// magnitudes use the bits, and each kernel's loads are issued together before its first branch.
+// Microseconds within an evaluation of 240 templates, start to start of the next kernel, before /
+// after: k_fit_eval with an accepted step 8.0 / 6.1, k_fit_hgemv 6.4 / 4.3, k_fit_hupdate 6.5 /
+// 5.4, k_fit_trial with a new direction 5.1 / 3.8, each with 1.1 us between two kernels (as
+// programmatic dependents of one another the whole fit took the same time).  A fit of 331
+// evaluations: 11.6 ms / 10.4 ms.
+
+// Tree sums of N = 2 or 4 values over a warp (pairs 16 lanes apart, then 8, 4, 2, 1): value k ends
+// in lane 32 k / N.  While lanes still hold several values, half of them go on with one half of
+// the values and the other half with the rest, so an instruction adds for all.
+template <int N>
+__device__ __forceinline__ double warp_sums(const double (&v)[N]) {
+    static_assert(N == 2 || N == 4, "");
+    const int l = threadIdx.x & 31;
+    double u[N / 2];
+    const bool up = (l & 16) != 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            const double u = __shfl_xor_sync(0xffffffffu, v[k], o);
-            v[k] = MAX ? nanmax(v[k], u) : v[k] + u;
-        }
-    __syncthreads();
-    if (l == 0)
-#pragma unroll
-        for (int k = 0; k < N; ++k) sh[32 * k + w] = v[k];
-    __syncthreads();
-    for (int k = w; k < N; k += nw) {
-        double t = l < nw ? sh[32 * k + l] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double u = __shfl_xor_sync(0xffffffffu, t, o);
-            t = MAX ? nanmax(t, u) : t + u;
-        }
-        __syncwarp();
-        if (l == 0) sh[32 * k] = t;
+    for (int k = 0; k < N / 2; ++k) {
+        const double send = up ? v[k] : v[k + N / 2], keep = up ? v[k + N / 2] : v[k];
+        u[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
     }
-    __syncthreads();
+    double t;
+    if constexpr (N == 4) {
+        const bool up8 = (l & 8) != 0;
+        const double send = up8 ? u[0] : u[1], keep = up8 ? u[1] : u[0];
+        t = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    } else {
+        t = u[0] + __shfl_xor_sync(0xffffffffu, u[0], 8);
+    }
 #pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = sh[32 * k];
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// Sums of N values over the block: all threads call it, every lane of warp 0 gets the results (the
+// others get nothing of use).  The order of a sum does not depend on the block's size while a
+// thread holds one element.  sh: 32 N doubles, free again after the caller's next barrier.
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N], double *sh) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    double t = warp_sums<N>(v);
+    if (l % (32 / N) == 0) sh[32 * (l / (32 / N)) + w] = t;
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] = l < nw ? sh[32 * k + l] : 0.0;
+        t = warp_sums<N>(v);
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] = __shfl_sync(0xffffffffu, t, 32 / N * k);
+    }
+}
+
+// The same for NaN-propagating maxima of two magnitudes.
+__device__ __forceinline__ void block_max(double (&v)[2], double *sh) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const auto warp_max = [&]() {
+        const bool up = l >= 16;
+        double t = nanmax(up ? v[1] : v[0], __shfl_xor_sync(0xffffffffu, up ? v[0] : v[1], 16));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t = nanmax(t, __shfl_xor_sync(0xffffffffu, t, o));
+        return t;
+    };
+    double t = warp_max();
+    if (l % 16 == 0) sh[2 * l + w] = t;
+    __syncthreads();
+    if (w == 0) {
+        v[0] = l < nw ? sh[l] : 0.0;
+        v[1] = l < nw ? sh[32 + l] : 0.0;
+        t = warp_max();
+        v[0] = __shfl_sync(0xffffffffu, t, 0);
+        v[1] = __shfl_sync(0xffffffffu, t, 16);
+    }
 }
 
 __device__ __forceinline__ double to_coeff(int transform, double th) {
@@ -112,52 +154,74 @@ __global__ void k_fit_init(FitState *S, FitVecs V) {
 
 __global__ void __launch_bounds__(kVecThreads) k_fit_trial(FitState *S, FitVecs V) {
     __shared__ double sh[64];
-    const int64_t nt = V.nt;
+    __shared__ double s_alpha;
+    __shared__ int s_descent;
+    const int64_t nt = V.nt, i0 = threadIdx.x;
+    // the thread's first element (the only one up to kVecThreads templates) and the state
+    const bool own = i0 < nt;
+    const double th0 = own ? V.theta[i0] : 0.0, g0 = own ? V.g[i0] : 0.0;
+    double d0 = own ? V.d[i0] : 0.0;
+    const int first = S->first, accept = S->accept, newdir = S->newdir;
+    int reset = accept ? 0 : S->reset_h;  // an accepted step consumed the pending reset
+    double alpha = S->alpha;
     if (S->done) {
         if (threadIdx.x == 0) S->skip = 1;
         return;
     }
-    const int first = S->first, accept = S->accept, newdir = S->newdir;
-    int reset = accept ? 0 : S->reset_h;  // an accepted step consumed the pending reset
-    double alpha = S->alpha;
-    __syncthreads();
-    if (first) {
-        for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) V.theta_t[i] = V.theta[i];
-    } else {
-        if (newdir) {
-            double sums[2] = {0.0, 0.0};
-            for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
-                sums[0] += V.g[i] * V.d[i];
-                sums[1] += V.d[i] * V.d[i];
-            }
-            block_reduce<2, false>(sums, sh);
-            double dg = sums[0], dd = sums[1];
-            if (!(dg < 0.0)) {  // not a descent direction: steepest descent, H restarts at I
-                double gg[1] = {0.0};
-                for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
-                    V.d[i] = -V.g[i];
-                    gg[0] += V.g[i] * V.g[i];
-                }
-                block_reduce<1, false>(gg, sh);
-                dg = -gg[0];
-                dd = gg[0];
-                reset = 1;
-            }
+    if (!first && newdir) {
+        double sums[2] = {0.0, 0.0};
+        if (own) {
+            sums[0] += g0 * d0;
+            sums[1] += d0 * d0;
+        }
+        for (int64_t i = i0 + blockDim.x; i < nt; i += blockDim.x) {
+            sums[0] += V.g[i] * V.d[i];
+            sums[1] += V.d[i] * V.d[i];
+        }
+        block_sums<2>(sums, sh);
+        const auto step = [](double dd) {
             const double nd = sqrt(dd);
-            alpha = nd > 0.0 ? fmin(1.0, nd) / nd : 1.0;  // InitialStatic(1.0, scaled=true)
+            return nd > 0.0 ? fmin(1.0, nd) / nd : 1.0;  // InitialStatic(1.0, scaled=true)
+        };
+        if (threadIdx.x < 32) {
+            const double dg = sums[0], a = step(sums[1]);
             if (threadIdx.x == 0) {
+                s_descent = dg < 0.0;
+                s_alpha = a;
                 S->dg0 = dg;
                 S->backtracks = 0;
                 S->expansions = 0;
                 S->best_valid = 0;
             }
         }
-        for (int64_t i = threadIdx.x; i < nt; i += blockDim.x)
-            V.theta_t[i] = V.theta[i] + alpha * V.d[i];
+        __syncthreads();
+        if (!s_descent) {  // not a descent direction: steepest descent, H restarts at I
+            double gg[2] = {0.0, 0.0};
+            for (int64_t i = i0; i < nt; i += blockDim.x) {
+                V.d[i] = -V.g[i];
+                gg[0] += V.g[i] * V.g[i];
+            }
+            d0 = -g0;
+            block_sums<2>(gg, sh);
+            if (threadIdx.x < 32) {
+                const double a = step(gg[0]);
+                if (threadIdx.x == 0) {
+                    s_alpha = a;
+                    S->dg0 = -gg[0];
+                }
+            }
+            __syncthreads();
+            reset = 1;
+        }
+        alpha = s_alpha;
     }
-    if (V.transform != kFitObjective)  // a general objective maps θ itself
-        for (int64_t i = threadIdx.x; i < nt; i += blockDim.x)
-            V.r[i] = to_coeff(V.transform, V.theta_t[i]);
+    for (int64_t i = i0; i < nt; i += blockDim.x) {
+        const double th = i == i0 ? th0 : V.theta[i];
+        const double t = first ? th : th + alpha * (i == i0 ? d0 : V.d[i]);
+        V.theta_t[i] = t;
+        if (V.transform != kFitObjective)  // a general objective maps θ itself
+            V.r[i] = to_coeff(V.transform, t);
+    }
     if (threadIdx.x == 0) {
         S->alpha = alpha;
         S->newdir = 0;
@@ -168,103 +232,126 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_trial(FitState *S, FitVecs 
     }
 }
 
+enum : int { kExpand, kBacktrack, kAccept, kAcceptBest };  // what an evaluation leads to
+
 __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V) {
-    __shared__ double sh[64];
-    const int64_t nt = V.nt;
-    if (S->done) return;
+    __shared__ double sh[64], sh_max[64];
+    __shared__ int s_next;
+    const int64_t nt = V.nt, i0 = threadIdx.x;
+    // the thread's first element (the only one up to kVecThreads templates) and the state
+    const bool own = i0 < nt;
+    const double th0 = own ? V.theta_t[i0] : 0.0, G0 = own ? V.Graw[i0] : 0.0, r0 = own ? V.r[i0] : 0.0,
+                 d0 = own ? V.d[i0] : 0.0, g0 = own ? V.g[i0] : 0.0;
+    const double negLogL = *V.negLogL;
     const int first = S->first, nexp = S->expansions, have_best = S->best_valid;
     const double f0 = S->f, alpha = S->alpha, dg0 = S->dg0, f_b = S->f_b, alpha_b = S->alpha_b;
-    __syncthreads();
+    if (S->done) return;
     // transformed gradient at θt, in place of the raw one, and the slope φ'(α) = gtᵀd
     double sums[2] = {0.0, 0.0};  // Σθ, gtᵀd
-    for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
-        const double th = V.theta_t[i], G = V.Graw[i];
-        double gt;
-        if (V.transform == kFitObjective) {
-            gt = G;  // the objective wrote the gradient of f in θ
-        } else if (V.transform == SFH_FIT_SQRT) {
-            gt = G * 2.0 * th;
-        } else {
-            gt = V.transform == SFH_FIT_LOG_MAP ? G * V.r[i] - 1.0 : G * V.r[i];
-            sums[0] += th;
-        }
+    const auto gradient = [&](double th, double G, double r) {
+        if (V.transform == kFitObjective) return G;  // the objective wrote the gradient of f in θ
+        // (rounded products: not contracted into the differences they enter below)
+        if (V.transform == SFH_FIT_SQRT) return __dmul_rn(G * 2.0, th);
+        return V.transform == SFH_FIT_LOG_MAP ? G * r - 1.0 : __dmul_rn(G, r);
+    };
+    const bool logs = V.transform != kFitObjective && V.transform != SFH_FIT_SQRT;
+    const double gt0 = gradient(th0, G0, r0);
+    for (int64_t i = i0; i < nt; i += blockDim.x) {
+        const bool here = i == i0;
+        const double th = here ? th0 : V.theta_t[i];
+        const double gt = here ? gt0 : gradient(th, V.Graw[i], V.r[i]);
+        if (logs) sums[0] += th;
         V.Graw[i] = gt;
-        if (!first) sums[1] += gt * V.d[i];
+        if (!first) sums[1] += gt * (here ? d0 : V.d[i]);
     }
-    block_reduce<2, false>(sums, sh);
-    const double sumth = sums[0], dgt = sums[1];
-    const double ft = *V.negLogL - (V.transform == SFH_FIT_LOG_MAP ? sumth : 0.0);
-    bool use_best = false;
-    if (!first) {
-        const bool finite = fabs(ft) < INFINITY && fabs(dgt) < INFINITY;
-        // sufficient decrease, or Hager-Zhang's approximate Wolfe conditions (slope reduced
-        // to within [σ φ'(0), (2δ - 1) φ'(0)], σ = 0.9, δ = 0.1, and f at most ε |f| higher,
-        // ε = 1e-6), which keep making progress where f differences fall below rounding
-        const bool armijo = finite && ft <= f0 + kArmijo * alpha * dg0;
-        const bool approx = finite && ft <= f0 + kApproxEps * fabs(f0) && dgt >= kSigma * dg0 &&
-                            dgt <= (2.0 * kDelta - 1.0) * dg0;
-        const bool ok = armijo || approx;
-        if (ok && dgt < kSigma * dg0 && nexp < kMaxExpand) {
-            // decrease but the slope is still steep (curvature condition fails): keep this
-            // point and try further along d, as HagerZhang's bracketing expands
-            for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
-                V.theta_b[i] = V.theta_t[i];
-                V.g_b[i] = V.Graw[i];
-            }
-            if (threadIdx.x == 0) {
+    block_sums<2>(sums, sh);
+    double ft = 0.0;  // of use in warp 0
+    if (threadIdx.x < 32) {
+        const double sumth = sums[0], dgt = sums[1];
+        ft = negLogL - (V.transform == SFH_FIT_LOG_MAP ? sumth : 0.0);
+        int next = kAccept;
+        if (!first) {
+            const bool finite = fabs(ft) < INFINITY && fabs(dgt) < INFINITY;
+            // sufficient decrease, or Hager-Zhang's approximate Wolfe conditions (slope reduced
+            // to within [σ φ'(0), (2δ - 1) φ'(0)], σ = 0.9, δ = 0.1, and f at most ε |f| higher,
+            // ε = 1e-6), which keep making progress where f differences fall below rounding
+            const bool armijo = finite && ft <= f0 + kArmijo * alpha * dg0;
+            const bool steep = dgt < kSigma * dg0;
+            const bool approx = finite && ft <= f0 + kApproxEps * fabs(f0) && dgt >= kSigma * dg0 &&
+                                dgt <= (2.0 * kDelta - 1.0) * dg0;
+            const bool ok = armijo || approx;
+            if (ok && steep && nexp < kMaxExpand) {
+                // decrease but the slope is still steep (curvature condition fails): keep this
+                // point and try further along d, as HagerZhang's bracketing expands
+                next = kExpand;
                 double a = dgt > dg0 ? alpha * dg0 / (dg0 - dgt) : 4.0 * alpha;  // secant of φ'
                 a = fmin(fmax(a, 2.0 * alpha), 10.0 * alpha);
-                S->f_b = ft;
-                S->alpha_b = alpha;
-                S->best_valid = 1;
-                S->expansions = nexp + 1;
-                S->alpha = a;
-            }
-            return;
-        }
-        use_best = !ok && have_best;  // the expansion overshot: take the kept point
-        if (!ok && !use_best) {
-            if (threadIdx.x == 0) {
-                const int bt = S->backtracks + 1;
-                S->backtracks = bt;
-                double a = 0.5 * alpha;
-                if (finite) {
-                    // root of the secant of φ' when the slope turned positive, else the
-                    // minimiser of the quadratic through φ(0), φ'(0), φ(α)
-                    const double q = dgt > 0.0
-                                         ? alpha * dg0 / (dg0 - dgt)
-                                         : -dg0 * alpha * alpha / (2.0 * (ft - f0 - dg0 * alpha));
-                    a = fmin(fmax(q, 0.1 * alpha), 0.5 * alpha);
-                    if (!(a == a)) a = 0.5 * alpha;
+                if (threadIdx.x == 0) {
+                    S->f_b = ft;
+                    S->alpha_b = alpha;
+                    S->best_valid = 1;
+                    S->expansions = nexp + 1;
+                    S->alpha = a;
                 }
-                S->alpha = a;
-                if (bt >= kMaxBacktracks) {
-                    S->status = SFH_FIT_LINESEARCH;
-                    S->done = 1;
+            } else if (!ok && have_best) {
+                next = kAcceptBest;  // the expansion overshot: take the kept point
+            } else if (!ok) {
+                next = kBacktrack;
+                if (threadIdx.x == 0) {
+                    const int bt = S->backtracks + 1;
+                    S->backtracks = bt;
+                    double a = 0.5 * alpha;
+                    if (finite) {
+                        // root of the secant of φ' when the slope turned positive, else the
+                        // minimiser of the quadratic through φ(0), φ'(0), φ(α)
+                        const double q = dgt > 0.0
+                                             ? alpha * dg0 / (dg0 - dgt)
+                                             : -dg0 * alpha * alpha / (2.0 * (ft - f0 - dg0 * alpha));
+                        a = fmin(fmax(q, 0.1 * alpha), 0.5 * alpha);
+                        if (!(a == a)) a = 0.5 * alpha;
+                    }
+                    S->alpha = a;
+                    if (bt >= kMaxBacktracks) {
+                        S->status = SFH_FIT_LINESEARCH;
+                        S->done = 1;
+                    }
                 }
             }
-            return;
         }
+        if (threadIdx.x == 0) s_next = next;
     }
-    const double *th_src = use_best ? V.theta_b : V.theta_t;
-    const double *g_src = use_best ? V.g_b : V.Graw;
-    const double a_acc = use_best ? alpha_b : alpha, f_acc = use_best ? f_b : ft;
+    __syncthreads();
+    const int next = s_next;
+    if (next == kBacktrack) return;
+    if (next == kExpand) {
+        for (int64_t i = i0; i < nt; i += blockDim.x) {
+            V.theta_b[i] = i == i0 ? th0 : V.theta_t[i];
+            V.g_b[i] = i == i0 ? gt0 : V.Graw[i];
+        }
+        return;
+    }
+    const bool use_best = next == kAcceptBest;
+    const double a_acc = use_best ? alpha_b : alpha;
     double most[2] = {0.0, 0.0};  // |g|, |s|
-    for (int64_t i = threadIdx.x; i < nt; i += blockDim.x) {
-        const double gt = g_src[i];
+    for (int64_t i = i0; i < nt; i += blockDim.x) {
+        const bool here = i == i0;
+        const double gt = use_best ? V.g_b[i] : here ? gt0 : V.Graw[i];
+        const double th = use_best ? V.theta_b[i] : here ? th0 : V.theta_t[i];
         if (first) {
             V.d[i] = -gt;
         } else {
-            const double s = a_acc * V.d[i];
+            const double s = a_acc * (here ? d0 : V.d[i]);
             V.s[i] = s;
-            V.y[i] = gt - V.g[i];
+            V.y[i] = gt - (here ? g0 : V.g[i]);
             most[1] = nanmax(most[1], s);
         }
-        V.theta[i] = th_src[i];
+        V.theta[i] = th;
         V.g[i] = gt;
         most[0] = nanmax(most[0], gt);
     }
-    block_reduce<2, true>(most, sh);
+    const double f_acc = use_best ? f_b : ft;
+    const bool flat = threadIdx.x < 32 && fabs(f0 - f_acc) <= V.f_reltol * fabs(f_acc);
+    block_max(most, sh_max);
     const double gmax = most[0], smax = most[1];
     if (threadIdx.x == 0) {
         S->f_prev = first ? f_acc : f0;
@@ -279,7 +366,7 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V
         } else if (gmax <= V.g_abstol) {
             status = SFH_FIT_CONVERGED_G;
         } else if (!first) {
-            if (fabs(f0 - f_acc) <= V.f_reltol * fabs(f_acc)) status = SFH_FIT_CONVERGED_F;
+            if (flat) status = SFH_FIT_CONVERGED_F;
             else if (smax <= V.x_abstol) status = SFH_FIT_CONVERGED_X;
         }
         if (!first) S->iter += 1;
@@ -295,62 +382,93 @@ __global__ void __launch_bounds__(kVecThreads) k_fit_eval(FitState *S, FitVecs V
 
 // Hy = H y, Hg = H g (H as I while a reset is pending), one warp per row.
 __global__ void __launch_bounds__(kRowWarps * 32) k_fit_hgemv(const FitState *S, FitVecs V) {
-    if (!S->accept) return;
     const int64_t nt = V.nt;
     const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= nt) return;
-    if (S->reset_h) {
+    const int accept = S->accept, reset = S->reset_h;
+    const double *row = V.H + i * nt;
+    double a = 0.0, b = 0.0;
+    for (int64_t j0 = 0; j0 < nt; j0 += 8 * 32) {  // eight columns' loads together
+        double h[8], y[8], g[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int64_t j = j0 + 32 * u + lane;
+            h[u] = j < nt ? row[j] : 0.0;
+            y[u] = j < nt ? V.y[j] : 0.0;
+            g[u] = j < nt ? V.g[j] : 0.0;
+        }
+        if (!accept) return;
+        if (reset) break;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (j0 + 32 * u + lane < nt) {
+                a = fma(h[u], y[u], a);
+                b = fma(h[u], g[u], b);
+            }
+    }
+    if (reset) {
         if (lane == 0) {
             V.Hy[i] = V.y[i];
             V.Hg[i] = V.g[i];
         }
         return;
     }
-    const double *row = V.H + i * nt;
-    double a = 0.0, b = 0.0;
-#pragma unroll 8
-    for (int64_t j = lane; j < nt; j += 32) {
-        const double h = row[j];
-        a = fma(h, V.y[j], a);
-        b = fma(h, V.g[j], b);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (lane == 0) {
-        V.Hy[i] = a;
-        V.Hg[i] = b;
-    }
+    const double ab[2] = {a, b};
+    const double t = warp_sums<2>(ab);
+    if (lane == 0) V.Hy[i] = t;
+    if (lane == 16) V.Hg[i] = t;
 }
 
 // H += c1 s sᵀ - c2 (Hy sᵀ + s Hyᵀ) with c1 = (sᵀy + yᵀHy) / (sᵀy)², c2 = 1 / sᵀy when
-// sᵀy > 0 (Optim's BFGS update_h!), and d = -H_new g from the same vectors.  Every CTA
+// sᵀy > 0 (Optim's BFGS update_h!), and d = -H_new g from the same vectors (contractions written
+// out: the iterates' bits do not hang on the compiler's choice).  Every CTA
 // forms the four dot products in the same order, so all see the same scalars.
 // A CTA takes `rows` rows; its threads share their elements.
 __global__ void __launch_bounds__(kRowWarps * 32) k_fit_hupdate(const FitState *S, FitVecs V, int rows) {
     __shared__ double sh[128];
-    if (!S->accept) return;
-    const int64_t nt = V.nt;
+    __shared__ double s_c[4];  // c1, c2, sᵀg, (Hy)ᵀg
+    __shared__ int s_upd;
+    const int64_t nt = V.nt, j0 = threadIdx.x;
+    const bool own = j0 < nt;
+    const double s0 = own ? V.s[j0] : 0.0, hy0 = own ? V.Hy[j0] : 0.0, g0 = own ? V.g[j0] : 0.0,
+                 y0 = own ? V.y[j0] : 0.0;
+    const int64_t i0 = (int64_t)blockIdx.x * rows;
+    const int nr = (int)min((int64_t)rows, nt - i0);
     const int reset = S->reset_h;
+    const double *vs = V.s, *vhy = V.Hy;
+    const bool mine = (int)threadIdx.x < nr;
+    const double my_hg = mine ? V.Hg[i0 + threadIdx.x] : 0.0, my_s = mine ? vs[i0 + threadIdx.x] : 0.0,
+                 my_hy = mine ? vhy[i0 + threadIdx.x] : 0.0;
+    if (!S->accept) return;
     double dots[4] = {0.0, 0.0, 0.0, 0.0};  // sᵀy, yᵀHy, sᵀg, (Hy)ᵀg
-    for (int64_t j = threadIdx.x; j < nt; j += blockDim.x) {
-        const double s = V.s[j], hy = V.Hy[j], g = V.g[j];
-        dots[0] += s * V.y[j];
-        dots[1] += V.y[j] * hy;
+    for (int64_t j = j0; j < nt; j += blockDim.x) {
+        const bool here = j == j0;
+        const double s = here ? s0 : vs[j], hy = here ? hy0 : vhy[j], g = here ? g0 : V.g[j],
+                     y = here ? y0 : V.y[j];
+        dots[0] += s * y;
+        dots[1] += y * hy;
         dots[2] += s * g;
         dots[3] += hy * g;
     }
-    block_reduce<4, false>(dots, sh);
-    const double sty = dots[0], yhy = dots[1], sg = dots[2], hyg = dots[3];
-    const bool upd = sty > 0.0 && sty < INFINITY && fabs(yhy) < INFINITY;
-    const double c1 = upd ? (sty + yhy) / (sty * sty) : 0.0, c2 = upd ? 1.0 / sty : 0.0;
-    const int64_t i0 = (int64_t)blockIdx.x * rows;
-    const int nr = (int)min((int64_t)rows, nt - i0);
+    block_sums<4>(dots, sh);
+    if (threadIdx.x < 32) {
+        const double sty = dots[0], yhy = dots[1];
+        const bool upd = sty > 0.0 && sty < INFINITY && fabs(yhy) < INFINITY;
+        // c1 in lane 0 and c2 in the others by one division
+        const bool l0 = threadIdx.x == 0;
+        const double c = upd ? (l0 ? sty + yhy : 1.0) / (l0 ? sty * sty : sty) : 0.0;
+        if (threadIdx.x < 2) s_c[threadIdx.x] = c;
+        if (l0) {
+            s_c[2] = dots[2];
+            s_c[3] = dots[3];
+            s_upd = upd;
+        }
+    }
+    __syncthreads();
+    const bool upd = s_upd != 0;
+    const double c1 = s_c[0], c2 = s_c[1], sg = s_c[2], hyg = s_c[3];
     double *H = V.H + i0 * nt;
-    const double *vs = V.s, *vhy = V.Hy;
     if (upd || reset) {
         const int total = nr * (int)nt, step = kRowWarps * 32;  // rows <= 8, nt < 2^27
         for (int k0 = threadIdx.x; k0 < total; k0 += 4 * step) {
@@ -369,14 +487,13 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_fit_hupdate(const FitState *
 #pragma unroll
             for (int u = 0; u < 4; ++u)
                 if (k0 + u * step < total)
-                    H[k0 + u * step] = h[u] + c1 * si[u] * sj[u] - c2 * (hyi[u] * sj[u] + si[u] * hyj[u]);
+                    H[k0 + u * step] = fma(-c2, fma(hyi[u], sj[u], __dmul_rn(si[u], hyj[u])),
+                                           fma(__dmul_rn(c1, si[u]), sj[u], h[u]));
         }
     }
-    if ((int)threadIdx.x < nr) {
-        const int64_t i = i0 + threadIdx.x;
-        const double si = vs[i], hyi = vhy[i];
-        V.d[i] = -(V.Hg[i] + c1 * si * sg - c2 * (hyi * sg + si * hyg));
-    }
+    if (mine)
+        V.d[i0 + threadIdx.x] =
+            -fma(-c2, fma(my_s, hyg, __dmul_rn(my_hy, sg)), fma(__dmul_rn(c1, my_s), sg, my_hg));
 }
 
 }  // namespace
