@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -120,6 +121,12 @@ __device__ __forceinline__ unsigned long long star_strips(const StarRec &r) {
 }
 struct StarId {
     int32_t t, q;  // template, star of the template
+};
+// What decides whether a warp wants a wide or mid star: first and last row, strips (none of a mid
+// star).  No rows for the other classes.
+struct __align__(16) StarKey {
+    int ylo, yhi;
+    unsigned long long strips;
 };
 // bits lo .. hi
 __device__ __forceinline__ unsigned long long strip_bits(int lo, int hi) {
@@ -347,13 +354,14 @@ __device__ __forceinline__ unsigned long long smooth_strips(const StarRec &r, co
     return m;
 }
 
-// Completes a star's record with its smooth strips, stores it, and lists it when it is narrow:
+// Completes a star's record with its smooth strips, stores it and its key, and lists it when it is narrow:
 // the narrow stars of all templates are in one list (one atomic per warp).
-__device__ __forceinline__ void store_record(StarRec &r, const Grid2 &g, StarId id, StarRec *to,
+__device__ __forceinline__ void store_record(StarRec &r, const Grid2 &g, StarId id, StarRec *to, StarKey *key,
                                              StarId *narrow, int *n_narrow) {
+    unsigned long long m = 0ull;
     if (r.cls == kStarWide) {
         const Smooth sm = smooth_tiling(g, true);
-        const unsigned long long m = sm.on ? smooth_strips(r, g, sm) : 0ull;
+        m = sm.on ? smooth_strips(r, g, sm) : 0ull;
         r.p[10] = __uint_as_float((unsigned int)m);
         r.p[11] = __uint_as_float((unsigned int)(m >> 32));
     }
@@ -366,6 +374,7 @@ __device__ __forceinline__ void store_record(StarRec &r, const Grid2 &g, StarId 
         narrow[at + __popc(nar & ((1u << lane) - 1u))] = id;
     }
     *to = r;
+    *key = r.cls == kStarWide || r.cls == kStarMid ? StarKey{r.ylo, r.yhi, m} : StarKey{INT_MAX, -1, 0ull};
 }
 
 constexpr int kPrepThreads = 64;  // small blocks: a few hundred stars already spread over the SMs
@@ -376,7 +385,7 @@ k_star_prep(const double *__restrict__ xs, const double *__restrict__ ys,
             const double *__restrict__ ws, const int64_t *__restrict__ start,
             const int32_t *__restrict__ count, const int32_t *__restrict__ covs, Grid2 g0,
             const Grid2 *__restrict__ grids, int t0, StarRec *__restrict__ rec,
-            StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
+            StarKey *__restrict__ key, StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
     const int t = t0 + blockIdx.y;
     const int q = blockIdx.x * kPrepThreads + threadIdx.x;
     if (q >= count[t]) return;
@@ -384,7 +393,7 @@ k_star_prep(const double *__restrict__ xs, const double *__restrict__ ys,
     StarRec r{};
     const Grid2 g = grids ? grids[t] : g0;
     star_record(r, g, xs[s], ys[s], sxs[s], sys[s], ws[s], covs[t]);
-    store_record(r, g, StarId{t, q}, rec + s, narrow, n_narrow);
+    store_record(r, g, StarId{t, q}, rec + s, key + s, narrow, n_narrow);
 }
 
 // ---------------------------------------------------------------- narrow stars
@@ -683,6 +692,7 @@ struct StampStars {
     const StarRec *rec;  // one per star, where the star counts are known to the host
     const int64_t *start;
     const int32_t *count, *cov;
+    const StarKey *key = nullptr;  // with rec
 };
 
 struct WarpStars {
@@ -694,21 +704,32 @@ struct WarpStars {
 // sg + ns, ...: 32 at a time, one per lane, those wanted are compacted into its slots in
 // order.  Wanted: wide or mid, with a window that reaches rows ty0 .. ty1; of the wide stars
 // those that have (NODES) or lack (else) one of the strips.
+// With records the stars are chosen by their keys, fetched 32 ahead (16 bytes a star and one load;
+// reading the record's class, rows and strips one after the other waited three times as long).
+__device__ __forceinline__ StarKey star_key(const StampStars &st, int64_t s0, int n, int q) {
+    if (q >= n) return StarKey{INT_MAX, -1, 0ull};
+    const int4 k = __ldg(reinterpret_cast<const int4 *>(st.key + s0 + q));
+    return StarKey{k.x, k.y, (unsigned int)k.z | (unsigned long long)(unsigned int)k.w << 32};
+}
+
 template <bool NODES, bool REC>
-__device__ __forceinline__ int next_stars(StarRec *slot, const StampStars &st, int64_t s0, int n,
-                                          int q0, int sg, int ns, const Grid2 &g, int cov, int ty0,
-                                          int ty1, unsigned long long strips) {
+__device__ __forceinline__ int next_stars(StarRec *slot, StarKey &key, const StampStars &st, int64_t s0,
+                                          int n, int q0, int sg, int ns, const Grid2 &g, int cov,
+                                          int ty0, int ty1, unsigned long long strips) {
     const int lane = threadIdx.x & 31, q = (q0 + lane) * ns + sg;
-    bool take = false;
     StarRec tmp;
     const StarRec *r = &tmp;
-    if (q < n) {
-        if (REC) r = st.rec + s0 + q;
-        else star_record(tmp, g, st.x[s0 + q], st.y[s0 + q], st.sx[s0 + q], st.sy[s0 + q], st.w[s0 + q], cov);
-        take = (r->cls == kStarWide || (!NODES && r->cls == kStarMid)) && r->ylo <= ty1 && r->yhi >= ty0;
-        if (take && r->cls == kStarWide)
-            take = ((NODES ? star_strips(*r) : ~star_strips(*r)) & strips) != 0ull;
+    if (REC) {
+        r = st.rec + s0 + q;
+    } else {
+        key = StarKey{INT_MAX, -1, 0ull};
+        if (q < n) {
+            star_record(tmp, g, st.x[s0 + q], st.y[s0 + q], st.sx[s0 + q], st.sy[s0 + q], st.w[s0 + q], cov);
+            if (tmp.cls == kStarWide || tmp.cls == kStarMid) key = StarKey{tmp.ylo, tmp.yhi, 0ull};
+        }
     }
+    const bool take = key.ylo <= ty1 && key.yhi >= ty0 && ((NODES ? key.strips : ~key.strips) & strips) != 0ull;
+    if (REC) key = star_key(st, s0, n, q + 32 * ns);
     const unsigned m = __ballot_sync(0xffffffffu, take);
     if (take) {
         const float4 *from = reinterpret_cast<const float4 *>(r);
@@ -741,8 +762,10 @@ __device__ __forceinline__ void add_stars(float2 (&acc)[8][4], WarpStars &W, con
     for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[j][c] = make_float2(0.f, 0.f);
+    StarKey key{};
+    if (REC) key = star_key(st, s0, n, lane * ns + sg);
     for (int q0 = 0; q0 * ns + sg < n; q0 += 32) {
-        const int nw = next_stars<NODES, REC>(W.rec, st, s0, n, q0, sg, ns, g, cov, ty0, ty1, strips);
+        const int nw = next_stars<NODES, REC>(W.rec, key, st, s0, n, q0, sg, ns, g, cov, ty0, ty1, strips);
 #pragma unroll 1
         for (int k = 0; k < nw; ++k) {
             const StarRec &r = W.rec[k];
@@ -850,13 +873,17 @@ __host__ __device__ inline int tile_groups(int64_t nx, int64_t ny) {
 
 template <bool REC>
 __global__ void __launch_bounds__(kTileWarpsMax * 32, 1)
-k_stamp_tiles(StampStars st, Grid2 g0, const StampGroup *__restrict__ groups,
+k_stamp_tiles(StampStars st, Grid2 g0, int ntempl, const StampGroup *__restrict__ groups,
               const Grid2 *__restrict__ grids, const int64_t *__restrict__ out_off,
               const int64_t *__restrict__ node_off, const float *__restrict__ node,
               float *__restrict__ out) {
     extern __shared__ __align__(16) float smem[];  // [2048] node rows, [ns > 1: 2048] sums, warps
     const int ns = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const StampGroup gr = groups ? groups[blockIdx.x] : StampGroup{(int)blockIdx.y, (int)blockIdx.x};
+    // on one grid the groups of the last rows first, all templates' together: magnitudes grow with
+    // the row, and the faint end's groups take longest
+    const StampGroup gr = groups ? groups[blockIdx.x]
+                                 : StampGroup{(int)(blockIdx.x % (unsigned)ntempl),
+                                              (int)((gridDim.x - 1 - blockIdx.x) / (unsigned)ntempl)};
     const int t = gr.t, cov = st.cov[t];
     const Grid2 g = grids ? grids[t] : g0;
     float *mid = smem, *sum = smem + 2048;
@@ -1133,8 +1160,8 @@ k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
             const int64_t *__restrict__ iso_off, const int32_t *__restrict__ iso_len,
             const double *__restrict__ dmods, const double *__restrict__ norms, IsoParams P,
             const double *__restrict__ dmag_t, const int64_t *__restrict__ star_off, Grid2 g0,
-            const Grid2 *__restrict__ grids, StarRec *__restrict__ rec, StarId *__restrict__ narrow,
-            int *__restrict__ n_narrow, int32_t *__restrict__ count, int *__restrict__ err_flag) {
+            const Grid2 *__restrict__ grids, StarRec *__restrict__ rec, StarKey *__restrict__ key,
+            StarId *__restrict__ narrow, int *__restrict__ n_narrow, int32_t *__restrict__ count, int *__restrict__ err_flag) {
     __shared__ IsoPoint s_pt[kIsoThreads];
     __shared__ int s_cnt[kIsoMaxPts];
     __shared__ int s_pos[kIsoMaxPts];
@@ -1174,7 +1201,7 @@ k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
             StarRec r{};
             star_record(r, g, a.xcol + (b.xcol - a.xcol) * 0.5, a.ymag + (b.ymag - a.ymag) * 0.5,
                         a.cerr + (b.cerr - a.cerr) * 0.5, a.yerr + (b.yerr - a.yerr) * 0.5, w, cov);
-            store_record(r, g, StarId{t, q}, rec + so + q, narrow, n_narrow);
+            store_record(r, g, StarId{t, q}, rec + so + q, key + so + q, narrow, n_narrow);
         }
     }
 }
@@ -1203,6 +1230,7 @@ size_t node_bytes(const Grid2 &g, int64_t ntempl) {
 // Device workspace of the stamps, where the star counts are known to the host.
 struct StampWork {
     StarRec *rec = nullptr;    // one per star, indexed as the star arrays
+    StarKey *key = nullptr;    // the same
     StarId *narrow = nullptr;  // room for every star
     int *n_narrow = nullptr;
     float *node = nullptr;     // node_bytes() / the ragged batch's nodes
@@ -1210,15 +1238,17 @@ struct StampWork {
     bool made = false;         // the records are there already (k_iso_stars)
     static size_t bytes(int64_t stars, size_t node) {
         const size_t n = (size_t)std::max<int64_t>(stars, 1);
-        return 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarId)) + sfh_align256(node);
+        return 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarKey)) +
+               sfh_align256(n * sizeof(StarId)) + sfh_align256(node);
     }
     StampWork() = default;
     StampWork(char *b, int64_t stars, int64_t maxcount_) : maxcount(maxcount_) {
         const size_t n = (size_t)std::max<int64_t>(stars, 1);
         n_narrow = (int *)b;
-        rec = (StarRec *)(b + 256);
-        narrow = (StarId *)(b + 256 + sfh_align256(n * sizeof(StarRec)));
-        node = (float *)(b + 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarId)));
+        rec = (StarRec *)(b += 256);
+        key = (StarKey *)(b += sfh_align256(n * sizeof(StarRec)));
+        narrow = (StarId *)(b += sfh_align256(n * sizeof(StarKey)));
+        node = (float *)(b + sfh_align256(n * sizeof(StarId)));
     }
 };
 
@@ -1244,6 +1274,7 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
         return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
     const bool have = w.rec != nullptr;
     st.rec = w.rec;
+    st.key = w.key;
     const Smooth sm = smooth_tiling(g, have && !rg);
     const int node_groups = rg ? rg->max_node_groups : sm.on ? sm.groups() : 0;
     cudaStream_t s = ctx->stream;
@@ -1264,7 +1295,7 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
             k_star_prep<<<dim3((unsigned)((w.maxcount + kPrepThreads - 1) / kPrepThreads), nt),
                           kPrepThreads, 0, s>>>(st.x, st.y, st.sx, st.sy, st.w, st.start, st.count,
                                                 st.cov, g, rg ? rg->grids : nullptr, (int)t0, w.rec,
-                                                w.narrow, w.n_narrow);
+                                                w.key, w.narrow, w.n_narrow);
             SFH_LAUNCHED(ctx);
         }
         if (node_groups > 0) {
@@ -1275,11 +1306,10 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     }
     const int64_t groups = rg ? rg->ngroups : ntempl * tile_groups(g.nx, g.ny);
     const int ns = tile_warps(groups, ctx->sm_count);
-    const dim3 grid = rg ? dim3((unsigned)groups) : dim3((unsigned)tile_groups(g.nx, g.ny), (unsigned)ntempl);
     auto tiles = have ? k_stamp_tiles<true> : k_stamp_tiles<false>;
-    tiles<<<grid, 32 * ns, tile_smem(ns), s>>>(st, g, rg ? rg->groups : nullptr, rg ? rg->grids : nullptr,
-                                               rg ? rg->out_off : nullptr, rg ? rg->node_off : nullptr,
-                                               node_groups > 0 ? w.node : nullptr, d_out);
+    tiles<<<(unsigned)groups, 32 * ns, tile_smem(ns), s>>>(
+        st, g, (int)ntempl, rg ? rg->groups : nullptr, rg ? rg->grids : nullptr, rg ? rg->out_off : nullptr,
+        rg ? rg->node_off : nullptr, node_groups > 0 ? w.node : nullptr, d_out);
     SFH_LAUNCHED(ctx);
     const int buf = (int)nx + kNarrowRows;
     const unsigned blocks = 8u * (unsigned)ctx->sm_count;
@@ -1507,7 +1537,7 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
         d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len),
         (const double *)(b + o_dm), (const double *)(b + o_nm), P, dmag(),
         (const int64_t *)(b + o_soff), g, rg ? (const Grid2 *)(b + o_grid) : nullptr, work.rec,
-        work.narrow, work.n_narrow, (int32_t *)(b + o_cnt), (int *)(b + o_err));
+        work.key, work.narrow, work.n_narrow, (int32_t *)(b + o_cnt), (int *)(b + o_err));
     SFH_LAUNCHED(ctx);
     StampGrids sg{};
     if (rg)
@@ -1565,6 +1595,7 @@ extern "C" int sfh_partial_cmd_smooth_ragged_dev(
     rg.out_off.resize((size_t)ntempl);
     rg.node_off.resize((size_t)ntempl);
     rg.dmag.resize((size_t)ntempl);
+    int64_t ngroups = 0;
     for (int64_t t = 0; t < ntempl; ++t) {
         const sfh_hess_grid &h = h_grids[t];
         if (h.nx < 1 || h.ny < 1 || h.nx > (1 << 20) || h.ny > (1 << 20) || !(h.x_step != 0) ||
@@ -1584,10 +1615,18 @@ extern "C" int sfh_partial_cmd_smooth_ragged_dev(
         }
         rg.dmag[(size_t)t] = std::fmin(std::fabs(h.x_step), std::fabs(h.y_step));  // :851
         rg.max_nx = std::max(rg.max_nx, h.nx);
-        for (int k = 0; k < tile_groups(h.nx, h.ny); ++k) rg.groups.push_back(StampGroup{(int32_t)t, k});
+        ngroups += tile_groups(h.nx, h.ny);
     }
-    if (rg.groups.size() > 0x7fffffffu)
-        return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "too many stamp tiles");
+    if (ngroups > 0x7fffffff) return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "too many stamp tiles");
+    // the last rows of every grid first, as on one grid
+    rg.groups.reserve((size_t)ngroups);
+    constexpr int kBands = 16;
+    for (int q = kBands - 1; q >= 0; --q)
+        for (int64_t t = 0; t < ntempl; ++t) {
+            const int64_t n = tile_groups(rg.grids[(size_t)t].nx, rg.grids[(size_t)t].ny);
+            for (int64_t k = n * q / kBands; k < n * (q + 1) / kBands; ++k)
+                rg.groups.push_back(StampGroup{(int32_t)t, (int32_t)k});
+        }
     P.dmag = rg.dmag[0];
     return partial_run(ctx, d_m_ini, d_mags, h_iso_off, h_iso_len, ntempl, P, y_index, c1, h_dmod,
                        h_norm, &rg, 0.0, 0.0, 0, 0.0, 0.0, 0, d_models);
@@ -1740,7 +1779,7 @@ k_bin_count(const double *__restrict__ hist, int64_t nbins, int32_t *__restrict_
 __global__ void __launch_bounds__(kPairThreads)
 k_bin_points(IsoParams P, const double *__restrict__ hist, Grid2 g, const int64_t *__restrict__ start,
              const int32_t *__restrict__ first, int cov, StarRec *__restrict__ rec,
-             StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
+             StarKey *__restrict__ key, StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
     __shared__ int s_list[kSegBins];
     __shared__ int s_red[kPairThreads / 32];
     const int64_t nbins = (int64_t)g.nx * g.ny;
@@ -1785,7 +1824,10 @@ k_bin_points(IsoParams P, const double *__restrict__ hist, Grid2 g, const int64_
         const double xmag = (P.y_index == P.c1) ? cy - cx : cy + cx;  // :692-695
         StarRec r{};
         star_record(r, g, cx, cy, err_eval(P, xc, xmag), err_eval(P, P.y_index, cy), h[k], cov);
-        store_record(r, g, StarId{(int)blockIdx.y, q0 + p}, rec + start[blockIdx.y] + q0 + p, narrow, n_narrow);
+        {
+            const int64_t s = start[blockIdx.y] + q0 + p;
+            store_record(r, g, StarId{(int)blockIdx.y, q0 + p}, rec + s, key + s, narrow, n_narrow);
+        }
     }
 }
 
@@ -1908,7 +1950,7 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
         const int64_t *d_start = (const int64_t *)(b + o_up + 256);
         const int32_t *d_cnt = (const int32_t *)(b + o_up + 256 + sfh_align256(chunk * 8));
         k_bin_points<<<dim3((unsigned)nseg, (unsigned)nc), kPairThreads, 0, st>>>(
-            P, hist, g, d_start, (const int32_t *)(b + o_up + up), cov, work.rec, work.narrow, work.n_narrow);
+            P, hist, g, d_start, (const int32_t *)(b + o_up + up), cov, work.rec, work.key, work.narrow, work.n_narrow);
         SFH_LAUNCHED(ctx);
         rc = launch_stamps(ctx, StampStars{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d_start,
                                            d_cnt, (const int32_t *)(b + o_cov)},
