@@ -1210,12 +1210,15 @@ k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
 constexpr int64_t kMaxColumns = 3123;
 
 // Warps per tile group: as many as the stars can be dealt to while all groups together stay
-// within four waves of 16 warps (128 registers) per SM: a group in the dense part of a diagram takes
-// several times the mean, and one warp of it would be the tail (60 binary templates: 1.50 ms with
-// one warp per group, 0.59 ms with four).
-int tile_warps(int64_t groups, int sm_count) {
+// within six waves of 16 warps (128 registers) per SM: a group in the dense part of a diagram takes
+// several times the mean, and one warp of it would be the tail.  Templates on grids of their own
+// have different numbers of stars too: four times that.  k_stamp_tiles with 1, 2, 4, 8, 16 warps,
+// us: 60 binary templates (1,800 groups) 1,500, -, 335, 292, 394; 300 separable (5,100) 173, 180,
+// 201, 295; 1,200 (36,000) 2,540 with one; 768 templates of 64 galaxies (12,360) 1,880, 1,500, 1,360.
+int tile_warps(int64_t groups, bool uneven, int sm_count) {
+    const int64_t most = (uneven ? 384 : 96) * (int64_t)sm_count;
     int ns = 1;
-    while (ns < kTileWarpsMax && groups * 2 * ns <= 64 * (int64_t)sm_count) ns *= 2;
+    while (ns < kTileWarpsMax && groups * 2 * ns <= most) ns *= 2;
     return ns;
 }
 
@@ -1305,7 +1308,7 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
         }
     }
     const int64_t groups = rg ? rg->ngroups : ntempl * tile_groups(g.nx, g.ny);
-    const int ns = tile_warps(groups, ctx->sm_count);
+    const int ns = tile_warps(groups, rg != nullptr, ctx->sm_count);
     auto tiles = have ? k_stamp_tiles<true> : k_stamp_tiles<false>;
     tiles<<<(unsigned)groups, 32 * ns, tile_smem(ns), s>>>(
         st, g, (int)ntempl, rg ? rg->groups : nullptr, rg ? rg->grids : nullptr, rg ? rg->out_off : nullptr,
