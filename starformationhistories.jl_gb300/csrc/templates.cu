@@ -1045,7 +1045,7 @@ __device__ __forceinline__ double compl_eval(const IsoParams &P, int f, double m
 
 // Resampled point q of the isochrone (mini_spacing + interpolate_mini + callables).
 __device__ IsoPoint iso_point(const IsoParams &P, const double *m, const double *mags, int n,
-                              const int *pos, const int *cnt, double dmod, int q) {
+                              const int *pos, double dmod, int q) {
     int k = 0;
     double mass, frac;
     if (q == 0) {
@@ -1060,7 +1060,7 @@ __device__ IsoPoint iso_point(const IsoParams &P, const double *m, const double 
         }
         k = lo;
         const int j = q - pos[k] + 1;
-        const int c = cnt[k];
+        const int c = pos[k + 1] - pos[k];
         if (c == 1) {
             mass = m[k + 1];
             frac = 1.0;
@@ -1083,7 +1083,8 @@ __device__ IsoPoint iso_point(const IsoParams &P, const double *m, const double 
     IsoPoint p;
     p.mass = mass;
     const double e1 = err_eval(P, P.c1, mag[0]), e2 = err_eval(P, P.c2, mag[1]);
-    const double ey = err_eval(P, P.y_index, mag[2]);
+    // (the y filter is usually one of the two)
+    const double ey = P.y_index == P.c1 ? e1 : P.y_index == P.c2 ? e2 : err_eval(P, P.y_index, mag[2]);
     double comp = compl_eval(P, P.c1, mag[0]) * compl_eval(P, P.c2, mag[1]);
     if (P.covariant) {
         p.cerr = (P.y_index == P.c1) ? e2 : e1;  // error of the non-y filter, :862
@@ -1098,116 +1099,108 @@ __device__ IsoPoint iso_point(const IsoParams &P, const double *m, const double 
     return p;
 }
 
-// Segment insertion counts (:128-137) and their exclusive scan, in shared memory.
-// Returns N = 1 + sum(cnt) (number of resampled points); sets *bad when masses
-// are not strictly increasing.
-__device__ int iso_scan(const IsoParams &P, double dmag, const double *m, const double *mg, int n,
-                        int *s_cnt, int *s_pos, int *s_warp, int *bad) {
-    const int nseg = n - 1;
-    for (int k = threadIdx.x; k < nseg; k += blockDim.x) {
-        const double *vc1 = mg + (int64_t)P.c1 * P.total, *vc2 = mg + (int64_t)P.c2 * P.total;
-        const double *vy = mg + (int64_t)P.y_index * P.total;
-        const double dc = (vc1[k + 1] - vc2[k + 1]) - (vc1[k] - vc2[k]);
-        const double dy = vy[k + 1] - vy[k];
-        const double d = hypot(dc, dy);
-        int c = 1;
-        if (d > dmag) {
-            const double r = ceil(d / dmag);
-            c = r < 1.0e7 ? (int)r : 10000000;
-        }
-        if (!(m[k + 1] > m[k])) atomicExch(bad, 2);
-        s_cnt[k] = c;
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int carry = 1;
-    for (int base = 0; base < nseg; base += blockDim.x) {
-        const int k = base + threadIdx.x;
-        const int v = (k < nseg) ? s_cnt[k] : 0;
-        int incl = v;
-#pragma unroll
-        for (int o2 = 1; o2 < 32; o2 <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o2);
-            if (lane >= o2) incl += y;
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        int wpre = 0, tot = 0;
-        for (int w = 0; w < kIsoThreads / 32; ++w) {
-            if (w < warp) wpre += s_warp[w];
-            tot += s_warp[w];
-        }
-        if (k < nseg) s_pos[k] = carry + wpre + incl - v;
-        carry += tot;
-        __syncthreads();
-    }
-    return carry;
-}
-
+// Segment insertion counts (:128-137) and their exclusive scan: pos[k] is the number of the first
+// resampled point of segment k, pos[nseg] = N = 1 + sum(cnt) the number of points.  Flags masses
+// that are not strictly increasing.
 __global__ void __launch_bounds__(kIsoThreads)
 k_iso_count(const double *__restrict__ m_ini, const double *__restrict__ mags,
             const int64_t *__restrict__ iso_off, const int32_t *__restrict__ iso_len, IsoParams P,
-            const double *__restrict__ dmag_t, int64_t *__restrict__ nstars_out,
-            int *__restrict__ err_flag) {
-    __shared__ int s_cnt[kIsoMaxPts];
-    __shared__ int s_pos[kIsoMaxPts];
-    __shared__ int s_warp[kIsoThreads / 32];
-    const int t = blockIdx.x;
-    const int n = iso_len[t];
+            const double *__restrict__ dmag_t, const int64_t *__restrict__ pos_off,
+            int *__restrict__ pos_all, int64_t *__restrict__ nstars_out, int *__restrict__ err_flag) {
+    __shared__ int s_warp[2][kIsoThreads / 32];
+    const int t = blockIdx.x, nseg = iso_len[t] - 1;
     const double dmag = dmag_t ? dmag_t[t] : P.dmag;
-    const int npts = iso_scan(P, dmag, m_ini + iso_off[t], mags + iso_off[t], n, s_cnt, s_pos,
-                              s_warp, err_flag);
-    if (threadIdx.x == 0) nstars_out[t] = npts - 1;
+    const double *m = m_ini + iso_off[t], *mg = mags + iso_off[t];
+    const double *vc1 = mg + (int64_t)P.c1 * P.total, *vc2 = mg + (int64_t)P.c2 * P.total;
+    const double *vy = mg + (int64_t)P.y_index * P.total;
+    int *pos = pos_all + pos_off[t];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 1, round = 0;
+    for (int base = 0; base < nseg; base += kIsoThreads, round ^= 1) {
+        const int k = base + (int)threadIdx.x;
+        int v = 0;
+        if (k < nseg) {
+            const double dc = (vc1[k + 1] - vc2[k + 1]) - (vc1[k] - vc2[k]);
+            const double dy = vy[k + 1] - vy[k];
+            const double d = hypot(dc, dy);
+            v = 1;
+            if (d > dmag) {
+                const double r = ceil(d / dmag);
+                v = r < 1.0e7 ? (int)r : 10000000;
+            }
+            if (!(m[k + 1] > m[k])) atomicExch(err_flag, 2);
+        }
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_warp[round][warp] = incl;
+        __syncthreads();
+        int wpre = 0, tot = 0;
+        for (int w = 0; w < kIsoThreads / 32; ++w) {
+            if (w < warp) wpre += s_warp[round][w];
+            tot += s_warp[round][w];
+        }
+        if (k < nseg) pos[k] = carry + wpre + incl - v;
+        carry += tot;
+    }
+    if (threadIdx.x == 0) {
+        pos[max(nseg, 0)] = carry;
+        nstars_out[t] = carry - 1;
+    }
 }
 
-__global__ void __launch_bounds__(kIsoThreads)
+// One block of stars: template, first star.
+struct IsoBlock {
+    int32_t t, base;
+};
+constexpr int kStarThreads = 128;
+constexpr int kIsoStars = kStarThreads - 1;
+
+// A thread per point, blocks of points overlapping by one: a star is a point and its right
+// neighbour (midpoints and weight, :765-776, :884-888).  Bound by FP64.  Blocks of 127 stars of any
+// template.  With a block per template, which counted the segments over again and took the stars
+// in turn, and the y filter's error evaluated a second time: 679 us for 1,200 templates, 684 for
+// the 768 of 64 galaxies (0.2 to 5 thousand stars each), 152 for 300, 23 for 6; this way 645, 510,
+// 157, 18.
+__global__ void __launch_bounds__(kStarThreads)
 k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
             const int64_t *__restrict__ iso_off, const int32_t *__restrict__ iso_len,
             const double *__restrict__ dmods, const double *__restrict__ norms, IsoParams P,
-            const double *__restrict__ dmag_t, const int64_t *__restrict__ star_off, Grid2 g0,
+            const int64_t *__restrict__ pos_off, const int *__restrict__ pos_all,
+            const IsoBlock *__restrict__ blocks, const int64_t *__restrict__ star_off, Grid2 g0,
             const Grid2 *__restrict__ grids, StarRec *__restrict__ rec, StarKey *__restrict__ key,
-            StarId *__restrict__ narrow, int *__restrict__ n_narrow, int32_t *__restrict__ count, int *__restrict__ err_flag) {
-    __shared__ IsoPoint s_pt[kIsoThreads];
-    __shared__ int s_cnt[kIsoMaxPts];
+            StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
+    __shared__ IsoPoint s_pt[kStarThreads];
     __shared__ int s_pos[kIsoMaxPts];
-    __shared__ int s_warp[kIsoThreads / 32];
-    const int t = blockIdx.x;
-    const int n = iso_len[t];
-    const double *m = m_ini + iso_off[t];
-    const double *mg = mags + iso_off[t];
-    const int npts = iso_scan(P, dmag_t ? dmag_t[t] : P.dmag, m, mg, n, s_cnt, s_pos, s_warp,
-                              err_flag);
-    const int nstars = npts - 1;
-    if (nstars != (int)(star_off[t + 1] - star_off[t])) {  // counts come from k_iso_count
-        if (threadIdx.x == 0) { count[t] = 0; atomicExch(err_flag, 1); }
-        return;
-    }
-    if (threadIdx.x == 0) count[t] = nstars;
-    const double dmod = dmods[t];
-    const double wscale = norms[t] * P.inv_mean_mass;
+    const IsoBlock blk = blocks[blockIdx.x];
+    const int t = blk.t, n = iso_len[t];
+    const int *pos = pos_all + pos_off[t];
+    for (int k = threadIdx.x; k < n; k += kStarThreads) s_pos[k] = pos[k];
+    __syncthreads();
+    const double *m = m_ini + iso_off[t], *mg = mags + iso_off[t];
+    const int npts = s_pos[n - 1];
     const int64_t so = star_off[t];
-    // A thread per point, blocks of points overlapping by one: a star is a point and its right
-    // neighbour (midpoints and weight, :765-776, :884-888).
     const Grid2 g = grids ? grids[t] : g0;
     const int cov = P.covariant ? (P.y_index == P.c1 ? -1 : 1) : 0;
-    for (int base = 0; base < nstars; base += kIsoThreads - 1) {
-        const int q = base + (int)threadIdx.x;
-        IsoPoint a;
-        if (q < npts) {
-            a = iso_point(P, m, mg, n, s_pos, s_cnt, dmod, q);
-            a.pdf = imf_pdf(P, a.mass);
-        }
-        __syncthreads();  // the previous block's points are no longer read
-        if (q < npts) s_pt[threadIdx.x] = a;
-        __syncthreads();
-        if (threadIdx.x < kIsoThreads - 1 && q < nstars) {
-            const IsoPoint &b = s_pt[threadIdx.x + 1];
-            const double w = (b.mass - a.mass) * (a.pdf + b.pdf) * 0.5 * a.compl_ * wscale;
-            StarRec r{};
-            star_record(r, g, a.xcol + (b.xcol - a.xcol) * 0.5, a.ymag + (b.ymag - a.ymag) * 0.5,
-                        a.cerr + (b.cerr - a.cerr) * 0.5, a.yerr + (b.yerr - a.yerr) * 0.5, w, cov);
-            store_record(r, g, StarId{t, q}, rec + so + q, key + so + q, narrow, n_narrow);
-        }
+    const int q = blk.base + (int)threadIdx.x;
+    IsoPoint a;
+    if (q < npts) {
+        a = iso_point(P, m, mg, n, s_pos, dmods[t], q);
+        a.pdf = imf_pdf(P, a.mass);
+        s_pt[threadIdx.x] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x < kIsoStars && q < npts - 1) {
+        const IsoPoint &b = s_pt[threadIdx.x + 1];
+        const double wscale = norms[t] * P.inv_mean_mass;
+        const double w = (b.mass - a.mass) * (a.pdf + b.pdf) * 0.5 * a.compl_ * wscale;
+        StarRec r{};
+        star_record(r, g, a.xcol + (b.xcol - a.xcol) * 0.5, a.ymag + (b.ymag - a.ymag) * 0.5,
+                    a.cerr + (b.cerr - a.cerr) * 0.5, a.yerr + (b.yerr - a.yerr) * 0.5, w, cov);
+        store_record(r, g, StarId{t, q}, rec + so + q, key + so + q, narrow, n_narrow);
     }
 }
 
@@ -1487,38 +1480,47 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
                 const double *h_norm, const RaggedSpec *rg, double xf, double xs, int64_t nx,
                 double yf, double ys, int64_t ny, float *d_models) {
     cudaStream_t st = ctx->stream;
-    // What the host knows, in one upload: star offsets (known after pass 1) first, then the
-    // per-template inputs and the zeroed counters; the star counts follow the counters, so
-    // that pass 1 is read back in one copy.
+    // What the host knows, in one upload, ending in the zeroed counters; the star counts follow
+    // them, so that pass 1 is read back in one copy.
     std::vector<char> head;
-    auto add = [&](const void *src, size_t bytes) {
-        const size_t at = head.size();
-        head.resize(at + sfh_align256(bytes), 0);
-        if (src) std::memcpy(head.data() + at, src, bytes);
+    auto add = [](std::vector<char> &to, const void *src, size_t bytes) {
+        const size_t at = to.size();
+        to.resize(at + sfh_align256(bytes), 0);
+        if (src) std::memcpy(to.data() + at, src, bytes);
         return at;
     };
     const size_t n8 = (size_t)ntempl * 8, n4 = (size_t)ntempl * 4;
     const std::vector<int32_t> cov((size_t)ntempl, P.covariant ? (y_index == c1 ? -1 : 1) : 0);
-    const size_t o_soff = add(nullptr, n8 + 8);
-    const size_t o_off = add(h_iso_off, n8), o_len = add(h_iso_len, n4), o_dm = add(h_dmod, n8);
-    const size_t o_nm = add(h_norm, n8), o_cov = add(cov.data(), n4);
-    const size_t o_dmag = rg ? add(rg->dmag.data(), n8) : 0;
-    const size_t o_grid = rg ? add(rg->grids.data(), ntempl * sizeof(Grid2)) : 0;
-    const size_t o_oof = rg ? add(rg->out_off.data(), n8) : 0, o_noff = rg ? add(rg->node_off.data(), n8) : 0;
-    const size_t o_groups = rg ? add(rg->groups.data(), rg->groups.size() * sizeof(StampGroup)) : 0;
-    const size_t o_err = add(nullptr, 8), o_cnt64 = head.size();  // error flag, narrow stars
-    const size_t o_cnt = o_cnt64 + sfh_align256(n8), o_work = o_cnt + sfh_align256(n4);
+    std::vector<int64_t> poff((size_t)ntempl);
+    int64_t npos = 0;
+    for (int64_t t = 0; t < ntempl; ++t) {
+        poff[(size_t)t] = npos;
+        npos += std::max(h_iso_len[t], 1);
+    }
+    const size_t o_off = add(head, h_iso_off, n8), o_len = add(head, h_iso_len, n4);
+    const size_t o_dm = add(head, h_dmod, n8), o_nm = add(head, h_norm, n8);
+    const size_t o_cov = add(head, cov.data(), n4), o_poff = add(head, poff.data(), n8);
+    const size_t o_dmag = rg ? add(head, rg->dmag.data(), n8) : 0;
+    const size_t o_grid = rg ? add(head, rg->grids.data(), ntempl * sizeof(Grid2)) : 0;
+    const size_t o_oof = rg ? add(head, rg->out_off.data(), n8) : 0;
+    const size_t o_noff = rg ? add(head, rg->node_off.data(), n8) : 0;
+    const size_t o_groups = rg ? add(head, rg->groups.data(), rg->groups.size() * sizeof(StampGroup)) : 0;
+    const size_t o_err = add(head, nullptr, 8), o_cnt64 = head.size();  // error flag, narrow stars
+    const size_t o_pos = o_cnt64 + sfh_align256(n8), o_late = o_pos + sfh_align256((size_t)npos * 4);
     // Pass 1: resampled star count per template (one read-back), exact offsets.
-    int rc = sfh_scratch_reserve(ctx, o_work);
+    int rc = sfh_scratch_reserve(ctx, o_late);
     if (rc) return rc;
     char *b = (char *)ctx->scratch;
-    SFH_CK(ctx, cudaMemcpyAsync(b + o_off, head.data() + o_off, head.size() - o_off,
-                                cudaMemcpyHostToDevice, st));
     const auto dmag = [&] { return rg ? (const double *)(b + o_dmag) : nullptr; };  // per-template Δmag
-    k_iso_count<<<(unsigned)ntempl, kIsoThreads, 0, st>>>(
-        d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len), P, dmag(),
-        (int64_t *)(b + o_cnt64), (int *)(b + o_err));
-    SFH_LAUNCHED(ctx);
+    const auto pass1 = [&]() -> int {
+        SFH_CK(ctx, cudaMemcpyAsync(b, head.data(), head.size(), cudaMemcpyHostToDevice, st));
+        k_iso_count<<<(unsigned)ntempl, kIsoThreads, 0, st>>>(
+            d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len), P, dmag(),
+            (const int64_t *)(b + o_poff), (int *)(b + o_pos), (int64_t *)(b + o_cnt64), (int *)(b + o_err));
+        SFH_LAUNCHED(ctx);
+        return SFH_OK;
+    };
+    if ((rc = pass1())) return rc;
     std::vector<int64_t> back((o_cnt64 - o_err) / 8 + (size_t)ntempl);
     SFH_CK(ctx, cudaMemcpyAsync(back.data(), b + o_err, back.size() * 8, cudaMemcpyDeviceToHost, st));
     SFH_CK(ctx, cudaStreamSynchronize(st));
@@ -1526,31 +1528,49 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     std::memcpy(&flag, back.data(), 4);
     if (flag == 2) return sfh_set_error(ctx, SFH_ERR_ARG, "isochrone masses must be strictly increasing");
     const int64_t *nst = back.data() + (o_cnt64 - o_err) / 8;
-    int64_t *soff = (int64_t *)(head.data() + o_soff);
-    int64_t maxcount = 0;
+    std::vector<int64_t> soff((size_t)ntempl + 1);
+    std::vector<int32_t> count((size_t)ntempl);
+    int64_t maxcount = 0, nblocks = 0;
     for (int64_t t = 0; t < ntempl; ++t) {
-        soff[t + 1] = soff[t] + nst[t];
+        soff[(size_t)t + 1] = soff[(size_t)t] + nst[t];
+        count[(size_t)t] = (int32_t)nst[t];
         maxcount = std::max(maxcount, nst[t]);
+        nblocks += (nst[t] + kIsoStars - 1) / kIsoStars;
     }
-    const int64_t nstar_total = std::max<int64_t>(soff[ntempl], 1);
+    const int64_t nstar_total = std::max<int64_t>(soff[(size_t)ntempl], 1);
+    const size_t late_bytes = sfh_align256(n8 + 8) + sfh_align256(n4) +
+                              sfh_align256((size_t)nblocks * sizeof(IsoBlock));
+    const size_t o_work = o_late + late_bytes;
     // Pass 2: star records, then the stamps.
     const Grid2 g = make_grid(xf, xs, nx, yf, ys, ny);
     const size_t nodes = rg ? (size_t)rg->nodes * sizeof(float)
                             : nx <= kMaxColumns && ny <= (1 << 20) ? node_bytes(g, ntempl) : 0;
     rc = sfh_scratch_reserve(ctx, o_work + StampWork::bytes(nstar_total, nodes));
     if (rc) return rc;
-    const bool moved = b != (char *)ctx->scratch;
-    b = (char *)ctx->scratch;
-    SFH_CK(ctx, cudaMemcpyAsync(b, head.data(), moved ? head.size() : o_off, cudaMemcpyHostToDevice, st));
+    if (b != (char *)ctx->scratch) {  // a larger scratch: pass 1's results anew
+        b = (char *)ctx->scratch;
+        if ((rc = pass1())) return rc;
+    }
+    std::vector<IsoBlock> blocks;
+    blocks.reserve((size_t)nblocks);
+    for (int64_t t = 0; t < ntempl; ++t)
+        for (int64_t q = 0; q < nst[t]; q += kIsoStars) blocks.push_back(IsoBlock{(int32_t)t, (int32_t)q});
+    std::vector<char> late;  // known after pass 1
+    late.reserve(late_bytes);
+    const size_t o_soff = o_late + add(late, soff.data(), n8 + 8), o_cnt = o_late + add(late, count.data(), n4);
+    const size_t o_blk = o_late + add(late, blocks.data(), blocks.size() * sizeof(IsoBlock));
+    SFH_CK(ctx, cudaMemcpyAsync(b + o_late, late.data(), late.size(), cudaMemcpyHostToDevice, st));
     StampWork work(b + o_work, nstar_total, maxcount);
     work.made = true;
     work.n_narrow = (int *)(b + o_err) + 1;
-    k_iso_stars<<<(unsigned)ntempl, kIsoThreads, 0, st>>>(
-        d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len),
-        (const double *)(b + o_dm), (const double *)(b + o_nm), P, dmag(),
-        (const int64_t *)(b + o_soff), g, rg ? (const Grid2 *)(b + o_grid) : nullptr, work.rec,
-        work.key, work.narrow, work.n_narrow, (int32_t *)(b + o_cnt), (int *)(b + o_err));
-    SFH_LAUNCHED(ctx);
+    if (nblocks > 0) {
+        k_iso_stars<<<(unsigned)nblocks, kStarThreads, 0, st>>>(
+            d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len),
+            (const double *)(b + o_dm), (const double *)(b + o_nm), P, (const int64_t *)(b + o_poff),
+            (const int *)(b + o_pos), (const IsoBlock *)(b + o_blk), (const int64_t *)(b + o_soff), g,
+            rg ? (const Grid2 *)(b + o_grid) : nullptr, work.rec, work.key, work.narrow, work.n_narrow);
+        SFH_LAUNCHED(ctx);
+    }
     StampGrids sg{};
     if (rg)
         sg = StampGrids{(const Grid2 *)(b + o_grid), (const int64_t *)(b + o_oof),
@@ -1561,9 +1581,7 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
                                        (const int32_t *)(b + o_cov)},
                        ntempl, g, rg ? &sg : nullptr, work, d_models);
     if (rc) return rc;
-    SFH_CK(ctx, cudaMemcpyAsync(&flag, b + o_err, 4, cudaMemcpyDeviceToHost, st));
     SFH_CK(ctx, cudaStreamSynchronize(st));
-    if (flag) return sfh_set_error(ctx, SFH_ERR_CUDA, "resampled star count changed between passes");
     return SFH_OK;
 }
 }  // namespace
