@@ -1026,12 +1026,27 @@ struct IsoPoint {
     double mass, xcol, ymag, cerr, yerr, compl_, pdf;
 };
 
-__device__ __forceinline__ double imf_pdf(const IsoParams &P, double m) {
+// log2 to 2e-9 (the argument of an FP32 exponential, rounded to FP32 after a product with the
+// slope): 2^e c_j (1 + r), c_j = 1 + j / 128, |r| < 2^-7, r and log1p(r) in FP32; tab[j] = log c_j.
+// The library's FP64 log2 was a sixth of k_iso_stars.
+__device__ __forceinline__ double log2_fp32(double x, const sfh_df *__restrict__ tab) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)(b >> 52) - 1023, j = (int)(b >> 45) & 127;
+    if (e < -1000 || e > 1000) return log2(x);  // negative, subnormal, huge, inf or NaN
+    const float c = __uint_as_float(0x3f800000u | (unsigned)j << 16);
+    const float r = __fdividef((float)(unsigned)(b >> 13), c) * 1.8189894035458565e-12f;  // 2^-39
+    const sfh_df t = tab[j];
+    const float l = fmaf(r * r, fmaf(r, fmaf(r, -0.25f, 1.f / 3.f), -0.5f), r);
+    return fma((double)t.h + (double)(t.l + l), 1.4426950408889634, (double)e);
+}
+
+__device__ __forceinline__ double imf_pdf(const IsoParams &P, double m,
+                                          const sfh_df *__restrict__ tab = nullptr) {
     if (!(m >= P.imf_lo[0] && m <= P.imf_hi[P.nseg - 1])) return 0.0;
     int k = 0;
     while (k < P.nseg - 1 && m >= P.imf_hi[k]) ++k;
     return P.imf_scale[k] * P.imf_inv_norm *
-           (double)exp2f((float)(-P.imf_alpha[k] * log2(m)));
+           (double)exp2f((float)(-P.imf_alpha[k] * (tab ? log2_fp32(m, tab) : log2(m))));
 }
 
 __device__ __forceinline__ double err_eval(const IsoParams &P, int f, double m) {
@@ -1169,8 +1184,8 @@ __global__ void __launch_bounds__(kStarThreads)
 k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
             const int64_t *__restrict__ iso_off, const int32_t *__restrict__ iso_len,
             const double *__restrict__ dmods, const double *__restrict__ norms, IsoParams P,
-            const int64_t *__restrict__ pos_off, const int *__restrict__ pos_all,
-            const IsoBlock *__restrict__ blocks, const int64_t *__restrict__ star_off, Grid2 g0,
+            const sfh_df *__restrict__ tab, const int64_t *__restrict__ pos_off,
+            const int *__restrict__ pos_all, const IsoBlock *__restrict__ blocks, const int64_t *__restrict__ star_off, Grid2 g0,
             const Grid2 *__restrict__ grids, StarRec *__restrict__ rec, StarKey *__restrict__ key,
             StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
     __shared__ IsoPoint s_pt[kStarThreads];
@@ -1189,7 +1204,7 @@ k_iso_stars(const double *__restrict__ m_ini, const double *__restrict__ mags,
     IsoPoint a;
     if (q < npts) {
         a = iso_point(P, m, mg, n, s_pos, dmods[t], q);
-        a.pdf = imf_pdf(P, a.mass);
+        a.pdf = imf_pdf(P, a.mass, tab);
         s_pt[threadIdx.x] = a;
     }
     __syncthreads();
@@ -1566,7 +1581,8 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     if (nblocks > 0) {
         k_iso_stars<<<(unsigned)nblocks, kStarThreads, 0, st>>>(
             d_m_ini, d_mags, (const int64_t *)(b + o_off), (const int32_t *)(b + o_len),
-            (const double *)(b + o_dm), (const double *)(b + o_nm), P, (const int64_t *)(b + o_poff),
+            (const double *)(b + o_dm), (const double *)(b + o_nm), P, ctx->d_df_tab,
+            (const int64_t *)(b + o_poff),
             (const int *)(b + o_pos), (const IsoBlock *)(b + o_blk), (const int64_t *)(b + o_soff), g,
             rg ? (const Grid2 *)(b + o_grid) : nullptr, work.rec, work.key, work.narrow, work.n_narrow);
         SFH_LAUNCHED(ctx);
