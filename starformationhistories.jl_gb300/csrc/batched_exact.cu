@@ -406,28 +406,86 @@ __global__ void k_m_digits(const float *__restrict__ M, const float2 *__restrict
     }
 }
 
+// Σ_{i: n_i > 0} (n_i - n_i log n_i) in FP64: block k of kDcBlocks takes a contiguous chunk (the
+// log runs on the FP64 pipe, so the work is spread over the SMs), the last block sums the block
+// partials in block order (fixed order, reproducible) and re-arms the ticket.
+constexpr int kDcBlocks = 64;
+constexpr int kDigitThreads = 256;
+struct DataConst {
+    const double *n;  // NULL: not wanted
+    int64_t nbins;
+    double *part;
+    unsigned int *ticket;
+    double *kn;
+};
+__device__ __noinline__ void data_const(const DataConst &dc, int k) {
+    __shared__ double s[kDcBlocks];
+    __shared__ bool last;
+    const int64_t per = (dc.nbins + kDcBlocks - 1) / kDcBlocks;
+    const int64_t i0 = (int64_t)k * per, i1 = min(dc.nbins, i0 + per);
+    double a = 0.0;
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const double v = dc.n[i];
+        if (v > 0.0) a += v - v * log(v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s[w];
+        dc.part[k] = t;
+        __threadfence();
+        last = atomicAdd(dc.ticket, 1u) == kDcBlocks - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    if (threadIdx.x < kDcBlocks) {  // all partials on their way at once
+        __threadfence();
+        s[threadIdx.x] = ((volatile double *)dc.part)[threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int b = 0; b < kDcBlocks; ++b) t += s[b];
+        *dc.kn = t;
+        *dc.ticket = 0u;
+    }
+}
+
 // R digit planes: one block per vector b (B_pad blocks): S_b from max_j |R_bj|, then
 // plane p row b column j = d_p,bj for p < 8 (balanced base-64 digits of R_bj / S_b to
 // 2^-43, from integer arithmetic on the mantissa); padding rows and
 // columns zero.  The planes a launch needs: P = 6 while the ratio of the largest to the
 // smallest nonzero |R_bj| stays below 2^19, 7 below 2^25, else 8 (the maximum over the
-// batch, by atomicMax into *nplanes, which the caller zeroes first).
-__global__ void k_r_digits(const double *__restrict__ R, int64_t B, int64_t nt, int64_t B_pad,
-                           int64_t nt_pad, __nv_bfloat16 *__restrict__ planes,
-                           float *__restrict__ rscale, int *__restrict__ nplanes,
-                           const double *__restrict__ colsum, double *__restrict__ csum,
-                           int *__restrict__ negflag, const double *__restrict__ colsum_e,
-                           double *__restrict__ csum_e) {
+// batch, by atomicMax into *nplanes, which the caller zeroes first).  The first kDcBlocks blocks
+// form the data's constant when it is wanted (they overlap the rest; as a launch of its own it
+// took 14 us).  1,024 vectors of 1,200: 48 us with 64-bit digits, single stores and every
+// thread adding the warps' sums, now 27 us with the constant.
+__global__ void __launch_bounds__(kDigitThreads)
+k_r_digits(const double *__restrict__ R, int64_t B, int64_t nt, int64_t B_pad,
+           int64_t nt_pad, __nv_bfloat16 *__restrict__ planes,
+           float *__restrict__ rscale, int *__restrict__ nplanes,
+           const double *__restrict__ colsum, double *__restrict__ csum,
+           int *__restrict__ negflag, const double *__restrict__ colsum_e,
+           double *__restrict__ csum_e, const DataConst dc) {
     // integer operations wherever the result is exact (max / min of |R| on the bit patterns,
     // the digits from the mantissa): FP64 is the slow pipe; the two dot products stay FP64
-    __shared__ double s_d[2][32];
-    __shared__ unsigned long long s_m[2][32];
-    const int64_t b = blockIdx.x;
+    constexpr int kW = kDigitThreads / 32;
+    __shared__ double s_d[2][kW];
+    __shared__ unsigned long long s_m[2][kW];
+    const int first = dc.n ? kDcBlocks : 0;
+    if ((int)blockIdx.x < first) {
+        data_const(dc, blockIdx.x);
+        return;
+    }
+    const int64_t b = blockIdx.x - first;
     unsigned long long mxb = 0ull, mnb = ~0ull;  // |R| bit patterns: monotone in the value
     double dot = 0.0, dote = 0.0;
     bool neg = false;
     if (b < B)
-        for (int64_t j = threadIdx.x; j < nt; j += blockDim.x) {
+        for (int64_t j = threadIdx.x; j < nt; j += kDigitThreads) {
             const double v = R[b * nt + j];
             const unsigned long long ab = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
             mxb = ab > mxb ? ab : mxb;
@@ -454,54 +512,79 @@ __global__ void k_r_digits(const double *__restrict__ R, int64_t B, int64_t nt, 
     }
     __syncthreads();
     mxb = 0ull;
-    mnb = ~0ull;
-    dot = 0.0;
-    dote = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        mxb = s_m[0][w] > mxb ? s_m[0][w] : mxb;
-        mnb = s_m[1][w] < mnb ? s_m[1][w] : mnb;
-        dot += s_d[0][w];
-        dote += s_d[1][w];
-    }
-    if (threadIdx.x == 0) {
-        csum[b] = dot;
-        if (colsum_e) csum_e[b] = dote;
-    }
+#pragma unroll
+    for (int w = 0; w < kW; ++w) mxb = s_m[0][w] > mxb ? s_m[0][w] : mxb;
     const double mx = __longlong_as_double((long long)mxb);
     int e = 0;
     if (mx > 0.0) frexp(mx, &e);  // mx = f 2^e, f in [0.5, 1): |R_bj| < 2^e
     if (e < -120) e = -120;  // the scale stays a normal float
     if (e > 120) e = 120;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 2) {  // the dot products: a lane each
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kW; ++w) t += s_d[threadIdx.x][w];
+        if (threadIdx.x == 0) csum[b] = t;
+        else if (colsum_e) csum_e[b] = t;
+    }
+    if (threadIdx.x == 32) {
         rscale[b] = ldexpf(1.f, e);
         if (b < B && mx > 0.0) {
+            mnb = ~0ull;
+#pragma unroll
+            for (int w = 0; w < kW; ++w) mnb = s_m[1][w] < mnb ? s_m[1][w] : mnb;
             const double bits = log2(mx / __longlong_as_double((long long)mnb));
             atomicMax(nplanes, bits <= 19.0 ? 6 : bits <= 25.0 ? 7 : 8);
         }
     }
     // X = round(R_bj 2^(48 - e)) (|X| < 2^48: x = R 2^(6 - e) in units of 2^-42), then its
     // balanced base-64 digits from the top: d_p = round(X_p / 2^(42 - 6p)), X_{p+1} = X_p -
-    // d_p 2^(42 - 6p); |d_0| <= 64, |d_p| <= 32, Σ_p d_p 64^-p = x to 2^-43
-    for (int64_t j = threadIdx.x; j < nt_pad; j += blockDim.x) {
-        long long X = 0;
-        if (b < B && j < nt) {
-            const unsigned long long vb = (unsigned long long)__double_as_longlong(R[b * nt + j]);
-            const int E = (int)((vb >> 52) & 0x7ffu);
-            if (E) {  // subnormals are far below 2^(e - 48) unless every entry is: zero
-                const long long m = (long long)((vb & 0xfffffffffffffull) | (1ull << 52));
-                // m 2^(E - 1075 + 48 - e) = m / 2^sh, sh >= 5 for |R| < 2^e (sh is held at 5
-                // for coefficients beyond the clamped scale, 2^120)
-                const int sh = max(5, 1075 - 48 + e - E);
-                X = sh < 63 ? (m + (1ll << (sh - 1))) >> sh : 0;
-                if (vb >> 63) X = -X;
+    // d_p 2^(42 - 6p); |d_0| <= 64, |d_p| <= 32, Σ_p d_p 64^-p = x to 2^-43.  The halves of the
+    // digits' units above 2^18 are multiples of 2^18, so four digits come from X's upper 31 bits
+    // and the others from what is left of those and its lower 18, in 32-bit arithmetic.
+    for (int64_t j0 = 2 * (int64_t)threadIdx.x; j0 < nt_pad; j0 += 2 * kDigitThreads) {  // nt_pad is even
+        __nv_bfloat162 d2[kPMax];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t j = j0 + u;
+            long long X = 0;
+            if (b < B && j < nt) {
+                const unsigned long long vb = (unsigned long long)__double_as_longlong(R[b * nt + j]);
+                const int E = (int)((vb >> 52) & 0x7ffu);
+                if (E) {  // subnormals are far below 2^(e - 48) unless every entry is: zero
+                    const long long m = (long long)((vb & 0xfffffffffffffull) | (1ull << 52));
+                    // m 2^(E - 1075 + 48 - e) = m / 2^sh, sh >= 5 for |R| < 2^e (sh is held at 5
+                    // for coefficients beyond the clamped scale, 2^120)
+                    const int sh = max(5, 1075 - 48 + e - E);
+                    X = sh < 63 ? (m + (1ll << (sh - 1))) >> sh : 0;
+                    if (vb >> 63) X = -X;
+                }
+            }
+            int up = (int)(X >> 18), lo = (int)(X & 0x3ffff), d[kPMax];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const int sh = 24 - 6 * p;
+                d[p] = (up + (1 << (sh - 1))) >> sh;
+                up -= d[p] << sh;
+            }
+            const int carry = (lo + (1 << 17)) >> 18;
+            d[4] = up + carry;
+            lo -= carry << 18;
+#pragma unroll
+            for (int p = 5; p < kPMax; ++p) {
+                const int sh = 42 - 6 * p;
+                d[p] = sh ? (lo + (1 << (sh - 1))) >> sh : lo;
+                lo -= d[p] << sh;
+            }
+#pragma unroll
+            for (int p = 0; p < kPMax; ++p) {
+                const __nv_bfloat16 v = __float2bfloat16_rn((float)d[p]);
+                if (u) d2[p].y = v;
+                else d2[p].x = v;
             }
         }
-        for (int p = 0; p < kPMax; ++p) {
-            const int sh = 42 - 6 * p;
-            const long long d = sh ? (X + (1ll << (sh - 1))) >> sh : X;
-            X -= d << sh;
-            planes[((int64_t)p * B_pad + b) * nt_pad + j] = __float2bfloat16_rn((float)d);
-        }
+#pragma unroll
+        for (int p = 0; p < kPMax; ++p)
+            *reinterpret_cast<__nv_bfloat162 *>(planes + ((int64_t)p * B_pad + b) * nt_pad + j0) = d2[p];
     }
 }
 
@@ -532,42 +615,6 @@ __global__ void k_logl_reduce_x(const float2 *__restrict__ part, int n_mt, int B
     else if (csum_e) a -= csum_e[b];  // and a derived handle's parent's empty bins remain
     a += *kn;
     negLogL[b] = (a != 0.0) ? -a : INFINITY;
-}
-
-// Σ_{i: n_i > 0} (n_i - n_i log n_i) in FP64: each block a contiguous chunk (the log runs on
-// the FP64 pipe, so the work is spread over the SMs), the last block sums the block partials
-// in block order (fixed order, reproducible) and re-arms the ticket.
-constexpr int kDcBlocks = 64;
-__global__ void k_data_const(const double *__restrict__ n, int64_t nbins, double *__restrict__ part,
-                             unsigned int *ticket, double *__restrict__ kn) {
-    __shared__ double s[32];
-    __shared__ bool last;
-    const int64_t per = (nbins + gridDim.x - 1) / gridDim.x;
-    const int64_t i0 = (int64_t)blockIdx.x * per, i1 = min(nbins, i0 + per);
-    double a = 0.0;
-    for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const double v = n[i];
-        if (v > 0.0) a += v - v * log(v);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s[w];
-        part[blockIdx.x] = t;
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double t = 0.0;
-        for (int b = 0; b < (int)gridDim.x; ++b) t += ((volatile double *)part)[b];
-        *kn = t;
-        *ticket = 0u;
-    }
 }
 
 // Column sums Σ_i M_ij in FP64 (one block per template) and whether any value is negative.
@@ -694,15 +741,11 @@ int sfh_exact_launch(sfh_ctx *ctx, const sfh_models *m, const SfhExactPlan &xp, 
     }
     cudaStream_t st = ctx->stream;
     SFH_CK(ctx, cudaMemsetAsync(xp.nplanes, 0, 3 * sizeof(int), st));  // planes, flag, ticket
-    k_r_digits<<<(unsigned)xp.B_pad, 256, 0, st>>>(d_R, xp.B, m->nt, xp.B_pad, m->nt_pad, xp.Rd,
-                                                    xp.rscale, xp.nplanes, m->colsum, xp.csum,
-                                                    xp.nplanes + 1, m->colsum_e, xp.csum_e);
+    const DataConst dc{d_negLogL ? d_data : nullptr, m->nbins, xp.kpart, (unsigned int *)(xp.nplanes + 2), xp.kn};
+    k_r_digits<<<(unsigned)xp.B_pad + (dc.n ? kDcBlocks : 0), kDigitThreads, 0, st>>>(
+        d_R, xp.B, m->nt, xp.B_pad, m->nt_pad, xp.Rd, xp.rscale, xp.nplanes, m->colsum, xp.csum,
+        xp.nplanes + 1, m->colsum_e, xp.csum_e, dc);
     SFH_LAUNCHED(ctx);
-    if (d_negLogL) {
-        k_data_const<<<kDcBlocks, 256, 0, st>>>(d_data, m->nbins, xp.kpart,
-                                                (unsigned int *)(xp.nplanes + 2), xp.kn);
-        SFH_LAUNCHED(ctx);
-    }
     ExactParams P{};
     P.n_mt = xp.n_mt;
     P.n_vt = xp.n_vt;
