@@ -1,19 +1,20 @@
 // templates.cu -- template (Hess diagram) construction on sm_103a.
 //
-// k_stamps replaces bin_cmd_smooth (src/StarFormationHistories.jl:574-621) and
+// The stamp kernels replace bin_cmd_smooth (src/StarFormationHistories.jl:574-621) and
 // the two addstar! methods (:345-408) with their kernels
 // GaussianPSFAsymmetric / gaussian_int_general (:191-265) and
-// GaussianPSFCovariant / gaussian_psf_covariant (:272-340).  One CTA owns a
-// band of TY Hess rows of one template in shared memory (FP32).  Stars whose kernel is
-// wide against the bins (nearly all bin updates) are summed in registers, 8 x 8 bins per
-// lane, from 16 exponentials per tile and two FP32 operations per bin (wide_tile,
-// mid_tile); the rest are integrated bin by bin, a warp per star, and scattered into the
-// band with shared-memory atomics.  The band is flushed to HBM with coalesced stores.
+// GaussianPSFCovariant / gaussian_psf_covariant (:272-340).  A star takes one of three ways
+// (star_record): where its kernel is so smooth that 8 x 8 Chebyshev points stand for 40 x 16
+// bins (k_stamp_nodes); wide against the bins, 8 x 8 bins per lane in registers from 16
+// exponentials and two FP32 operations per bin (k_stamp_tiles, wide_tile and mid_tile, which
+// also interpolates the first and writes the template); the rest bin by bin, a warp per star,
+// added in global memory (k_stamp_narrow).
 // Window sizes, ties-to-even centroid rounding and the "both clipped lengths > 1" skip
 // follow the reference exactly.  The bound is FP32 issue: 5.6e10 (star, bin) updates for
-// 1,200 templates on 200 x 300 bins took 288 ms with nine exponentials and an atomic per
-// update, and 15.2 ms this way; 60 binary templates 10.3 -> 3.1 ms, 64 galaxies of 12
-// templates 180 -> 31 ms.
+// 1,200 templates on 200 x 300 bins took 288 ms with nine exponentials and a shared-memory atomic
+// per update, and 4.7 ms this way (tiles 2.5, nodes 0.8, star records 0.6, narrow stars 0.5); 300
+// separable templates 8.3 -> 0.71 ms, 60 binary ones 10.3 -> 0.89 ms, 64 galaxies of 12 templates
+// 180 -> 4.3 ms, 6 templates on 40 x 50 bins 475 -> 162 us.
 //
 // k_iso_stars replaces the single-star part of partial_cmd_smooth (:829-888):
 // mini_spacing resampling (:110-148, block-wide prefix scan over segments),
@@ -99,9 +100,8 @@ __device__ __forceinline__ float ex2f(float x) {
 // ---------------------------------------------------------------- star records
 // What the stamp loop needs of one star, in FP32: its clipped window and, by class, the
 // numbers of its kernel.  The FP64 work (pixel rounding, window sizes, variances) is done
-// once per star by one thread (k_star_prep, or the band kernel's staging when the caller
-// cannot size a record array); FP64 retires two operations per SM clock on this GPU, so
-// repeating it in every lane of every band's warp cost about a tenth of the build.
+// once per star by one thread (k_iso_stars, k_bin_points, k_star_prep; by next_stars when the
+// caller cannot size a record array): FP64 retires two operations per SM clock on this GPU.
 enum { kStarNone = 0, kStarWide = 1, kStarMid = 2, kStarNarrow = 3 };
 
 struct __align__(16) StarRec {
@@ -1716,13 +1716,14 @@ k_bin_prefac(IsoParams P, const double *__restrict__ m, const int64_t *__restric
 // fluxes of the two colour filters, of which one is the magnitude filter (:644, :700), and
 // IMF values.
 __global__ void k_bin_flux(IsoParams P, const double *__restrict__ m, const double *__restrict__ mags,
-                           int64_t total, double *__restrict__ fl, double *__restrict__ imfv) {
+                           int64_t total, double *__restrict__ fl, double *__restrict__ wv) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int fs[2] = {P.c1, P.c2};
 #pragma unroll
     for (int q = 0; q < 2; ++q) fl[q * total + i] = exp10(-0.4 * mags[(int64_t)fs[q] * total + i]);
-    imfv[i] = imf_pdf(P, m[i]);
+    // the interval's weight (of a template's last point: not used)
+    if (i + 1 < total) wv[i] = (m[i + 1] - m[i]) * (imf_pdf(P, m[i]) + imf_pdf(P, m[i + 1]));
 }
 
 // left-closed histogram bin of v (edges first + k step, step > 0), -1 outside: the product with
@@ -1760,40 +1761,84 @@ __device__ __forceinline__ double log_table(double x, const double2 *s_log) {
     return fma((double)e, 0.6931471805599453, t.y) + fma(r * r, p, r);
 }
 
+// -2.5 log10 x to 2e-9, as log2_fp32 (the same values out of range).
+__device__ __forceinline__ double mag_fp32(double x, const double2 *s_log, const float2 *s_mag) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)(b >> 52) - 1023, j = (int)(b >> 45) & 127;
+    if (e < -1000 || e > 1000) return -1.0857362047581296 * log_table(x, s_log);
+    const float c = __uint_as_float(0x3f800000u | (unsigned)j << 16);
+    const float r = __fdividef((float)(unsigned)(b >> 13), c) * 1.8189894035458565e-12f;  // 2^-39
+    const float2 t = s_mag[j];  // -2.5 log10 c_j as two floats
+    const float l = fmaf(r * r, fmaf(r, fmaf(r, -0.25f, 1.f / 3.f), -0.5f), r);
+    return fma((double)e, -0.7525749891599529, (double)t.x + (double)fmaf(l, -1.0857362f, t.y));
+}
+
+// hist_bin's axis, and how close to an edge a value known to 4e-9 can be binned with its position
+// rounded to FP32: nearer than tol bins it may belong to either side.
+struct BinAxis {
+    double first, step, inv;
+    int n;
+    float tol;
+    __device__ BinAxis(double f, double s, double i, int n_)
+        : first(f), step(s), inv(i), n(n_), tol(1e-6f + 2.4e-7f * (float)n_ + 8e-9f * (float)fabs(i)) {}
+    __device__ __forceinline__ int bin(double v, bool &near) const {
+        const float q = (float)((v - first) * inv), k = floorf(q);
+        if (!(q > -1.f && q < (float)n + 1.f)) return -1;
+        near |= !(q - k > tol && q - k < 1.f - tol);
+        return (q >= 0.f && q < (float)n) ? (int)k : -1;
+    }
+    __device__ __forceinline__ int exact(double v) const { return hist_bin(v, first, step, inv, n); }
+};
+
 // Grid: x -> left points i (a warp each), y -> template (chunk-relative); the lanes take the
-// pairs' right points j.  hist is [chunk][nx*ny].  FP64 throughput bounds it: with three library
-// log10 and two divisions a pair, 60 templates of 300 points took 946 us, now 480 us.
+// pairs' right points j.  hist is [chunk][nx*ny].  FP64 throughput bounds it: magnitudes take
+// their logarithm's series in FP32, and the pairs nearer to a bin's edge than that and an FP32
+// position can tell are binned from FP64 logarithms.  60 templates of 300 points: three library
+// log10 and two divisions a pair 946 us, FP64 tables and positions 500 us, this way 255 us.
 __global__ void __launch_bounds__(kPairThreads)
-k_bin_pairs(IsoParams P, const double *__restrict__ m, const double *__restrict__ fl,
-            const double *__restrict__ imfv, int64_t total, const int64_t *__restrict__ off,
-            const int32_t *__restrict__ len, const double *__restrict__ prefac, Grid2 g,
-            const sfh_df *__restrict__ tab, int t0, double *__restrict__ hist) {
+k_bin_pairs(IsoParams P, const double *__restrict__ fl, const double *__restrict__ wv, int64_t total,
+            const int64_t *__restrict__ off, const int32_t *__restrict__ len,
+            const double *__restrict__ prefac, Grid2 g, const sfh_df *__restrict__ tab, int t0,
+            double *__restrict__ hist) {
     __shared__ double2 s_log[128];
-    if (threadIdx.x < 128)
-        s_log[threadIdx.x] = make_double2(128.0 / (128.0 + (double)threadIdx.x),
-                                          (double)tab[threadIdx.x].h + (double)tab[threadIdx.x].l);
+    __shared__ float2 s_mag[128];
+    if (threadIdx.x < 128) {
+        const double lg = (double)tab[threadIdx.x].h + (double)tab[threadIdx.x].l;
+        s_log[threadIdx.x] = make_double2(128.0 / (128.0 + (double)threadIdx.x), lg);
+        const double mg = -1.0857362047581296 * lg;
+        s_mag[threadIdx.x] = make_float2((float)mg, (float)(mg - (double)(float)mg));
+    }
     __syncthreads();
     const int t = t0 + blockIdx.y, ns = len[t] - 1, lane = threadIdx.x & 31;
     const int64_t o = off[t];
-    const double *mt = m + o, *iv = imfv + o;
+    const double *wt = wv + o;
     const double *f1 = fl + o, *f2 = fl + total + o;
     double *h = hist + (int64_t)blockIdx.y * g.nx * g.ny;
     const double k = -1.0857362047581296, pre = prefac[t];  // flux2mag(f) = -2.5 log10 f (:656)
+    const BinAxis ax(g.xf, g.xs, g.ixs, g.nx), ay(g.yf, g.ys, g.iys, g.ny);
+    const double b1 = P.bias[P.c1], b2 = P.bias[P.c2], by = P.bias[P.y_index];
+    const bool y1 = P.y_index == P.c1;  // the magnitude is one of the colour's (:700)
+    const double cA = P.cA[P.c1] * P.cA[P.c2];
     for (int i = blockIdx.x * (kPairThreads / 32) + (threadIdx.x >> 5); i < ns;
          i += gridDim.x * (kPairThreads / 32)) {
-        const double fi1 = f1[i], fi2 = f2[i], wi = (mt[i + 1] - mt[i]) * (iv[i] + iv[i + 1]) * pre;
+        const double fi1 = f1[i], fi2 = f2[i], wi = wt[i] * pre;
         for (int j = i + 1 + lane; j < ns; j += 32) {
-            const double bm1 = k * log_table(fi1 + f1[j], s_log), bm2 = k * log_table(fi2 + f2[j], s_log);
-            double w = wi * ((mt[j + 1] - mt[j]) * (iv[j] + iv[j + 1]));
+            const double s1 = fi1 + f1[j], s2 = fi2 + f2[j];
+            const double m1 = mag_fp32(s1, s_log, s_mag), m2 = mag_fp32(s2, s_log, s_mag);
+            bool near = false;
+            int ix = ax.bin((m1 + b1) - (m2 + b2), near), iy = ay.bin((y1 ? m1 : m2) + by, near);
+            if (near) {
+                const double x1 = k * log_table(s1, s_log), x2 = k * log_table(s2, s_log);
+                ix = ax.exact((x1 + b1) - (x2 + b2));
+                iy = ay.exact((y1 ? x1 : x2) + by);
+            }
+            if (ix < 0 || iy < 0) continue;
+            double w = wi * wt[j];
             // the product of the two colour filters' completeness (compl_eval) over one division
-            const double e1 = (double)__expf((float)((bm1 - P.cm50[P.c1]) * P.crho_inv[P.c1]));
-            const double e2 = (double)__expf((float)((bm2 - P.cm50[P.c2]) * P.crho_inv[P.c2]));
-            w *= P.cA[P.c1] * P.cA[P.c2] * rcp_nr((1.0 + e1) * (1.0 + e2));
-            const double col = (bm1 + P.bias[P.c1]) - (bm2 + P.bias[P.c2]);
-            // the magnitude is one of the colour's (:700)
-            const double ym = (P.y_index == P.c1 ? bm1 : bm2) + P.bias[P.y_index];
-            const int ix = hist_bin(col, g.xf, g.xs, g.ixs, g.nx), iy = hist_bin(ym, g.yf, g.ys, g.iys, g.ny);
-            if (ix >= 0 && iy >= 0) atomicAdd(h + ix + (int64_t)g.nx * iy, w);
+            const double e1 = (double)__expf((float)((m1 - P.cm50[P.c1]) * P.crho_inv[P.c1]));
+            const double e2 = (double)__expf((float)((m2 - P.cm50[P.c2]) * P.crho_inv[P.c2]));
+            w *= cA * rcp_nr((1.0 + e1) * (1.0 + e2));
+            atomicAdd(h + ix + (int64_t)g.nx * iy, w);
         }
     }
 }
@@ -1940,7 +1985,7 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
         at += sfh_align256(bytes);
         return o;
     };
-    const size_t o_fl = carve(2 * total_points * 8), o_imf = carve(total_points * 8), o_pre = carve(ntempl * 8);
+    const size_t o_fl = carve(2 * total_points * 8), o_w = carve(total_points * 8), o_pre = carve(ntempl * 8);
     const size_t up = sfh_align256(256) + sfh_align256(chunk * 8) + sfh_align256(chunk * 4);
     const size_t o_up = carve(up + chunk * nseg * 4);  // narrow counter, starts, counts, firsts
     const size_t o_seg = carve(chunk * nseg * 4), o_hist = carve(chunk * nbins * 8);
@@ -1948,11 +1993,11 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
     char *b = (char *)ctx->scratch;
     const int64_t *d_off = (const int64_t *)(b + o_off);
     const int32_t *d_len = (const int32_t *)(b + o_len);
-    double *fl = (double *)(b + o_fl), *imfv = (double *)(b + o_imf), *prefac = (double *)(b + o_pre);
+    double *fl = (double *)(b + o_fl), *wv = (double *)(b + o_w), *prefac = (double *)(b + o_pre);
     double *hist = (double *)(b + o_hist);
     SFH_CK(ctx, cudaMemcpyAsync(b, head.data(), head.size(), cudaMemcpyHostToDevice, st));
     k_bin_flux<<<(unsigned)((total_points + 255) / 256), 256, 0, st>>>(P, d_m_ini, d_mags, total_points,
-                                                                    fl, imfv);
+                                                                    fl, wv);
     SFH_LAUNCHED(ctx);
     k_bin_prefac<<<(unsigned)ntempl, kPairThreads, 0, st>>>(P, d_m_ini, d_off, d_len,
                                                             (const double *)(b + o_norm), prefac);
@@ -1967,7 +2012,7 @@ extern "C" int sfh_binary_hess_batch_dev(sfh_ctx *ctx, const double *d_m_ini, co
         const int64_t nc = std::min(chunk, ntempl - t0);
         SFH_CK(ctx, cudaMemsetAsync(hist, 0, nc * nbins * 8, st));
         const dim3 grid((unsigned)((nmax - 1 + kPairThreads / 32 - 1) / (kPairThreads / 32)), (unsigned)nc);
-        k_bin_pairs<<<grid, kPairThreads, 0, st>>>(P, d_m_ini, fl, imfv, total_points, d_off, d_len,
+        k_bin_pairs<<<grid, kPairThreads, 0, st>>>(P, fl, wv, total_points, d_off, d_len,
                                                     prefac, g, ctx->d_df_tab, (int)t0, hist);
         SFH_LAUNCHED(ctx);
         k_bin_count<<<dim3((unsigned)nseg, (unsigned)nc), kPairThreads, 0, st>>>(hist, nbins,
