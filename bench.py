@@ -1231,10 +1231,10 @@ def run_ours(args):
             "templates_per_s": templates_per_s, "template_build_ms": build_ms,
             "template_bin_updates_per_s": bin_updates / (build_ms / 1e3),
             "template_build_roofline": {
-                "kernel": "k_stamps", "bound": "fp32 pipes (instruction issue)",
-                "frac": _profile_value("fma_pipe_fraction k_stamps"),
-                "issue_frac": _profile_value("issue_fraction k_stamps"),
-                "unit": "FMA pipe share of its peak (ncu, profiles/k_stamps_production.md)"},
+                "kernel": "k_stamp_tiles", "bound": "fp32 pipes (instruction issue)",
+                "frac": _profile_value("fma_pipe_fraction k_stamp_tiles"),
+                "issue_frac": _profile_value("issue_fraction k_stamp_tiles"),
+                "unit": "FMA pipe share of its peak (ncu, profiles/k_stamp_tiles_production.md)"},
             "template_bin_updates_per_build": bin_updates,
             "negLogL": neglogl, "precision": plain_check, "gpu_launches": launches,
             "roofline": roofline,

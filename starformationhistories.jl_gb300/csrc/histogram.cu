@@ -4,8 +4,9 @@
 // Bin k of an axis holds e[k] <= v < e[k+1] against the STORED edge values (StatsBase
 // searches the range's own elements; a Julia range such as 0.0:0.1:1.0 holds 0.3 exactly,
 // not 0 + 3 * 0.1).  A point on the last edge, below the first, or NaN is dropped.  A
-// point's bin is guessed from the mean step and corrected against the edge values; blocks accumulate a private FP64 histogram in shared memory when the grid
-// fits (dense photometric catalogues pile up in few bins) and flush it with global atomics.
+// point's bin is guessed from the mean step and corrected against the edge values; blocks
+// accumulate a private FP64 histogram in shared memory when the grid fits (dense photometric
+// catalogues pile up in few bins) and flush it with global atomics.
 #include <algorithm>
 #include <cmath>
 

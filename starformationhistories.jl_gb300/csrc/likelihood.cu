@@ -19,6 +19,8 @@
 // templates.
 // k_gemv_t walks template columns in the reverse of k_gemv_n's launch order so
 // the tail of M that k_gemv_n streamed last is still resident in L2.
+// FP64 storage whose 64-bin tiles fit one wave takes a single launch instead, in which every tile
+// stays in shared memory between the two passes (k_fg_tile_f64).
 #include <cuda_runtime.h>
 #include <float.h>
 

@@ -18,7 +18,8 @@
 // the warp by a recursive-halving transpose (31 shuffles for 32 templates), across the
 // CTA in shared memory and across tiles by a fixed-order per-galaxy finish.  M is then
 // read once per evaluation.  Fused galaxies are launched by register class (nt <= 8,
-// <= 16, <= 32), so a batch with a few wide galaxies does not widen every tile.
+// <= 16, <= 32), so a batch with a few wide galaxies does not widen every tile.  The rows come
+// through shared memory by cp.async, several ahead of the arithmetic (k_ragged_fused).
 #include <cuda_runtime.h>
 
 #include <algorithm>

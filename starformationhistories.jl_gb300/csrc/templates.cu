@@ -406,7 +406,7 @@ __device__ void star_asym(float *__restrict__ out, float *bx_buf, float *by_buf,
     const float invx = r.p[0], invy = r.p[1], dx0 = r.p[2], dy0 = r.p[3], a4 = r.p[4];
     // segments of W columns, each lane on its column: a product and an add per bin (a bin's row and
     // column from its number took two conversions, 16 a clock: 262 us for the narrow stars of
-    // 300 separable templates on 150 x 225 bins, 230 us this way in the same grid of blocks)
+    // 300 separable templates on 151 x 213 bins, 230 us this way in the same grid of blocks)
     const int W = (lx + (lx + 31) / 32 - 1) / ((lx + 31) / 32), rows_per = 32 / W;
     const int seg = lane / W, pos = lane - seg * W;
     for (int m = lane; m < lx; m += 32) bx_buf[m] = gauss_bin((dx0 + (float)m) * invx, invx);
