@@ -33,7 +33,9 @@
 
 namespace {
 
-constexpr int kNodeWarps = 8;     // warps of a k_stamp_nodes CTA
+// Warps of a k_stamp_nodes CTA, which wait for one another at its end.  2, 4, 8, us: 1,200 templates
+// 769, 759, 800; 768 of 64 galaxies 1,057, 854, 871; 60 binary ones 45, 28, 27.
+constexpr int kNodeWarps = 4;
 constexpr int kTileWarpsMax = 16;  // most warps of a k_stamp_tiles CTA
 constexpr int kNarrowWarps = 4;   // warps of a k_stamp_narrow CTA
 constexpr int kNarrowRows = 64;   // rows of a separable star's y table at a time
@@ -834,7 +836,7 @@ __device__ __forceinline__ void lagrange8(float x, float (&L)[8]) {
 // node: the tiles' 64 values each, rows of 8.  Most updates come from stars far below the
 // detection limit whose errors span the whole diagram (of 5.6e10 updates of the 1,200-template
 // build about seven eighths): on these tiles 64 values stand for 640 bins.
-__global__ void __launch_bounds__(kNodeWarps * 32, 2)
+__global__ void __launch_bounds__(kNodeWarps * 32, 16 / kNodeWarps)
 k_stamp_nodes(StampStars st, Grid2 g0, const Grid2 *__restrict__ grids,
               const int64_t *__restrict__ node_off, int t0, float *__restrict__ node) {
     __shared__ __align__(16) WarpStars W[kNodeWarps];
