@@ -12,9 +12,9 @@
 // Window sizes, ties-to-even centroid rounding and the "both clipped lengths > 1" skip
 // follow the reference exactly.  The bound is FP32 issue: 5.6e10 (star, bin) updates for
 // 1,200 templates on 200 x 300 bins took 288 ms with nine exponentials and a shared-memory atomic
-// per update, and 4.7 ms this way (tiles 2.5, nodes 0.8, star records 0.6, narrow stars 0.5); 300
-// separable templates 8.3 -> 0.71 ms, 60 binary ones 10.3 -> 0.89 ms, 64 galaxies of 12 templates
-// 180 -> 4.3 ms, 6 templates on 40 x 50 bins 475 -> 162 us.
+// per update, and 4.5 ms this way (tiles 2.4, nodes 0.8, star records 0.6, narrow stars 0.5); 300
+// separable templates 8.3 -> 0.70 ms, 60 binary ones 10.3 -> 0.89 ms, 64 galaxies of 12 templates
+// 180 -> 4.2 ms, 6 templates on 40 x 50 bins 475 -> 159 us.
 //
 // k_iso_stars replaces the single-star part of partial_cmd_smooth (:829-888):
 // mini_spacing resampling (:110-148, block-wide prefix scan over segments),
@@ -644,11 +644,14 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
     const float2 c1 = make_float2(c1f, c1f), c2 = make_float2(c2f, c2f);
     const unsigned cols = window_bits(r.xlo - col0, r.xhi - col0);
     const unsigned rows = window_bits(r.ylo - row0, r.yhi - row0);
-    float2 X0[4], Xm[4], Xp[4], hd[4];
+    float2 X0[4], Xm[4], Xp[4];
+    // u from one pair of columns to the next: its own registers per pair were spilled (k_stamp_tiles of
+    // 1,200 templates 2,540 us, 2,420 this way)
+    const float2 h0 = make_float2(-3.5f * hx, -2.5f * hx), h2 = make_float2(2.f * hx, 2.f * hx);
     const float hx2 = hx * hx, g0 = -2.f * hx * u, gd = -2.f * hx * dn;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        float x0[2], xm[2], xp[2], h2[2];
+        float x0[2], xm[2], xp[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const float d = tile_node(false, 2 * c + q), cx = hx2 * d * d;
@@ -656,12 +659,10 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
             xm[q] = ex2f(fmaf(g0 - gd, d, -cx));
             xp[q] = ex2f(fmaf(g0 + gd, d, -cx));
             if (!(cols >> (2 * c + q) & 1u)) x0[q] = xm[q] = xp[q] = 0.f;
-            h2[q] = hx * d;
         }
         X0[c] = make_float2(x0[0], x0[1]);
         Xm[c] = make_float2(xm[0], xm[1]);
         Xp[c] = make_float2(xp[0], xp[1]);
-        hd[c] = make_float2(h2[0], h2[1]);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -672,14 +673,15 @@ __device__ __forceinline__ void mid_tile(float2 (&acc)[8][4], const StarRec &r,
         const float ym = 0.625f * a * ex2f(-fmaf(um, um, vm * vm));
         const float yp = 0.625f * a * ex2f(-fmaf(up, up, vp * vp));
         const float2 y02 = make_float2(y0, y0), ym2 = make_float2(ym, ym), yp2 = make_float2(yp, yp);
-        const float2 uj2 = make_float2(uj, uj);
+        float2 uu = __fadd2_rn(make_float2(uj, uj), h0);
         const float4 t0 = *reinterpret_cast<const float4 *>(T + 8 * j);
         const float4 t1 = *reinterpret_cast<const float4 *>(T + 8 * j + 4);
         const float2 t[4] = {make_float2(t0.x, t0.y), make_float2(t0.z, t0.w),
                              make_float2(t1.x, t1.y), make_float2(t1.z, t1.w)};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const float2 uu = __fadd2_rn(uj2, hd[c]), s = __fmul2_rn(uu, uu);
+            const float2 s = __fmul2_rn(uu, uu);
+            uu = __fadd2_rn(uu, h2);
             const float2 R = __ffma2_rn(s, __ffma2_rn(s, c2, c1), c0);
             const float2 f = __ffma2_rn(Xp[c], yp2, __ffma2_rn(X0[c], y02, __fmul2_rn(Xm[c], ym2)));
             acc[j][c] = __ffma2_rn(__fmul2_rn(f, t[c]), R, acc[j][c]);
