@@ -213,8 +213,11 @@ k_ragged_pass2(const float *__restrict__ M, const GalDesc *__restrict__ gals,
 // shared memory, kept fused_depth(NT) rows ahead (each thread copies and reads only its own
 // elements, so no barrier; bins past the end and templates up to a multiple of four are
 // zeroed).  256 galaxies of 12 templates (431 MB): 210 us with the rows loaded as they were
-// needed, 181 us now (2.4 TB/s; the arithmetic of a bin, about 600 instructions, is the rest).
-__host__ __device__ constexpr int fused_depth(int NT) { return NT <= 16 ? kFuseRows : 2; }
+// needed, 176 us now (2.4 TB/s; the arithmetic of a bin, about 600 instructions, is the rest).
+// Four rows of more than 12 templates leave too little of the SM's memory as L1: calls of 197
+// galaxies of 8, 12, 16 templates 127, 151, 156 us without, 124, 142, 170 four rows ahead, -, 139,
+// 144 two ahead.
+__host__ __device__ constexpr int fused_depth(int NT) { return NT <= 8 ? kFuseRows : 2; }
 __host__ __device__ inline int64_t fused_pad(int64_t nt) { return (nt + 3) / 4 * 4; }
 size_t fused_smem(int NT, int64_t nt) {  // counts, then rows of M: [depth][pad][kRT]
     return (size_t)fused_depth(NT) * kRT * (8 + 4 * (size_t)fused_pad(nt));
