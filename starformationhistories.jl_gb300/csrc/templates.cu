@@ -1231,7 +1231,7 @@ constexpr int64_t kMaxColumns = 3123;
 // several times the mean, and one warp of it would be the tail.  Templates on grids of their own
 // have different numbers of stars too: four times that.  k_stamp_tiles with 1, 2, 4, 8, 16 warps,
 // us: 60 binary templates (1,800 groups) 1,500, -, 335, 292, 394; 300 separable (5,100) 173, 180,
-// 201, 295; 1,200 (36,000) 2,540 with one; 768 templates of 64 galaxies (12,360) 1,880, 1,500, 1,360.
+// 201, 295; 1,200 (36,000) 2,420 with one; 768 templates of 64 galaxies (12,360) 1,880, 1,500, 1,360.
 int tile_warps(int64_t groups, bool uneven, int sm_count) {
     const int64_t most = (uneven ? 384 : 96) * (int64_t)sm_count;
     int ns = 1;
