@@ -1564,9 +1564,10 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     const Grid2 g = make_grid(xf, xs, nx, yf, ys, ny);
     const size_t nodes = rg ? (size_t)rg->nodes * sizeof(float)
                             : nx <= kMaxColumns && ny <= (1 << 20) ? node_bytes(g, ntempl) : 0;
+    const size_t had = ctx->scratch_bytes;
     rc = sfh_scratch_reserve(ctx, o_work + StampWork::bytes(nstar_total, nodes));
     if (rc) return rc;
-    if (b != (char *)ctx->scratch) {  // a larger scratch: pass 1's results anew
+    if (ctx->scratch_bytes != had) {  // a new scratch, perhaps at the old address: pass 1's results anew
         b = (char *)ctx->scratch;
         if ((rc = pass1())) return rc;
     }
