@@ -47,8 +47,8 @@ struct Grid2 {
 };
 
 Grid2 make_grid(double xf, double xs, int64_t nx, double yf, double ys, int64_t ny) {
-    return Grid2{xf, xs, yf, ys, (int)std::min<int64_t>(nx, INT32_MAX), (int)std::min<int64_t>(ny, INT32_MAX),
-                 1.0 / xs, 1.0 / ys};
+    return Grid2{xf, xs, yf, ys, (int)std::clamp<int64_t>(nx, 0, INT32_MAX),
+                 (int)std::clamp<int64_t>(ny, 0, INT32_MAX), 1.0 / xs, 1.0 / ys};
 }
 
 // Signed erfc table entry: |value| = erfc(|t|), sign bit = sign of t.
@@ -1239,6 +1239,14 @@ int tile_warps(int64_t groups, bool uneven, int sm_count) {
     return ns;
 }
 
+int check_grid(sfh_ctx *ctx, int64_t nx, int64_t ny) {
+    if (nx < 1 || ny < 1 || nx > (1 << 20) || ny > (1 << 20))
+        return sfh_set_error(ctx, SFH_ERR_ARG, "stamp grid or template count out of range");
+    if (nx > kMaxColumns)
+        return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
+    return SFH_OK;
+}
+
 size_t tile_smem(int ns) { return (ns > 1 ? 16384 : 8192) + ns * sizeof(WarpStars); }
 
 // Bytes of the node values of ntempl templates on one grid.
@@ -1288,10 +1296,9 @@ struct StampGrids {
 int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const StampGrids *rg,
                   const StampWork &w, float *d_out) {
     const int64_t nx = rg ? rg->max_nx : g.nx;
-    if (!rg && (g.nx < 1 || g.ny < 1 || g.nx > (1 << 20) || g.ny > (1 << 20) || ntempl < 1 || ntempl > 65535))
+    if (!rg && (ntempl < 1 || ntempl > 65535))
         return sfh_set_error(ctx, SFH_ERR_ARG, "stamp grid or template count out of range");
-    if (nx > kMaxColumns)
-        return sfh_set_error(ctx, SFH_ERR_UNSUPPORTED, "Hess grid too wide for a shared-memory band");
+    if (int rc = rg ? SFH_OK : check_grid(ctx, nx, g.ny)) return rc;
     const bool have = w.rec != nullptr;
     st.rec = w.rec;
     st.key = w.key;
@@ -1546,6 +1553,7 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     int flag = 0;
     std::memcpy(&flag, back.data(), 4);
     if (flag == 2) return sfh_set_error(ctx, SFH_ERR_ARG, "isochrone masses must be strictly increasing");
+    if (!rg && (rc = check_grid(ctx, nx, ny))) return rc;  // (a ragged batch's grids were checked)
     const int64_t *nst = back.data() + (o_cnt64 - o_err) / 8;
     std::vector<int64_t> soff((size_t)ntempl + 1);
     std::vector<int32_t> count((size_t)ntempl);
@@ -1562,8 +1570,7 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     const size_t o_work = o_late + late_bytes;
     // Pass 2: star records, then the stamps.
     const Grid2 g = make_grid(xf, xs, nx, yf, ys, ny);
-    const size_t nodes = rg ? (size_t)rg->nodes * sizeof(float)
-                            : nx <= kMaxColumns && ny <= (1 << 20) ? node_bytes(g, ntempl) : 0;
+    const size_t nodes = rg ? (size_t)rg->nodes * sizeof(float) : node_bytes(g, ntempl);
     const size_t had = ctx->scratch_bytes;
     rc = sfh_scratch_reserve(ctx, o_work + StampWork::bytes(nstar_total, nodes));
     if (rc) return rc;
