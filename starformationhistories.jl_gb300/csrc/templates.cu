@@ -257,8 +257,10 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     r.jr = (float)(jrl - 1);
     if (wide || mid) {
         const double sy2 = sy * sy, Syy = wide ? fma(g.ys * (1.0 / 12.0), g.ys, sy2) : sy2;
-        const double ry = rsqrt_nr(Syy), m = wide ? -c * sy2 * (ry * ry) : -c;
-        const double vx = fma(sx, sx, fma(g.xs * (1.0 / 12.0), g.xs, wide ? (c * c + c * m) * sy2 : 0.0));
+        const double ry = rsqrt_nr(Syy), s2 = sy2 * (ry * ry), m = wide ? -c * s2 : -c;
+        // the y box's share c^2 sy^2 - (c sy^2)^2 / Syy as a product: the difference loses vx where sy >> sx
+        const double box = wide ? c * c * s2 * (g.ys * g.ys * (1.0 / 12.0)) : 0.0;
+        const double vx = fma(sx, sx, fma(g.xs * (1.0 / 12.0), g.xs, box));
         const double rx = rsqrt_nr(vx), qx = 0.8493218002880191 * rx, qy = 0.8493218002880191 * ry;  // g / √2
         const double wsh = -m * g.ys * qx;
         const float wxf = (float)(g.xs * qx), wshf = (float)wsh, wyf = (float)(g.ys * qy);

@@ -1,0 +1,26 @@
+"""Stars whose two errors differ by many orders of magnitude, against the FP64 oracle.
+
+Tolerance, that of the template tests: per bin 1e-5 |ref| + 1e-6 max(ref)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(sfh, O, x, y, sx, sy, cov, xe, ye):
+    x, y, sx, sy = (np.atleast_1d(np.asarray(v, dtype=float)) for v in np.broadcast_arrays(x, y, sx, sy))
+    w = np.linspace(0.5, 1.5, x.size)
+    H = sfh.bin_cmd_smooth(x, y, sx, sy, cov, weights=w, edges=(xe, ye)).weights
+    nx, ny = xe.size - 1, ye.size - 1
+    R = O.bin_cmd_smooth(x, y, sx, sy, w, cov, (xe[0], (xe[-1] - xe[0]) / nx, nx),
+                         (ye[0], (ye[-1] - ye[0]) / ny, ny))
+    assert np.isfinite(H).all() and np.abs(R).max() > 0
+    assert np.all(np.abs(H - R) <= 1e-5 * np.abs(R) + 1e-6 * np.abs(R).max())
+
+
+@pytest.mark.parametrize("cov", [1, -1])
+@pytest.mark.parametrize("sy", [1e2, 1e4, 1e5, 1e6])
+def test_wide_star_with_a_far_larger_y_error(sfh, O, cov, sy):
+    xe, ye = np.linspace(-0.6, 2.4, 201), np.linspace(19.0, 30.0, 301)
+    _check(sfh, O, [0.4, 0.9, 1.3], [24.0, 25.1, 27.3], [0.4, 0.5, 0.7], [sy, 1.3 * sy, 1.7 * sy],
+           cov, xe, ye)
