@@ -54,13 +54,13 @@ Grid2 make_grid(double xf, double xs, int64_t nx, double yf, double ys, int64_t 
 // Signed erfc table entry: |value| = erfc(|t|), sign bit = sign of t.
 __device__ __forceinline__ float erfc_signed(float t) { return copysignf(erfcf(fabsf(t)), t); }
 
-// erf(tb) - erf(ta) for ta <= tb from signed erfc entries, without cancellation
-// when both edges sit in the same tail.
+// erf(tb) - erf(ta) from signed erfc entries, without cancellation when both edges sit in the
+// same tail.
 __device__ __forceinline__ float erf_diff(float ea, float eb) {
     const float a = fabsf(ea), b = fabsf(eb);
-    if (!signbit(ea)) return a - b;  // 0 <= ta <= tb
-    if (signbit(eb)) return b - a;   // ta <= tb < 0
-    return (2.0f - a) - b;           // ta < 0 <= tb
+    if (signbit(ea) == signbit(eb)) return signbit(ea) ? b - a : a - b;
+    const float d = (2.0f - a) - b;      // ta < 0 <= tb
+    return signbit(ea) ? d : -d;         // tb < 0 <= ta: descending edges
 }
 
 // Gauss-Legendre 3-point weights, src/StarFormationHistories.jl:303-304.

@@ -1,4 +1,5 @@
-"""Stars whose two errors differ by many orders of magnitude, against the FP64 oracle.
+"""Stars whose two errors differ by many orders of magnitude and descending bin edges, against the
+FP64 oracle.
 
 Tolerance, that of the template tests: per bin 1e-5 |ref| + 1e-6 max(ref)."""
 import numpy as np
@@ -24,3 +25,20 @@ def test_wide_star_with_a_far_larger_y_error(sfh, O, cov, sy):
     xe, ye = np.linspace(-0.6, 2.4, 201), np.linspace(19.0, 30.0, 301)
     _check(sfh, O, [0.4, 0.9, 1.3], [24.0, 25.1, 27.3], [0.4, 0.5, 0.7], [sy, 1.3 * sy, 1.7 * sy],
            cov, xe, ye)
+
+
+@pytest.mark.parametrize("cov", [1, -1])
+@pytest.mark.parametrize("flip", [(True, False), (False, True), (True, True)])
+def test_descending_edges(sfh, O, cov, flip):
+    """A negative bin step of a covariant star: the window of three bins and the integrals of the
+    opposite sign that the reference's formulas give."""
+    rng = np.random.default_rng(3)
+    n, nx, ny = 40, 30, 25
+    xe, ye = np.linspace(-0.6, 2.4, nx + 1), np.linspace(19.0, 30.0, ny + 1)
+    xe, ye = xe[::-1].copy() if flip[0] else xe, ye[::-1].copy() if flip[1] else ye
+    x, y, w = rng.uniform(-0.5, 2.3, n), rng.uniform(19.5, 29.5, n), rng.random(n) + 0.1
+    sx, sy = rng.uniform(0.5, 1.5, n), rng.uniform(2.0, 6.0, n)
+    H = sfh.bin_cmd_smooth(x, y, sx, sy, cov, weights=w, edges=(xe, ye)).weights
+    R = O.bin_cmd_smooth(x, y, sx, sy, w, cov, (xe[0], (xe[-1] - xe[0]) / nx, nx),
+                         (ye[0], (ye[-1] - ye[0]) / ny, ny))
+    assert np.all(np.abs(H - R) <= 1e-5 * np.abs(R) + 1e-6 * np.abs(R).max())
