@@ -1122,7 +1122,7 @@ __device__ IsoPoint iso_point(const IsoParams &P, const double *m, const double 
 
 // Segment insertion counts (:128-137) and their exclusive scan: pos[k] is the number of the first
 // resampled point of segment k, pos[nseg] = N = 1 + sum(cnt) the number of points.  Flags masses
-// that are not strictly increasing.
+// that are not strictly increasing (2) and more points than an int counts (1).
 __global__ void __launch_bounds__(kIsoThreads)
 k_iso_count(const double *__restrict__ m_ini, const double *__restrict__ mags,
             const int64_t *__restrict__ iso_off, const int32_t *__restrict__ iso_len, IsoParams P,
@@ -1136,7 +1136,8 @@ k_iso_count(const double *__restrict__ m_ini, const double *__restrict__ mags,
     const double *vy = mg + (int64_t)P.y_index * P.total;
     int *pos = pos_all + pos_off[t];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int carry = 1, round = 0;
+    int64_t carry = 1;
+    int round = 0;
     for (int base = 0; base < nseg; base += kIsoThreads, round ^= 1) {
         const int k = base + (int)threadIdx.x;
         int v = 0;
@@ -1149,7 +1150,7 @@ k_iso_count(const double *__restrict__ m_ini, const double *__restrict__ mags,
                 const double r = ceil(d / dmag);
                 v = r < 1.0e7 ? (int)r : 10000000;
             }
-            if (!(m[k + 1] > m[k])) atomicExch(err_flag, 2);
+            if (!(m[k + 1] > m[k])) atomicMax(err_flag, 2);
         }
         int incl = v;
 #pragma unroll
@@ -1159,17 +1160,18 @@ k_iso_count(const double *__restrict__ m_ini, const double *__restrict__ mags,
         }
         if (lane == 31) s_warp[round][warp] = incl;
         __syncthreads();
-        int wpre = 0, tot = 0;
+        int64_t wpre = 0, tot = 0;
         for (int w = 0; w < kIsoThreads / 32; ++w) {
             if (w < warp) wpre += s_warp[round][w];
             tot += s_warp[round][w];
         }
-        if (k < nseg) pos[k] = carry + wpre + incl - v;
+        if (k < nseg) pos[k] = (int)(carry + wpre + incl - v);
         carry += tot;
     }
     if (threadIdx.x == 0) {
-        pos[max(nseg, 0)] = carry;
+        pos[max(nseg, 0)] = (int)carry;
         nstars_out[t] = carry - 1;
+        if (carry > INT_MAX) atomicMax(err_flag, 1);
     }
 }
 
@@ -1556,6 +1558,7 @@ int partial_run(sfh_ctx *ctx, const double *d_m_ini, const double *d_mags,
     std::memcpy(&flag, back.data(), 4);
     if (flag == 2) return sfh_set_error(ctx, SFH_ERR_ARG, "isochrone masses must be strictly increasing");
     if (!rg && (rc = check_grid(ctx, nx, ny))) return rc;  // (a ragged batch's grids were checked)
+    if (flag == 1) return sfh_set_error(ctx, SFH_ERR_NOMEM, "too many resampled points in an isochrone");
     const int64_t *nst = back.data() + (o_cnt64 - o_err) / 8;
     std::vector<int64_t> soff((size_t)ntempl + 1);
     std::vector<int32_t> count((size_t)ntempl);

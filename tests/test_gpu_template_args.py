@@ -39,3 +39,25 @@ def test_grids_out_of_range(sfh, nx, ny, name):
         1.1, ny, out.data_ptr()) == want
     ctx.synchronize()
     assert not out.cpu().numpy().any()
+
+
+@pytest.mark.parametrize("npts", [216, 300, 500])
+def test_more_resampled_points_than_an_int_counts(sfh, npts):
+    """Bins so fine that a template's resampled points pass 2^31 (and, wrapped, come out negative or
+    small again): refused, and the next call is served."""
+    import torch
+    from sfhgpu import _lib
+    from sfhgpu import synthetic as S
+    dev = torch.device("cuda", 0)
+    m, mags = S.isochrone(9.0, -1.0, npts)
+
+    def build(step):
+        xe, ye = 0.5 + step * np.arange(11), 25.0 + step * np.arange(11)
+        return sfh.partial_cmd_smooth_batch(
+            torch.tensor(np.concatenate([m, m]), device=dev),
+            torch.tensor(np.concatenate([mags, mags], axis=1), device=dev), [0, npts], [npts, npts],
+            1, (0, 1), S.error_models(), S.completeness_models(), S.imf(), 25.0, 1.0, (xe, ye))
+    with pytest.raises(_lib.SFHError) as e:
+        build(2.0**-40)
+    assert e.value.status == _lib.SFH_ERR_NOMEM
+    assert np.isfinite(build(0.25).cpu().numpy()).all()
