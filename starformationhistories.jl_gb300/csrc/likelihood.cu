@@ -869,14 +869,12 @@ int sfh_launch_fg(sfh_ctx *ctx, const sfh_models *m, const FgArgs &a, cudaEvent_
         const int grid = (int)((nbins + kTile64 - 1) / kTile64);
         int rc = sfh_scratch_reserve(ctx, (size_t)grid * (nt + 1) * sizeof(double));
         if (rc) return rc;
-        static thread_local bool attr_set = false;
-        if (!attr_set) {
+        const size_t smem = tile64_smem(nt);
+        if (smem > 48 * 1024)  // at every launch: the limit belongs to the device; the same for all threads
             SFH_CK(ctx, cudaFuncSetAttribute(k_fg_tile_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              213 * 1024));
-            attr_set = true;
-        }
         if (ev) SFH_CK(ctx, cudaEventRecord(ev[0], ctx->stream));
-        k_fg_tile_f64<<<grid, kThreads, tile64_smem(nt), ctx->stream>>>(
+        k_fg_tile_f64<<<grid, kThreads, smem, ctx->stream>>>(
             Tile64Args{(const double *)Mptr, nbins, (int)nt, a.coeffs, a.data, a.eps, a.composite, a.G,
                        a.negLogL, a.gsign, (double *)ctx->scratch, ctx->d_counters + SFH_CNT_LOGL});
         SFH_LAUNCHED(ctx);

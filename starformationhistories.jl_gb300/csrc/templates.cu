@@ -1309,16 +1309,6 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     const Smooth sm = smooth_tiling(g, have && !rg);
     const int node_groups = rg ? rg->max_node_groups : sm.on ? sm.groups() : 0;
     cudaStream_t s = ctx->stream;
-    static thread_local bool attr_set = false;
-    if (!attr_set) {
-        for (auto k : {k_stamp_tiles<true>, k_stamp_tiles<false>})
-            SFH_CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)tile_smem(kTileWarpsMax)));
-        for (auto k : {k_stamp_narrow<true>, k_stamp_narrow<false>})
-            SFH_CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(kNarrowWarps * (kMaxColumns + kNarrowRows) * 4)));
-        attr_set = true;
-    }
     if (have && !w.made) SFH_CK(ctx, cudaMemsetAsync(w.n_narrow, 0, sizeof(int), s));
     for (int64_t t0 = 0; have && t0 < ntempl; t0 += 65535) {
         const unsigned nt = (unsigned)std::min<int64_t>(65535, ntempl - t0);
@@ -1338,6 +1328,10 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     const int64_t groups = rg ? rg->ngroups : ntempl * tile_groups(g.nx, g.ny);
     const int ns = tile_warps(groups, rg != nullptr, ctx->sm_count);
     auto tiles = have ? k_stamp_tiles<true> : k_stamp_tiles<false>;
+    // (raised at every launch: a limit belongs to the device; always the most, for all threads)
+    if (tile_smem(ns) > 48 * 1024)
+        SFH_CK(ctx, cudaFuncSetAttribute(tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)tile_smem(kTileWarpsMax)));
     tiles<<<(unsigned)groups, 32 * ns, tile_smem(ns), s>>>(
         st, g, (int)ntempl, rg ? rg->groups : nullptr, rg ? rg->grids : nullptr, rg ? rg->out_off : nullptr,
         rg ? rg->node_off : nullptr, node_groups > 0 ? w.node : nullptr, d_out);
@@ -1350,7 +1344,11 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     const unsigned blocks = 56u * (unsigned)ctx->sm_count;
     const dim3 ngrid = have ? dim3(blocks) : dim3(std::max(1u, blocks / (unsigned)ntempl), (unsigned)ntempl);
     auto narrow = have ? k_stamp_narrow<true> : k_stamp_narrow<false>;
-    narrow<<<ngrid, kNarrowWarps * 32, kNarrowWarps * buf * sizeof(float), s>>>(
+    const size_t nsmem = kNarrowWarps * (size_t)buf * sizeof(float);
+    if (nsmem > 47 * 1024)  // (beside the records)
+        SFH_CK(ctx, cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kNarrowWarps * (kMaxColumns + kNarrowRows) * sizeof(float))));
+    narrow<<<ngrid, kNarrowWarps * 32, nsmem, s>>>(
         st, g, rg ? rg->grids : nullptr, rg ? rg->out_off : nullptr, w.narrow, w.n_narrow, buf, d_out);
     SFH_LAUNCHED(ctx);
     return SFH_OK;
