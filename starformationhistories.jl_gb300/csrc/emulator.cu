@@ -937,23 +937,23 @@ extern "C" int sfh_emu_reconstruct_groups(sfh_ctx *ctx, const float *d_coef,
         return SFH_ERR_ARG;
     SFH_CK(ctx, cudaSetDevice(ctx->device));
     size_t shm = (size_t)kRecRows * K * sizeof(float);
+    // raised limits are the most of all calls: a thread must not lower another's before its launch
+    constexpr size_t most = kRecRows * 1024 * sizeof(float), ring = kRecDepth * kRecThreads * sizeof(float4);
     // float4 rows need every basis, offset and output row on a 16-byte boundary
     const bool vec = nbins % 4 == 0 && ((uintptr_t)d_basis | (uintptr_t)d_offset |
                                         (uintptr_t)d_out) % 16 == 0;
     if (vec) {
-        shm += (size_t)kRecDepth * kRecThreads * sizeof(float4);
+        shm += ring;
         if (shm > 40 * 1024)
             SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups<4>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)shm));
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most + ring)));
         dim3 grid((unsigned)((nbins + 4 * kRecThreads - 1) / (4 * kRecThreads)), (unsigned)nseg);
         k_recon_groups<4><<<grid, kRecThreads, shm, ctx->stream>>>(
             d_coef, d_rows, d_seg, B, ngroups, d_basis, d_offset, K, nbins, mode, d_out);
     } else {
         if (shm > 40 * 1024)
             SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups<1>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)shm));
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         dim3 grid((unsigned)((nbins + kRecThreads - 1) / kRecThreads), (unsigned)nseg);
         k_recon_groups<1><<<grid, kRecThreads, shm, ctx->stream>>>(
             d_coef, d_rows, d_seg, B, ngroups, d_basis, d_offset, K, nbins, mode, d_out);
