@@ -310,7 +310,7 @@ __global__ void k_mlp_rows(const float *__restrict__ P, int64_t pstride, int64_t
 // layer's weights are read once per segment instead of once per row, in coalesced tiles.  A
 // thread owns an output and all rows of the segment; every row's sums run over k in order as in
 // k_mlp_rows, so the results are the same bits.  1,200 rows of 64 groups, 3 -> 256 -> 256 -> 64:
-// 335 us a row at a time (each lane walking a weight row of its own), 56 us this way.
+// 335 us a row at a time (each lane walking a weight row of its own), 48 us this way.
 constexpr int kMlpRows = 16;
 constexpr int kMlpTile = 32;       // weights of an output staged at a time
 constexpr int kMlpThreads = 256;
@@ -368,8 +368,11 @@ __device__ __forceinline__ void mlp_layer(const float *__restrict__ W, const flo
     __syncthreads();
 }
 
+// Blocks go to the groups by their rows: one each, and gridDim.x - ngroups more shared out in
+// proportion to the groups' runs of kMlpRows rows, so that a group that holds most of the rows is
+// worked on by most of the blocks.  Every block counts the groups' rows for itself.
 __global__ void __launch_bounds__(kMlpThreads)
-k_mlp_groups(const float *__restrict__ P, int64_t pstride, int64_t ngroups, MlpShape S,
+k_mlp_groups(const float *__restrict__ P, int64_t pstride, int ngroups, MlpShape S,
              const float *__restrict__ X, const int32_t *__restrict__ group, int64_t B,
              float *__restrict__ Y) {
     extern __shared__ __align__(16) float sm[];
@@ -377,11 +380,76 @@ k_mlp_groups(const float *__restrict__ P, int64_t pstride, int64_t ngroups, MlpS
           *a2 = a1 + S.h1 * kMlpRows;
     __shared__ int32_t s_row[kMlpRows];
     __shared__ int s_count[kMlpThreads / 32];
+    __shared__ int s_mine[3];  // the block's group, its number among the group's blocks, their number
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t g = blockIdx.x;
-    const float *p = P + g * pstride;
-    // The block's rows: of the group's rows in order, every gridDim.y-th run of kMlpRows.
-    int64_t at = 0;  // rows of the group before the 256 looked at
+    int *s_n = reinterpret_cast<int *>(s_w);  // rows of each group, until the weights come
+    for (int k = threadIdx.x; k < ngroups; k += kMlpThreads) s_n[k] = 0;
+    if (threadIdx.x == 0) s_mine[0] = -1;
+    __syncthreads();
+    const unsigned n = (unsigned)B;  // at most 2^31 - 1
+    for (unsigned i0 = threadIdx.x; i0 < n; i0 += 4 * kMlpThreads) {
+        int gi[4];  // four rows' loads together
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned i = i0 + u * kMlpThreads;
+            gi[u] = group && i < n ? __ldg(group + i) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned i = i0 + u * kMlpThreads;
+            if (i >= n) break;
+            if (gi[u] >= 0 && gi[u] < ngroups) atomicAdd(s_n + gi[u], 1);
+            else if (blockIdx.x == 0)  // invalid group: NaN row
+                for (int j = 0; j < S.out; ++j) Y[(int64_t)i * S.out + j] = __int_as_float(0x7fc00000);
+        }
+    }
+    __syncthreads();
+    const int per = (ngroups + kMlpThreads - 1) / kMlpThreads;
+    const int k0 = min(ngroups, (int)threadIdx.x * per), k1 = min(ngroups, k0 + per);
+    const auto runs_of = [&](int k) { return (int)(((unsigned)s_n[k] + kMlpRows - 1) / kMlpRows); };
+    int mine = 0, runs = 0;
+    for (int k = k0; k < k1; ++k) mine += runs_of(k);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if (lane == 0) s_count[warp] = mine;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kMlpThreads / 32; ++w) runs += s_count[w];
+    const auto blocks_of = [&](int k) {
+        const int n = runs_of(k);
+        return n ? (int)min((int64_t)n, 1 + (int64_t)n * ((int)gridDim.x - ngroups) / runs) : 0;
+    };
+    int blocks = 0;
+    for (int k = k0; k < k1; ++k) blocks += blocks_of(k);
+    int first = blocks;  // inclusive, then exclusive scan over the threads
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, first, o);
+        if (lane >= o) first += v;
+    }
+    __syncthreads();  // s_count has been read
+    if (lane == 31) s_count[warp] = first;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kMlpThreads / 32; ++w) first += w < warp ? s_count[w] : 0;
+    first -= blocks;
+    if ((int)blockIdx.x >= first && (int)blockIdx.x < first + blocks)
+        for (int k = k0, at = first; k < k1; ++k) {
+            const int n = blocks_of(k);
+            if ((int)blockIdx.x < at + n) {
+                s_mine[0] = k;
+                s_mine[1] = (int)blockIdx.x - at;
+                s_mine[2] = n;
+                break;
+            }
+            at += n;
+        }
+    __syncthreads();
+    const int g = s_mine[0], part = s_mine[1], parts = s_mine[2];
+    if (g < 0) return;
+    const float *p = P + (int64_t)g * pstride;
+    // The block's rows: of the group's rows in order, every `parts`-th run of kMlpRows.
+    int at = 0;      // rows of the group before the 256 looked at
     int have = 0;    // rows gathered for the segment
     const auto segment = [&](int cnt) {
         for (int t = threadIdx.x; t < S.in * kMlpRows; t += kMlpThreads) {
@@ -393,11 +461,12 @@ k_mlp_groups(const float *__restrict__ P, int64_t pstride, int64_t ngroups, MlpS
         mlp_layer<true>(p + S.oW2, p + S.ob2, a1, a2, s_w, S.h1, S.h2, s_row, cnt, nullptr);
         mlp_layer<false>(p + S.oW3, p + S.ob3, a2, nullptr, s_w, S.h2, S.out, s_row, cnt, Y);
     };
-    for (int64_t i0 = 0; i0 < B; i0 += kMlpThreads) {
-        const int64_t i = i0 + threadIdx.x;
-        const int64_t gi = i < B ? (group ? (int64_t)group[i] : 0) : ngroups;
-        if (g == 0 && blockIdx.y == 0 && i < B && (gi < 0 || gi >= ngroups))  // invalid group: NaN row
-            for (int j = 0; j < S.out; ++j) Y[i * S.out + j] = __int_as_float(0x7fc00000);
+    const auto row_group = [&](unsigned i) { return i < n ? (group ? __ldg(group + i) : 0) : -1; };
+    int ahead = row_group(threadIdx.x);
+    for (unsigned i0 = 0; i0 < n; i0 += kMlpThreads) {
+        const unsigned i = i0 + threadIdx.x;
+        const int gi = ahead;
+        ahead = row_group(i + kMlpThreads);
         const unsigned hit = __ballot_sync(0xffffffffu, gi == g);
         if (lane == 0) s_count[warp] = __popc(hit);
         __syncthreads();
@@ -407,14 +476,13 @@ k_mlp_groups(const float *__restrict__ P, int64_t pstride, int64_t ngroups, MlpS
             if (w < warp) before += s_count[w];
             all += s_count[w];
         }
-        const int64_t rank = at + before + __popc(hit & ((1u << lane) - 1u));
+        const int rank = at + before + __popc(hit & ((1u << lane) - 1u));
         // the runs that end or begin among these rows, in order
-        for (int64_t run = at / kMlpRows; run * kMlpRows < at + all; ++run) {
-            if (run % gridDim.y != blockIdx.y) continue;
-            const int64_t r = rank - run * kMlpRows;
+        for (int run = at / kMlpRows; run * kMlpRows < at + all; ++run) {
+            if (run % parts != part) continue;
+            const int r = rank - run * kMlpRows;
             if (gi == g && r >= 0 && r < kMlpRows) s_row[r] = (int32_t)i;
-            const int64_t upto = at + all - run * kMlpRows;
-            have = upto < kMlpRows ? (int)upto : kMlpRows;
+            have = min(kMlpRows, at + all - run * kMlpRows);
             __syncthreads();
             if (have == kMlpRows) {
                 segment(kMlpRows);
@@ -801,18 +869,23 @@ extern "C" int sfh_mlp_forward_rows(sfh_ctx *ctx, int in, int h1, int h2, int ou
     const MlpShape S = mlp_shape(in, h1, h2, out);
     // Rows of a group share its weights where a group has two of them on average and the
     // activations fit shared memory.  Networks of fewer than 24 K weights finish sooner a row
-    // per block while the blocks fit a few waves, both being latency.  us a row per block / in
-    // groups, hidden layers of 256: 1 group x 16 rows 49 / 47, 64 x 2 49 / 37, 64 x 64 1,200 /
-    // 72, 512 x 4 581 / 117; of 64: 64 x 8 16.6 / 14.7, 512 x 2 22.7 / 31.8, 512 x 3 45 / 35;
-    // of 1,024: 1 x 2 660 / 342, 64 x 16 4,590 / 405.
+    // per block while the blocks fit a few waves, both being latency.  A block of the grouped form
+    // looks at all rows' groups twice, which costs more than a row's network of S.n weights from
+    // S.n / 6 groups on.  us a row per block / in groups, hidden layers of 256: 1 group x 16 rows
+    // 50 / 44, 64 x 2 50 / 40, 64 x 64 1,210 / 68, 512 x 4 583 / 124, 8,000 x 2 4,360 / 2,410; of
+    // 64: 64 x 19 38 / 21, 512 x 3 64 / 38, 2,000 x 2 130 / 143, 8,000 x 2 466 / 1,390; of 96:
+    // 2,000 x 2 239 / 179, 8,000 x 2 840 / 1,520; of 1,024: 1 x 2 575 / 337, 64 x 19 4,480 / 372.
+    // Uneven groups, calls of 10,000 rows in 64 groups, hidden layers of 256: spread evenly 192, all
+    // in one group 344 (3,180 when every group had as many blocks as the mean needs; 2,810 a row
+    // per block).
     const size_t grp_smem = (size_t)(kMlpThreads * (kMlpTile + 1) + kMlpRows * (in + h1 + h2)) * sizeof(float);
-    if (B >= 2 * ngroups && (S.n >= 24 * 1024 || B >= 8 * (int64_t)ctx->sm_count) && grp_smem <= 200 * 1024) {
-        // as many blocks to a group as it has runs of rows, up to four blocks per SM altogether
-        const int64_t runs = (B / ngroups + kMlpRows - 1) / kMlpRows + 1;
-        const int64_t ny = std::min(runs, std::max<int64_t>(1, 4 * ctx->sm_count / ngroups));
+    if (B >= 2 * ngroups && (S.n >= 24 * 1024 || B >= 8 * (int64_t)ctx->sm_count) &&
+        ngroups <= kMlpThreads * (kMlpTile + 1) && 6 * ngroups <= S.n && grp_smem <= 200 * 1024) {
+        // a block per group and up to four per SM more, as many as there can be runs of rows
+        const int64_t blocks = ngroups + std::min<int64_t>(4 * ctx->sm_count, B / kMlpRows + ngroups);
         SFH_CK(ctx, cudaFuncSetAttribute(k_mlp_groups, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        k_mlp_groups<<<dim3((unsigned)ngroups, (unsigned)ny), kMlpThreads, grp_smem, ctx->stream>>>(
-            d_params, S.n, ngroups, S, d_X, d_group, B, d_Y);
+        k_mlp_groups<<<(unsigned)blocks, kMlpThreads, grp_smem, ctx->stream>>>(
+            d_params, S.n, (int)ngroups, S, d_X, d_group, B, d_Y);
         SFH_LAUNCHED(ctx);
         return SFH_OK;
     }
