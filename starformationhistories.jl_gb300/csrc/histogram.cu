@@ -40,22 +40,34 @@ struct HistAxis {
     int n;
 };
 
-// One axis as a thread needs it: the first and last edges' keys and the mean inverse step.
+// One axis as a thread needs it: the first and last edges' keys and the mean inverse step.  far: the
+// axis lies so far from zero that values in FP32 are several bins off (a time axis at 2.4e6 in steps of
+// 1e-2); the difference to the first edge is then taken in FP64.  2e6 points, guesses from FP32 values /
+// FP64 differences, us: 300 bins of 1 / 300 at 1e5 (3 bins off at most) 53 / 57, 300 bins of 0.01 at 2.45e6
+// (24) 85 / 57, 4,000 bins of 5e-5 there (thousands) 6,190 / 57; near zero 50 / 57.
 struct AxisGuess {
     long long first, last;
-    float e0, inv;
+    double e0;
+    float e0f, inv;
+    bool far;
 };
 __device__ __forceinline__ AxisGuess axis_guess(const HistAxis &a) {
     const double e0 = a.e[0], e1 = a.e[a.n];
-    return AxisGuess{order_key(e0), order_key(e1), (float)e0, (float)((double)a.n / (e1 - e0))};
+    const float e0f = (float)e0, inv = (float)((double)a.n / (e1 - e0));
+    // (2^-22: a truncated value, the rounded edge and their difference; in FP32, since every thread
+    // decides this)
+    const float most = fmaxf(fabsf(e0f), fabsf((float)e1));
+    return AxisGuess{order_key(e0), order_key(e1), e0, e0f, inv, !(most * 2.3841858e-7f * inv <= 8.f)};
 }
 
 // The bin of v, e[k] <= v < e[k + 1], or -1: the guess from the mean step, then a walk along
-// the edges (one step at most on evenly spaced ones).
+// the edges (a few steps at most on evenly spaced ones).  FAR: the guess from the FP64 difference.
+template <bool FAR>
 __device__ __forceinline__ int edge_bin(double v, const HistAxis &a, const AxisGuess &g) {
     const long long key = order_key(v);
     if (key < g.first || key >= g.last) return -1;
-    int k = (int)fminf(fmaxf((guess_float(v) - g.e0) * g.inv, 0.f), (float)(a.n - 1));
+    const float d = FAR ? (float)(v - g.e0) : guess_float(v) - g.e0f;
+    int k = (int)fminf(fmaxf(d * g.inv, 0.f), (float)(a.n - 1));
     k = min(k, a.n - 1);
     while (k > 0 && key < order_key(__ldg(a.e + k))) --k;
     while (k < a.n - 1 && key >= order_key(__ldg(a.e + k + 1))) ++k;
@@ -66,20 +78,11 @@ struct HistAxes {
     HistAxis x, y;
 };
 
-// SHARED: a block's own FP64 histogram in shared memory, added to `out` at the end; else every
-// point goes to `out` in L2.
-template <bool SHARED>
-__global__ void __launch_bounds__(kHistThreads)
-k_bin_cmd(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ w,
-          int64_t n, HistAxes A, double *__restrict__ out) {
-    extern __shared__ double s_hist[];
-    const AxisGuess gx = axis_guess(A.x), gy = axis_guess(A.y);
-    double *to = SHARED ? s_hist : out;
-    const int nb = A.x.n * A.y.n;
-    if (SHARED) {
-        for (int k = threadIdx.x; k < nb; k += blockDim.x) s_hist[k] = 0.0;
-        __syncthreads();
-    }
+// The thread's points, added to `to`.
+template <bool FAR>
+__device__ __forceinline__ void bin_points(const double *__restrict__ x, const double *__restrict__ y,
+                                           const double *__restrict__ w, int64_t n, const HistAxes &A,
+                                           const AxisGuess &gx, const AxisGuess &gy, double *to) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
         double vx[4], vy[4], vw[4];  // four points' loads in flight
@@ -93,13 +96,33 @@ k_bin_cmd(const double *__restrict__ x, const double *__restrict__ y, const doub
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int ix = edge_bin(vx[u], A.x, gx);
+            const int ix = edge_bin<FAR>(vx[u], A.x, gx);
             if (ix < 0) continue;
-            const int iy = edge_bin(vy[u], A.y, gy);
+            const int iy = edge_bin<FAR>(vy[u], A.y, gy);
             if (iy < 0) continue;
             atomicAdd(to + ix + (int64_t)A.x.n * iy, vw[u]);
         }
     }
+}
+
+// SHARED: a block's own FP64 histogram in shared memory, added to `out` at the end; else every
+// point goes to `out` in L2.
+template <bool SHARED>
+__global__ void __launch_bounds__(kHistThreads, SHARED ? 4 : 6)
+k_bin_cmd(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ w,
+          int64_t n, HistAxes A, double *__restrict__ out) {
+    extern __shared__ double s_hist[];
+    const AxisGuess gx = axis_guess(A.x), gy = axis_guess(A.y);
+    double *to = SHARED ? s_hist : out;
+    const int nb = A.x.n * A.y.n;
+    if (SHARED) {
+        for (int k = threadIdx.x; k < nb; k += blockDim.x) s_hist[k] = 0.0;
+        __syncthreads();
+    }
+    // (two loops: a choice per point made every point pay for both guesses, 80 us instead of 50 for
+    // 2e6 points)
+    if (gx.far || gy.far) bin_points<true>(x, y, w, n, A, gx, gy, to);
+    else bin_points<false>(x, y, w, n, A, gx, gy, to);
     if (SHARED) {
         __syncthreads();
         for (int k = threadIdx.x; k < nb; k += blockDim.x)
