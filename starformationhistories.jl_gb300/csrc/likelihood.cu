@@ -348,11 +348,29 @@ constexpr int kTile64 = 64, kPad64 = kTile64 + 1;  // padded: templates fall on 
 
 size_t tile64_smem(int64_t nt) { return ((size_t)nt * (kPad64 + 1) + 6 * kTile64) * sizeof(double); }
 
-// Two CTAs of 256 threads fit an SM up to 106 KB each, one up to 213 KB.
+// Where one launch is the faster form.  Its cost grows with the FP64 operations of the busiest SM
+// (templates x its tiles) and with the last CTA's sums, a chain of loads over all CTAs' shares that
+// 256 / (nt + 1) threads divide among themselves: one thread an entry from 128 templates on, one
+// thread two entries from 256 on.  us four kernels / one launch, host-array calls (in brackets calls
+// queued one behind another on the device):
+//   templates    38 tiles       76            152           228 (225)     304
+//      20        55 / 35        55 / 36       57 / 37       55 / 40       59 / 40 (31 / 15)
+//     100        57 / 39        58 / 43       60 / 47       62 / 59       59 / 60 (35 / 33)
+//     120        59 / 40        60 / 43       60 / 49       64 / 60       60 / 63 (35 / 35)
+//     128        59 / 43        60 / 46       60 / 56       62 / 68       66 / 78
+//     199        58 / 45        60 / 50       63 / 62       69 / 78       77 / 91
+//     255        61 / 47        62 / 52       68 / 66 (42 / 35)
+//     256        60 / 51        63 / 58       69 / 76
+//     300        60 / 57        62 / 66       69 / 85
+//     400        62 / 60 (35 / 34)  65 / 69 (37 / 42)  71 / 88
+// So up to 127 templates the tiles of two CTAs per SM, as long as templates x tiles stay within 192
+// per SM; up to 255 one CTA per SM; beyond that templates x tiles within 100 per SM.  Two CTAs of 256
+// threads fit an SM up to 106 KB each (198 templates), one up to 213 KB (407).
 bool tile64_fits(const sfh_ctx *ctx, int64_t nbins, int64_t nt) {
-    const size_t smem = tile64_smem(nt);
-    const int per_sm = smem <= 106 * 1024 ? 2 : smem <= 213 * 1024 ? 1 : 0;
-    return (nbins + kTile64 - 1) / kTile64 <= (int64_t)per_sm * ctx->sm_count;
+    const int64_t tiles = (nbins + kTile64 - 1) / kTile64, sms = ctx->sm_count;
+    if (nt < 128) return tiles <= 2 * sms && nt * tiles <= 192 * sms;
+    if (nt < 256) return tiles <= sms;
+    return tile64_smem(nt) <= 213 * 1024 && tiles <= sms && nt * tiles <= 100 * sms;
 }
 
 struct Tile64Args {
