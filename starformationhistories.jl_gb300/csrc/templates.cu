@@ -361,10 +361,10 @@ __device__ __forceinline__ unsigned long long smooth_strips(const StarRec &r, co
 // Completes a star's record with its smooth strips, stores it and its key, and lists it when it is narrow:
 // the narrow stars of all templates are in one list (one atomic per warp).
 __device__ __forceinline__ void store_record(StarRec &r, const Grid2 &g, StarId id, StarRec *to, StarKey *key,
-                                             StarId *narrow, int *n_narrow) {
+                                             StarId *narrow, int *n_narrow, bool smooth = true) {
     unsigned long long m = 0ull;
     if (r.cls == kStarWide) {
-        const Smooth sm = smooth_tiling(g, true);
+        const Smooth sm = smooth_tiling(g, smooth);
         m = sm.on ? smooth_strips(r, g, sm) : 0ull;
         r.p[10] = __uint_as_float((unsigned int)m);
         r.p[11] = __uint_as_float((unsigned int)(m >> 32));
@@ -388,7 +388,7 @@ k_star_prep(const double *__restrict__ xs, const double *__restrict__ ys,
             const double *__restrict__ sxs, const double *__restrict__ sys,
             const double *__restrict__ ws, const int64_t *__restrict__ start,
             const int32_t *__restrict__ count, const int32_t *__restrict__ covs, Grid2 g0,
-            const Grid2 *__restrict__ grids, int t0, StarRec *__restrict__ rec,
+            const Grid2 *__restrict__ grids, int t0, bool smooth, StarRec *__restrict__ rec,
             StarKey *__restrict__ key, StarId *__restrict__ narrow, int *__restrict__ n_narrow) {
     const int t = t0 + blockIdx.y;
     const int q = blockIdx.x * kPrepThreads + threadIdx.x;
@@ -397,7 +397,7 @@ k_star_prep(const double *__restrict__ xs, const double *__restrict__ ys,
     StarRec r{};
     const Grid2 g = grids ? grids[t] : g0;
     star_record(r, g, xs[s], ys[s], sxs[s], sys[s], ws[s], covs[t]);
-    store_record(r, g, StarId{t, q}, rec + s, key + s, narrow, n_narrow);
+    store_record(r, g, StarId{t, q}, rec + s, key + s, narrow, n_narrow, smooth);
 }
 
 // ---------------------------------------------------------------- narrow stars
@@ -1236,10 +1236,13 @@ constexpr int64_t kMaxColumns = 3123;
 // have different numbers of stars too: four times that.  k_stamp_tiles with 1, 2, 4, 8, 16 warps,
 // us: 60 binary templates (1,800 groups) 1,500, -, 335, 292, 394; 300 separable (5,100) 173, 180,
 // 201, 295; 1,200 (36,000) 2,420 with one; 768 templates of 64 galaxies (12,360) 1,880, 1,500, 1,360.
-int tile_warps(int64_t groups, bool uneven, int sm_count) {
+// No more than a template has stars (the warps' sums are added one after the other), as the narrow
+// stars' blocks are no more than there can be stars for: one star on 200 x 300 bins 120 us a call without these
+// two limits, 116 with.
+int tile_warps(int64_t groups, bool uneven, int64_t maxcount, int sm_count) {
     const int64_t most = (uneven ? 384 : 96) * (int64_t)sm_count;
     int ns = 1;
-    while (ns < kTileWarpsMax && groups * 2 * ns <= most) ns *= 2;
+    while (ns < kTileWarpsMax && ns < maxcount && groups * 2 * ns <= most) ns *= 2;
     return ns;
 }
 
@@ -1266,15 +1269,16 @@ struct StampWork {
     StarId *narrow = nullptr;  // room for every star
     int *n_narrow = nullptr;
     float *node = nullptr;     // node_bytes() / the ragged batch's nodes
-    int64_t maxcount = 0;      // largest star count of a template
+    int64_t stars = 0, maxcount = 0;  // of all templates, of the one with the most
     bool made = false;         // the records are there already (k_iso_stars)
+    bool smooth = true;        // Chebyshev tiles are used (made records always expect them)
     static size_t bytes(int64_t stars, size_t node) {
         const size_t n = (size_t)std::max<int64_t>(stars, 1);
         return 256 + sfh_align256(n * sizeof(StarRec)) + sfh_align256(n * sizeof(StarKey)) +
                sfh_align256(n * sizeof(StarId)) + sfh_align256(node);
     }
     StampWork() = default;
-    StampWork(char *b, int64_t stars, int64_t maxcount_) : maxcount(maxcount_) {
+    StampWork(char *b, int64_t stars_, int64_t maxcount_) : stars(stars_), maxcount(maxcount_) {
         const size_t n = (size_t)std::max<int64_t>(stars, 1);
         n_narrow = (int *)b;
         rec = (StarRec *)(b += 256);
@@ -1283,6 +1287,12 @@ struct StampWork {
         node = (float *)(b + sfh_align256(n * sizeof(StarId)));
     }
 };
+
+// bin_cmd_smooth of fewer stars does without the Chebyshev tiles: a launch and the interpolation cost
+// more than they save.  200 x 300 bins, 1, 10, 30 separable stars of 0.2 bins' error, call in us: 116,
+// 116, 118 with, 100, 109, 110 without (a block per band of rows, as once, 108, 116, 121); covariant
+// stars of 30 bins' error 116, 118, 121 with, 100, 106, 115 without.
+constexpr int kSmoothStars = 64;
 
 // Per-template grids of a ragged batch on the device.
 struct StampGrids {
@@ -1306,7 +1316,7 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     const bool have = w.rec != nullptr;
     st.rec = w.rec;
     st.key = w.key;
-    const Smooth sm = smooth_tiling(g, have && !rg);
+    const Smooth sm = smooth_tiling(g, have && !rg && w.smooth);
     const int node_groups = rg ? rg->max_node_groups : sm.on ? sm.groups() : 0;
     cudaStream_t s = ctx->stream;
     if (have && !w.made) SFH_CK(ctx, cudaMemsetAsync(w.n_narrow, 0, sizeof(int), s));
@@ -1315,8 +1325,8 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
         if (w.maxcount > 0 && !w.made) {
             k_star_prep<<<dim3((unsigned)((w.maxcount + kPrepThreads - 1) / kPrepThreads), nt),
                           kPrepThreads, 0, s>>>(st.x, st.y, st.sx, st.sy, st.w, st.start, st.count,
-                                                st.cov, g, rg ? rg->grids : nullptr, (int)t0, w.rec,
-                                                w.key, w.narrow, w.n_narrow);
+                                                st.cov, g, rg ? rg->grids : nullptr, (int)t0, w.smooth,
+                                                w.rec, w.key, w.narrow, w.n_narrow);
             SFH_LAUNCHED(ctx);
         }
         if (node_groups > 0) {
@@ -1326,7 +1336,7 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
         }
     }
     const int64_t groups = rg ? rg->ngroups : ntempl * tile_groups(g.nx, g.ny);
-    const int ns = tile_warps(groups, rg != nullptr, ctx->sm_count);
+    const int ns = tile_warps(groups, rg != nullptr, have ? w.maxcount : INT_MAX, ctx->sm_count);
     auto tiles = have ? k_stamp_tiles<true> : k_stamp_tiles<false>;
     // (raised at every launch: a limit belongs to the device; always the most, for all threads)
     if (tile_smem(ns) > 48 * 1024)
@@ -1342,7 +1352,8 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     // eighth alone in a second wave), 610 with 7, 529 with 56, 515 with 112; 300 separable ones 230,
     // 202, 164, 162; 6 small ones 13 with any.
     const unsigned blocks = 56u * (unsigned)ctx->sm_count;
-    const dim3 ngrid = have ? dim3(blocks) : dim3(std::max(1u, blocks / (unsigned)ntempl), (unsigned)ntempl);
+    const dim3 ngrid = have ? dim3((unsigned)std::clamp<int64_t>((w.stars + kNarrowWarps - 1) / kNarrowWarps, 1, blocks))
+                            : dim3(std::max(1u, blocks / (unsigned)ntempl), (unsigned)ntempl);
     auto narrow = have ? k_stamp_narrow<true> : k_stamp_narrow<false>;
     const size_t nsmem = kNarrowWarps * (size_t)buf * sizeof(float);
     if (nsmem > 47 * 1024)  // (beside the records)
@@ -1409,12 +1420,14 @@ extern "C" int sfh_bin_cmd_smooth(sfh_ctx *ctx, const double *x, const double *y
     struct { int64_t start; int32_t count; int32_t cov; } meta{0, (int32_t)npts, cov_mult};
     SFH_CK(ctx, cudaMemcpyAsync(b + o_meta, &meta, sizeof(meta), cudaMemcpyHostToDevice, ctx->stream));
     float *d_out = (float *)(b + o_out);
+    StampWork work(b + o_work, npts, npts);
+    work.smooth = npts >= kSmoothStars;
     rc = launch_stamps(ctx, StampStars{(const double *)b, (const double *)(b + a5),
                                        (const double *)(b + 2 * a5), (const double *)(b + 3 * a5),
                                        (const double *)(b + 4 * a5), nullptr,
                                        (const int64_t *)(b + o_meta), (const int32_t *)(b + o_meta + 8),
                                        (const int32_t *)(b + o_meta + 12)},
-                       1, g, nullptr, StampWork(b + o_work, npts, npts), d_out);
+                       1, g, nullptr, work, d_out);
     if (rc) return rc;
     std::vector<float> tmp((size_t)nbins);
     SFH_CK(ctx, cudaMemcpyAsync(tmp.data(), d_out, nbins * 4, cudaMemcpyDeviceToHost, ctx->stream));
