@@ -734,7 +734,8 @@ __device__ __forceinline__ int next_stars(StarRec *slot, StarKey &key, const Sta
         r = st.rec + s0 + q;
     } else {
         key = StarKey{INT_MAX, -1, 0ull};
-        if (q < n) {
+        // (a star whose x step is above 0.1 sqrt 2 sigma is narrow: its FP64 work is not for this kernel)
+        if (q < n && 0.70710678f * (float)g.xs / (float)st.sx[s0 + q] <= 0.11f) {
             star_record(tmp, g, st.x[s0 + q], st.y[s0 + q], st.sx[s0 + q], st.sy[s0 + q], st.w[s0 + q], cov);
             if (tmp.cls == kStarWide || tmp.cls == kStarMid) key = StarKey{tmp.ylo, tmp.yhi, 0ull};
         }
@@ -914,7 +915,7 @@ k_stamp_tiles(StampStars st, Grid2 g0, int ntempl, const StampGroup *__restrict_
         add_stars<true, false, REC>(acc, W, st, st.start[t], st.count[t], warp, ns, g, cov, wa, wb, strips, tl);
     else
         add_stars<false, false, REC>(acc, W, st, st.start[t], st.count[t], warp, ns, g, cov, wa, wb, strips, tl);
-    if (ns > 1) sum_warps(sum, acc, ns);
+    if (ns > 1) sum_warps(sum, acc, max(1, min(ns, st.count[t])));  // (warps beyond the stars have none)
     if (sm.on) {
         // the tile's 8 columns of its Chebyshev tile's 8 node rows: mid[8 n + i][lane]
         const float *f = node + (node_off ? node_off[t] : (int64_t)t * 64 * sm.tiles()) +
@@ -937,7 +938,7 @@ k_stamp_tiles(StampStars st, Grid2 g0, int ntempl, const StampGroup *__restrict_
     }
     if (!tl.live) return;
     float *dst = out + (out_off ? out_off[t] : (int64_t)t * g.nx * g.ny) + (int64_t)tl.row0 * g.nx + tl.col0;
-    const bool wide = (g.nx & 7) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+    const bool wide = (g.nx & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         if ((ns > 1 && j % ns != warp) || tl.row0 + j >= g.ny) continue;
@@ -960,7 +961,7 @@ k_stamp_tiles(StampStars st, Grid2 g0, int ntempl, const StampGroup *__restrict_
         float *row = dst + (int64_t)j * g.nx;
         if (wide) {
             reinterpret_cast<float4 *>(row)[0] = make_float4(v[0], v[1], v[2], v[3]);
-            reinterpret_cast<float4 *>(row)[1] = make_float4(v[4], v[5], v[6], v[7]);
+            if (tl.col0 + 4 < g.nx) reinterpret_cast<float4 *>(row)[1] = make_float4(v[4], v[5], v[6], v[7]);
         } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
@@ -970,36 +971,57 @@ k_stamp_tiles(StampStars st, Grid2 g0, int ntempl, const StampGroup *__restrict_
 }
 
 // The narrow stars of all templates (REC: from k_star_prep's list, dealt out star by star; else
-// grid y -> template, every star looked at), added to the templates.
+// grid y -> template, every star looked at), added to the templates.  Without records a warp makes
+// those of its next stars first, a star per lane and as many as leave work for the other warps: a
+// record made by one lane holds the FP64 pipe as long as 32.  Calls on 100 x 150 bins, separable narrow
+// stars, us, with a record at a time / this way and k_stamp_tiles without their records: 3,000 templates of
+// 30 stars 783 / 178, of 100 2,360 / 272, 30 of 3,000 745 / 132, 1 of 30,000 1,044 / 120.
 template <bool REC>
 __global__ void __launch_bounds__(kNarrowWarps * 32)
 k_stamp_narrow(StampStars st, Grid2 g0, const Grid2 *__restrict__ grids,
                const int64_t *__restrict__ out_off, const StarId *__restrict__ narrow,
                const int *__restrict__ n_narrow, int buf, float *__restrict__ out) {
     extern __shared__ float smem[];
-    __shared__ __align__(16) StarRec s_rec[kNarrowWarps];
+    __shared__ __align__(16) StarRec s_rec[kNarrowWarps][REC ? 1 : 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float *bx_buf = smem + (size_t)warp * buf, *by_buf = bx_buf + buf - kNarrowRows;
-    const int n = REC ? *n_narrow : st.count[blockIdx.y];
-    for (int k = blockIdx.x * kNarrowWarps + warp; k < n; k += gridDim.x * kNarrowWarps) {
-        const StarId id = REC ? narrow[k] : StarId{(int)blockIdx.y, k};
-        const Grid2 g = grids ? grids[id.t] : g0;
-        const int64_t s = st.start[id.t] + id.q;
-        __syncwarp();  // the previous star is done with
-        if (REC) {
+    StarRec *rec = s_rec[warp];
+    const int w0 = blockIdx.x * kNarrowWarps + warp, nw = gridDim.x * kNarrowWarps;
+    if (REC) {
+        const int n = *n_narrow;
+        for (int k = w0; k < n; k += nw) {
+            const StarId id = narrow[k];
+            const Grid2 g = grids ? grids[id.t] : g0;
+            const int64_t s = st.start[id.t] + id.q;
+            __syncwarp();  // the previous star is done with
             if (lane < (int)(sizeof(StarRec) / 4))
-                reinterpret_cast<int *>(&s_rec[warp])[lane] = reinterpret_cast<const int *>(st.rec + s)[lane];
-        } else if (lane == 0) {
-            StarRec r;
-            star_record(r, g, st.x[s], st.y[s], st.sx[s], st.sy[s], st.w[s], st.cov[id.t]);
-            s_rec[warp] = r;
+                reinterpret_cast<int *>(rec)[lane] = reinterpret_cast<const int *>(st.rec + s)[lane];
+            __syncwarp();
+            float *dst = out + (out_off ? out_off[id.t] : (int64_t)id.t * g.nx * g.ny);
+            if (rec->cov != 0) star_cov(dst, *rec, g.nx, lane);
+            else star_asym(dst, bx_buf, by_buf, *rec, g.nx, lane);
         }
-        __syncwarp();
-        const StarRec &r = s_rec[warp];
-        if (!REC && r.cls != kStarNarrow) continue;
-        float *dst = out + (out_off ? out_off[id.t] : (int64_t)id.t * g.nx * g.ny);
-        if (r.cov != 0) star_cov(dst, r, g.nx, lane);
-        else star_asym(dst, bx_buf, by_buf, r, g.nx, lane);
+    } else {
+        const int t = blockIdx.y, n = st.count[t], cov = st.cov[t];
+        const int take = (int)min((int64_t)32, ((int64_t)n + nw - 1) / nw);  // stars of a warp at a time
+        const int64_t s0 = st.start[t];
+        float *dst = out + (int64_t)t * g0.nx * g0.ny;
+        for (int64_t k0 = (int64_t)w0 * take; k0 < n; k0 += (int64_t)nw * take) {
+            const int64_t s = s0 + k0 + lane;
+            bool mine = false;
+            __syncwarp();  // the previous stars are done with
+            if (lane < take && k0 + lane < n) {
+                star_record(rec[lane], g0, st.x[s], st.y[s], st.sx[s], st.sy[s], st.w[s], cov);
+                mine = rec[lane].cls == kStarNarrow;
+            }
+            const unsigned all = __ballot_sync(0xffffffffu, mine);
+            __syncwarp();  // the records are seen by every lane
+            for (unsigned m = all; m; m &= m - 1u) {
+                const StarRec &r = rec[__ffs(m) - 1];
+                if (cov != 0) star_cov(dst, r, g0.nx, lane);
+                else star_asym(dst, bx_buf, by_buf, r, g0.nx, lane);
+            }
+        }
     }
 }
 
@@ -1351,12 +1373,13 @@ int launch_stamps(sfh_ctx *ctx, StampStars st, int64_t ntempl, Grid2 g, const St
     // small part and the stars' sizes even out: 1,200 templates 696 us with eight blocks per SM (the
     // eighth alone in a second wave), 610 with 7, 529 with 56, 515 with 112; 300 separable ones 230,
     // 202, 164, 162; 6 small ones 13 with any.
+    // Without records twice the resident ones: a warp takes up to 32 stars at a time there.
     const unsigned blocks = 56u * (unsigned)ctx->sm_count;
     const dim3 ngrid = have ? dim3((unsigned)std::clamp<int64_t>((w.stars + kNarrowWarps - 1) / kNarrowWarps, 1, blocks))
-                            : dim3(std::max(1u, blocks / (unsigned)ntempl), (unsigned)ntempl);
+                            : dim3(std::max(1u, 14u * (unsigned)ctx->sm_count / (unsigned)ntempl), (unsigned)ntempl);
     auto narrow = have ? k_stamp_narrow<true> : k_stamp_narrow<false>;
     const size_t nsmem = kNarrowWarps * (size_t)buf * sizeof(float);
-    if (nsmem > 47 * 1024)  // (beside the records)
+    if (nsmem > 36 * 1024)  // (beside the records)
         SFH_CK(ctx, cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(kNarrowWarps * (kMaxColumns + kNarrowRows) * sizeof(float))));
     narrow<<<ngrid, kNarrowWarps * 32, nsmem, s>>>(
