@@ -552,59 +552,76 @@ __device__ __forceinline__ void recon_fetch(float4 *s_b, const float *vb, int64_
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-template <int R, int V>
+template <int R>
 __device__ __forceinline__ void recon_segment(const float *__restrict__ sc, float4 *s_b, int K,
                                               const float *__restrict__ vb,
                                               const float *__restrict__ off, int64_t nbins,
                                               int64_t i0, const int32_t *__restrict__ srow,
                                               int cnt, int mode, float *__restrict__ out) {
-    float2 acc[R / 2][V];  // rows 2 r and 2 r + 1
+    float2 acc[R / 2][4];  // rows 2 r and 2 r + 1
 #pragma unroll
     for (int r = 0; r < R / 2; ++r)
 #pragma unroll
-        for (int v = 0; v < V; ++v) acc[r][v] = make_float2(0.f, 0.f);
+        for (int v = 0; v < 4; ++v) acc[r][v] = make_float2(0.f, 0.f);
     int slot = 0;
 #pragma unroll 1
     for (int k = 0; k < K; ++k) {
-        float b[V];
-        if constexpr (V == 4) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kRecDepth - 1) : "memory");  // row k is here
-            const float4 t = s_b[slot * kRecThreads];
-            recon_fetch(s_b + slot * kRecThreads, vb + i0, nbins, k + kRecDepth, K);
-            slot = (slot + 1) % kRecDepth;
-            b[0] = t.x;
-            b[1] = t.y;
-            b[2] = t.z;
-            b[3] = t.w;
-        } else {
-            b[0] = __ldg(vb + (int64_t)k * nbins + i0);
-        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRecDepth - 1) : "memory");  // row k is here
+        const float4 t = s_b[slot * kRecThreads];
+        recon_fetch(s_b + slot * kRecThreads, vb + i0, nbins, k + kRecDepth, K);
+        slot = (slot + 1) % kRecDepth;
+        const float b[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
         for (int r = 0; r < R / 2; r += 2) {
             const float4 c = *reinterpret_cast<const float4 *>(sc + k * kRecRows + 2 * r);
 #pragma unroll
-            for (int v = 0; v < V; ++v) {
+            for (int v = 0; v < 4; ++v) {
                 const float2 bb = make_float2(b[v], b[v]);
                 acc[r][v] = __ffma2_rn(make_float2(c.x, c.y), bb, acc[r][v]);
                 acc[r + 1][v] = __ffma2_rn(make_float2(c.z, c.w), bb, acc[r + 1][v]);
             }
         }
     }
-    float o[V];
+    float o[4];
 #pragma unroll
-    for (int v = 0; v < V; ++v) o[v] = __ldg(off + i0 + v);
+    for (int v = 0; v < 4; ++v) o[v] = __ldg(off + i0 + v);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         if (r >= cnt) break;
-        float *dst = out + (int64_t)srow[r] * nbins + i0;
-        float y[V];
+        float y[4];
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
+        for (int v = 0; v < 4; ++v) {
             const float t = fmaxf((r & 1 ? acc[r / 2][v].y : acc[r / 2][v].x) + o[v], 0.f);
             y[v] = mode == 1 ? t * t : t;
         }
-        if constexpr (V == 4) *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);
-        else *dst = y[0];
+        *reinterpret_cast<float4 *>(out + (int64_t)srow[r] * nbins + i0) = make_float4(y[0], y[1], y[2], y[3]);
+    }
+}
+
+// A bin a thread, where rows do not lie on 16-byte boundaries.  A short loop over k, which the
+// compiler unrolls, and few registers (48): many warps hide the loads' latency.  64 cells x 64
+// components x 60,001 bins, 1 / 6 / 16 rows a cell, us: 193 / 309 / 476; the loop of recon_segment
+// with one row in flight and 106 registers 765 / 792 / 844, eight rows in flight there 541 / 558 /
+// 558.  Coefficients r K + k.
+template <int R>
+__device__ __forceinline__ void recon_segment_1(const float *__restrict__ sc, int K, const float *__restrict__ vb,
+                                                const float *__restrict__ off, int64_t nbins, int64_t i0,
+                                                const int32_t *__restrict__ srow, int cnt, int mode,
+                                                float *__restrict__ out) {
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int k = 0; k < K; ++k) {
+        const float b = __ldg(vb + (int64_t)k * nbins + i0);
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = fmaf(sc[r * K + k], b, acc[r]);
+    }
+    const float o = __ldg(off + i0);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (r >= cnt) break;
+        const float t = fmaxf(acc[r] + o, 0.f);
+        out[(int64_t)srow[r] * nbins + i0] = mode == 1 ? t * t : t;
     }
 }
 
@@ -612,12 +629,11 @@ __device__ __forceinline__ void recon_segment(const float *__restrict__ sc, floa
 // of range writes NaN to the rows it can address and nothing else; a row index outside
 // [0, B) ends its segment at that row.
 template <int V>
-__global__ void __launch_bounds__(kRecThreads, 2)
-k_recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
-               const int32_t *__restrict__ seg, int64_t B, int64_t ngroups,
-               const float *__restrict__ basis, const float *__restrict__ offset, int K,
-               int64_t nbins, int mode, float *__restrict__ out) {
-    extern __shared__ __align__(16) float s_coef[];  // K x kRecRows; copies of basis rows
+__device__ __forceinline__ void recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
+                                             const int32_t *__restrict__ seg, int64_t B, int64_t ngroups,
+                                             const float *__restrict__ basis, const float *__restrict__ offset,
+                                             int K, int64_t nbins, int mode, float *__restrict__ out) {
+    extern __shared__ __align__(16) float s_coef[];  // kRecRows x K; V = 4: copies of basis rows
     __shared__ int32_t srow[kRecRows];
     const int s = blockIdx.y;
     const int g = seg[3 * s], start = seg[3 * s + 1];
@@ -647,18 +663,36 @@ k_recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
         if (srow[r] < 0 && r < cnt) cnt = r;  // a row index out of range ends the segment
     for (int t = threadIdx.x; t < kRecRows * K; t += kRecThreads) {
         const int r = t / K, k = t - r * K;
-        const float c = r < cnt ? coef[(int64_t)srow[r] * K + k] : 0.f;
-        s_coef[k * kRecRows + r] = c;
+        s_coef[V == 4 ? k * kRecRows + r : t] = r < cnt ? coef[(int64_t)srow[r] * K + k] : 0.f;
     }
     __syncthreads();
     if (i0 >= nbins) return;
     const float *off = offset + (int64_t)g * nbins;
-    if (cnt <= 4)
-        recon_segment<4, V>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
-    else if (cnt <= 8)
-        recon_segment<8, V>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
-    else
-        recon_segment<16, V>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
+    if constexpr (V == 4) {
+        if (cnt <= 4) recon_segment<4>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        else if (cnt <= 8) recon_segment<8>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        else recon_segment<16>(s_coef, s_b, K, vb, off, nbins, i0, srow, cnt, mode, out);
+    } else {
+        if (cnt <= 4) recon_segment_1<4>(s_coef, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        else if (cnt <= 8) recon_segment_1<8>(s_coef, K, vb, off, nbins, i0, srow, cnt, mode, out);
+        else recon_segment_1<16>(s_coef, K, vb, off, nbins, i0, srow, cnt, mode, out);
+    }
+}
+
+__global__ void __launch_bounds__(kRecThreads, 2)
+k_recon_groups(const float *__restrict__ coef, const int32_t *__restrict__ rows,
+               const int32_t *__restrict__ seg, int64_t B, int64_t ngroups,
+               const float *__restrict__ basis, const float *__restrict__ offset, int K,
+               int64_t nbins, int mode, float *__restrict__ out) {
+    recon_groups<4>(coef, rows, seg, B, ngroups, basis, offset, K, nbins, mode, out);
+}
+
+__global__ void __launch_bounds__(kRecThreads)
+k_recon_groups_1(const float *__restrict__ coef, const int32_t *__restrict__ rows,
+                 const int32_t *__restrict__ seg, int64_t B, int64_t ngroups,
+                 const float *__restrict__ basis, const float *__restrict__ offset, int K,
+                 int64_t nbins, int mode, float *__restrict__ out) {
+    recon_groups<1>(coef, rows, seg, B, ngroups, basis, offset, K, nbins, mode, out);
 }
 
 struct Acts {  // activations of one batch (G groups x B rows)
@@ -1018,17 +1052,17 @@ extern "C" int sfh_emu_reconstruct_groups(sfh_ctx *ctx, const float *d_coef,
     if (vec) {
         shm += ring;
         if (shm > 40 * 1024)
-            SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups<4>,
+            SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most + ring)));
         dim3 grid((unsigned)((nbins + 4 * kRecThreads - 1) / (4 * kRecThreads)), (unsigned)nseg);
-        k_recon_groups<4><<<grid, kRecThreads, shm, ctx->stream>>>(
+        k_recon_groups<<<grid, kRecThreads, shm, ctx->stream>>>(
             d_coef, d_rows, d_seg, B, ngroups, d_basis, d_offset, K, nbins, mode, d_out);
     } else {
         if (shm > 40 * 1024)
-            SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups<1>,
+            SFH_CK(ctx, cudaFuncSetAttribute(k_recon_groups_1,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         dim3 grid((unsigned)((nbins + kRecThreads - 1) / kRecThreads), (unsigned)nseg);
-        k_recon_groups<1><<<grid, kRecThreads, shm, ctx->stream>>>(
+        k_recon_groups_1<<<grid, kRecThreads, shm, ctx->stream>>>(
             d_coef, d_rows, d_seg, B, ngroups, d_basis, d_offset, K, nbins, mode, d_out);
     }
     SFH_LAUNCHED(ctx);
