@@ -1833,8 +1833,8 @@ struct BinAxis {
     __device__ BinAxis(double f, double s, double i, int n_)
         : first(f), step(s), inv(i), n(n_), tol(1e-6f + 2.4e-7f * (float)n_ + 8e-9f * (float)fabs(i)) {}
     __device__ __forceinline__ int bin(double v, bool &near) const {
-        const float q = (float)((v - first) * inv), k = floorf(q);
-        if (!(q > -1.f && q < (float)n + 1.f)) return -1;
+        const float q = (float)((v - first) * inv), k = floorf(q), out = fmaxf(1.f, tol);
+        if (!(q > -out && q < (float)n + out)) return -1;
         near |= !(q - k > tol && q - k < 1.f - tol);
         return (q >= 0.f && q < (float)n) ? (int)k : -1;
     }
