@@ -67,7 +67,7 @@ __device__ __forceinline__ double nanmax(double a, double b) {
 // after: k_fit_eval with an accepted step 8.0 / 6.1, k_fit_hgemv 6.4 / 4.3, k_fit_hupdate 6.5 /
 // 5.4, k_fit_trial with a new direction 5.1 / 3.8, each with 1.1 us between two kernels (as
 // programmatic dependents of one another the whole fit took the same time).  A fit of 331
-// evaluations: 11.6 ms / 10.4 ms.
+// evaluations: 11.6 ms / 10.2 ms.
 
 // Tree sums of N = 2 or 4 values over a warp (pairs 16 lanes apart, then 8, 4, 2, 1): value k ends
 // in lane 32 k / N.  While lanes still hold several values, half of them go on with one half of

@@ -216,7 +216,9 @@ k_ragged_pass2(const float *__restrict__ M, const GalDesc *__restrict__ gals,
 // needed, 176 us now (2.4 TB/s; the arithmetic of a bin, about 600 instructions, is the rest).
 // Four rows of more than 12 templates leave too little of the SM's memory as L1: calls of 197
 // galaxies of 8, 12, 16 templates 127, 151, 156 us without, 124, 142, 170 four rows ahead, -, 139,
-// 144 two ahead.
+// 144 two ahead.  256 galaxies of 17, 20, 24, 28, 32 templates on grids of 50 to 220 bins a side: 295,
+// 292, 303, 309, 331 us without, 259, 259, 278, 290, 319 two ahead.  Batches of up to 5,000 bins a
+// galaxy and 5 to 8 templates lose 1 to 2 us of 19 to 43 on the device, four rows or two ahead.
 __host__ __device__ constexpr int fused_depth(int NT) { return NT <= 8 ? kFuseRows : 2; }
 __host__ __device__ inline int64_t fused_pad(int64_t nt) { return (nt + 3) / 4 * 4; }
 size_t fused_smem(int NT, int64_t nt) {  // counts, then rows of M: [depth][pad][kRT]
