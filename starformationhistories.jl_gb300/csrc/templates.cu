@@ -109,7 +109,7 @@ enum { kStarNone = 0, kStarWide = 1, kStarMid = 2, kStarNarrow = 3 };
 struct __align__(16) StarRec {
     // wide: hx, bx, by, amp | uref, vref, kx, ky | cu, cv, strips (64 bits)   (see wide_tile)
     // mid: hx, bx, by, amp | uref, vref, kx, du | dv, -, -, -      (see mid_tile)
-    // narrow, covariant: uref, bx, bx low, sx | sx low, vref, by, pref | k4, k6, vref low, by low
+    // narrow, covariant: uref, bx, bx low, sx | sx low, vref, by, pref | k4, uref low, vref low, by low
     // narrow, separable: invx, invy, dx0, dy0 | A/4
     float p[12];
     int xlo, xhi, ylo, yhi;  // first and last bin of the window, 0-based, inside the grid
@@ -311,7 +311,9 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     // (a vanishing error: far edges at a large finite t, a hard histogram)
     const double scale = fmin(0.7071067811865476 * rx * (gauss ? gs : 1.0), 1.0e30);
     const double bxs = c * g.ys * scale, sxs = g.xs * scale;
-    r.p[0] = (float)((X + c * Y - (gauss ? 0.0 : g.xs * 0.5)) * scale);
+    const double uref = (X + c * Y - (gauss ? 0.0 : g.xs * 0.5)) * scale;
+    r.p[0] = (float)uref;
+    r.p[9] = (float)(uref - (double)r.p[0]);
     r.p[1] = (float)bxs;
     r.p[2] = (float)(bxs - (double)r.p[1]);
     r.p[3] = (float)sxs;
@@ -327,7 +329,6 @@ __device__ __forceinline__ void star_record(StarRec &r, const Grid2 &g, double x
     r.p[7] = (float)(A * bys * 0.11742965983745643 * (gauss ? 0.7978845608028654 * k : 1.0));
     const float k2 = (float)(k * k);
     r.p[8] = gauss ? k2 * k2 * (1.f / 2880.f) : -1.f;
-    r.p[9] = k2 * k2 * k2 * (1.f / 181440.f);
 }
 
 // The strips over which a wide star's contribution can be interpolated from 8 x 8 Chebyshev
@@ -435,7 +436,7 @@ __device__ void star_asym(float *__restrict__ out, float *bx_buf, float *by_buf,
 // u of a bin near the kernel's centre in that row (the shear and the bin's offset cancel there:
 // their sum is formed in two floats), which the warp then reads by shuffles.
 __device__ void star_cov(float *__restrict__ out, const StarRec &r, int nx, int lane) {
-    const float sx = r.p[3], k4 = r.p[8], k6 = r.p[9];
+    const float sx = r.p[3], k4 = r.p[8], k6 = 0.85183542f * fmaxf(k4, 0.f) * sqrtf(fmaxf(k4, 0.f));  // k^4 / 2880, k^6 / 181440
     const int lx = r.xhi - r.xlo + 1, nrows = r.yhi - r.ylo + 1;
     const float c_first = (float)r.xlo - r.ir, c_last = (float)(r.xhi + 1) - r.ir;
     float *row0 = out + (int64_t)r.ylo * nx + r.xlo;
@@ -451,16 +452,18 @@ __device__ void star_cov(float *__restrict__ out, const StarRec &r, int nx, int 
         // u (at the reference bin) and v of the row's centre as two floats each
         const float d = (float)(r.ylo + r0 + lane) - r.jr, bx = r.p[1], by = r.p[6];
         const float p = d * bx, uh = r.p[0] + p, z = uh - r.p[0];
-        const float ul = ((r.p[0] - (uh - z)) + (p - z)) + fmaf(d, r.p[2], fmaf(d, bx, -p));
+        const float ul = ((r.p[0] - (uh - z)) + (p - z)) + fmaf(d, r.p[2], fmaf(d, bx, -p) + r.p[9]);
         const float p2 = d * by, vh = r.p[5] + p2, z2 = vh - r.p[5];
         const float vl = ((r.p[5] - (vh - z2)) + (p2 - z2)) +
                          fmaf(d, r.p[11], fmaf(d, by, -p2) + r.p[10]);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const float gk = (float)(k - 1) * 0.38729835f, gl = (float)(k - 1) * -1.0945054e-8f;  // sqrt(3/5) / 2
-            ek[k] = fminf(fmaxf(rintf(-__fdividef(fmaf(gk, bx, uh), sx)), c_first), c_last);
-            const float t = fmaf(ek[k], sx, uh);
-            tk[k] = fmaf(gk, bx, t) + fmaf(gl, bx, fmaf(ek[k], r.p[4], ul));
+            // uh + gk bx as two floats: a y step of thousands of x sigmas leaves no bits to either
+            const float g = gk * bx, s = uh + g, zs = s - uh;
+            const float sl = ((uh - (s - zs)) + (g - zs)) + fmaf(gk, r.p[2], fmaf(gk, bx, -g));
+            ek[k] = fminf(fmaxf(rintf(-__fdividef(s, sx)), c_first), c_last);
+            tk[k] = fmaf(ek[k], sx, s) + (sl + fmaf(gl, bx, fmaf(ek[k], r.p[4], ul)));
             const float v = fmaf(gk, by, vh) + fmaf(gl, by, fmaf(gk, r.p[11], vl)), q = v * v;
             ck[k] = r.p[7] * c_glw[k] * ex2f(-q) * fmaf(-0.6931471805599453f, fmaf(v, v, -q), 1.f);
         }

@@ -42,3 +42,15 @@ def test_descending_edges(sfh, O, cov, flip):
     R = O.bin_cmd_smooth(x, y, sx, sy, w, cov, (xe[0], (xe[-1] - xe[0]) / nx, nx),
                          (ye[0], (ye[-1] - ye[0]) / ny, ny))
     assert np.all(np.abs(H - R) <= 1e-5 * np.abs(R) + 1e-6 * np.abs(R).max())
+
+
+@pytest.mark.parametrize("cov", [1, -1])
+@pytest.mark.parametrize("nx,ny,xs,ys", [(277, 6, 0.0034, 1.6), (92, 20, 0.007, 1.8), (74, 6, 0.008, 6.1)])
+def test_y_steps_of_thousands_of_x_errors(sfh, O, cov, nx, ny, xs, ys):
+    """Stars of a few bins or less in x whose shear over one row is up to 1e5 x errors."""
+    rng = np.random.default_rng(nx + cov)
+    xe, ye = 0.1 + xs * np.arange(nx + 1), 20.0 + ys * np.arange(ny + 1)
+    n = 400
+    sx = xs * np.exp(rng.uniform(np.log(0.01), np.log(5.0), n))
+    sy = np.where(rng.random(n) < 0.5, sx * ys / xs, ys * np.exp(rng.uniform(np.log(0.002), np.log(3.0), n)))
+    _check(sfh, O, rng.uniform(xe[0], xe[-1], n), rng.uniform(ye[0], ye[-1], n), sx, sy, cov, xe, ye)
